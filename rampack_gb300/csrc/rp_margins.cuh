@@ -50,14 +50,15 @@ inline FilterConsts hard_filter_consts(int kind, double r, double l, double lrow
         // Segment certificate.  Input errors move each cap by at most dend, which changes
         // the segment distance d by at most 2 dend; near the threshold (d ~ 2r; farther away
         // the decision has a margin larger than any of these terms) that is
-        // 2 (2r)(2 dend) + (2 dend)^2 in d^2.  FP32 evaluation of dP = w + s u - t v
-        // (|w| <= 2r + 2l, |u| = |v| = l) errs by at most 4 u32 sqrt(3) (|w| + 2 l) per
-        // vector, giving 2 (1.1 * 2r) ddp + ddp^2 in f; the gap G adds 4 u32 (2r) l.
+        // 2 (2r)(2 dend) + (2 dend)^2 in d^2.  FP32 evaluation of dP = d + mu a_j - lam a_i
+        // (|d| <= 2r + l, |lam|, |mu| <= l / 2; two roundings per component) errs by at most
+        // 4 u32 sqrt(3) (2r + 4 l) per vector, giving 2 (1.1 * 2r) ddp + ddp^2 in f; the gap G
+        // (two products dP . a of three roundings, each times at most l) adds 16 u32 (2r) l.
         double dend = std::sqrt(3.0) * (e_sep + l * e_axis);
         double ddp = 4.0 * u32 * std::sqrt(3.0) * (2 * r + 4 * l);
-        double eval = 2.0 * 1.1 * (2 * r) * ddp + ddp * ddp + 4.0 * u32 * (2 * r) * l;
+        double eval = 2.0 * 1.1 * (2 * r) * ddp + ddp * ddp + 16.0 * u32 * (2 * r) * l;
         // FP64 evaluates the distance at its own closest-point parameters, with its own
-        // inputs; rounding in sN = b e - c d and D = a c - b^2 (|b|, |c| <= l^2,
+        // inputs; rounding in sN = b e - c d and D = a c - b^2 = l^4 sin^2 (|b|, |c| <= l^2,
         // |d|, |e| <= l (2r + 2l)) moves the parameters by at most noise / D, which raises
         // its distance^2 above the minimum by at most g64 = 2 (2r) l sqrt(2) noise / D.
         // Pairs whose (cancellation-free) D is below d_min are re-decided in FP64; g64 at
@@ -68,8 +69,9 @@ inline FilterConsts hard_filter_consts(int kind, double r, double l, double lrow
         const double u64 = std::ldexp(1.0, -52);
         const double noise = 8.0 * u64 * 2.0 * l * l * l * (2 * r + 2 * l);
         const double g64 = 2e-6;
-        fc.d_min = static_cast<float>(std::max(4.0 * (2 * r) * l * std::sqrt(2.0) * noise / g64 * 10.0,
-                                               1e-9 * l * l * l * l));
+        const double l4 = l * l * l * l;
+        const double d_min = std::max(4.0 * (2 * r) * l * std::sqrt(2.0) * noise / g64 * 10.0, 1e-9 * l4);
+        fc.s2_min = l > 0 ? static_cast<float>(d_min / l4) : 2.0f;   // l = 0: every pair in FP64
         fc.seg_err = static_cast<float>(safety * (2.0 * (2 * r) * 2.0 * dend + 4.0 * dend * dend + eval) + g64);
         // Parallel branch (SegmentDistanceCalculator.h:35-39, taken when FP64's D < 1e-10):
         // FP64's D = l^4 sin^2(theta) up to ~4 ulp(l^4), so sin(theta) < theta_lim keeps it
@@ -78,13 +80,12 @@ inline FilterConsts hard_filter_consts(int kind, double r, double l, double lrow
         const double d_noise = 16.0 * l * l * l * u64 * (pmax + l);  // FP64 rounding in its D
         const double theta_lim = std::sqrt(std::max(0.0, 0.8e-10 - d_noise)) / (l * l) - 8.0 * u32;
         if (l > 0 && theta_lim > 0) {
-            fc.d_par = static_cast<float>(l * l * l * l * theta_lim * theta_lim * 0.5);
+            fc.s2_par = static_cast<float>(theta_lim * theta_lim * 0.5);
             fc.par_err = static_cast<float>(4.0 * (2 * r + 1e-3) * l * (theta_lim + 8.0 * u32) + 1e-6);
         } else {
-            fc.d_par = 0.0f;
+            fc.s2_par = 0.0f;
             fc.par_err = 0.0f;
         }
-        fc.len = static_cast<float>(l);
         fc.half_len = static_cast<float>(0.5 * l);
     }
     fc.cell_margin = 1e-5f;
