@@ -33,8 +33,8 @@ int axis_moment_blocks(int64_t n);
 cudaError_t launch_b_rebuild(const BatchRep *T, const int *pbase, const int *cbase, int R, int total_particles,
                              int total_cells, cudaStream_t st);
 cudaError_t launch_b_rescale(const BatchRep *T, const int *pbase, int R, int total_particles, cudaStream_t st);
-cudaError_t launch_b_count(const BatchRep *T, const int *pbase, int R, int total_particles, int kind, int early,
-                           unsigned long long *out, int *flags, cudaStream_t st);
+cudaError_t launch_b_count(const BatchRep *T, const int *pbase, const int *cbase, int R, int total_particles,
+                           int total_cells, int kind, int early, unsigned long long *out, int *flags, cudaStream_t st);
 size_t batch_smem_per_warp(int kind, int cap);
 cudaError_t launch_b_sweep(const BatchRep *T, const int *item_base, int R, int kind, int k, int *next_item, int cap,
                            int wpb, int blocks, bool rototranslation, cudaStream_t st);
@@ -3179,7 +3179,7 @@ int rp_batch_try_scaling(void *batch, const double *boxes, const uint8_t *propos
     }
     {
         BGroup grp(b, RP_KERNEL_COUNT, 1);
-        RB_CUDA(b, launch_b_count(b->d_table, pb, b->R, total_p, b->kind, 1, b->counts, b->flags, b->stream));
+        RB_CUDA(b, launch_b_count(b->d_table, pb, cb, b->R, total_p, total_c, b->kind, 1, b->counts, b->flags, b->stream));
     }
     RB_CUDA(b, cudaMemcpyAsync(b->h_counts, b->counts, sizeof(unsigned long long) * b->R, cudaMemcpyDeviceToHost,
                                b->stream));

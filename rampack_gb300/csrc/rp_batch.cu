@@ -129,6 +129,17 @@ __global__ void k_b_trans(const BatchRep *T, int R) {
     B.trans_dst[3 * m + 2] = tr.z;
 }
 
+constexpr int COUNT_WARPS = 8;
+template <int KIND>
+__global__ void __launch_bounds__(COUNT_WARPS * 32) k_b_count_cells(const BatchRep *T, const int *cbase, int R, int parts,
+                                                                    int early, unsigned long long *out, int *flags) {
+    __shared__ CountSmem sm[COUNT_WARPS];
+    const int w = threadIdx.x >> 5, item = blockIdx.x * COUNT_WARPS + w, c = item / parts;
+    if (c >= cbase[R]) return;
+    const int r = find_rep(cbase, R, c);
+    count_cell<KIND>(T[r].a.s, T[r].a.g, c - cbase[r], item - c * parts, parts, early, out + r, flags + r, sm[w]);
+}
+
 template <int KIND>
 __global__ void k_b_count(const BatchRep *T, const int *pbase, int R, int early, unsigned long long *out, int *flags) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -278,11 +289,18 @@ cudaError_t launch_b_rescale(const BatchRep *T, const int *pbase, int R, int tot
     return cudaGetLastError();
 }
 
-cudaError_t launch_b_count(const BatchRep *T, const int *pbase, int R, int total_particles, int kind, int early,
-                           unsigned long long *out, int *flags, cudaStream_t st) {
-    const unsigned nb = (unsigned)((total_particles + 127) / 128);
-    if (kind == 0) k_b_count<0><<<nb, 128, 0, st>>>(T, pbase, R, early, out, flags);
-    else k_b_count<1><<<nb, 128, 0, st>>>(T, pbase, R, early, out, flags);
+cudaError_t launch_b_count(const BatchRep *T, const int *pbase, const int *cbase, int R, int total_particles,
+                           int total_cells, int kind, int early, unsigned long long *out, int *flags, cudaStream_t st) {
+    if (!count_by_cells(total_particles, total_cells)) {
+        const unsigned nb = (unsigned)((total_particles + 127) / 128);
+        if (kind == 0) k_b_count<0><<<nb, 128, 0, st>>>(T, pbase, R, early, out, flags);
+        else k_b_count<1><<<nb, 128, 0, st>>>(T, pbase, R, early, out, flags);
+        return cudaGetLastError();
+    }
+    const int parts = count_parts(total_cells), th = COUNT_WARPS * 32;
+    const unsigned nb = (unsigned)(((int64_t)total_cells * parts + COUNT_WARPS - 1) / COUNT_WARPS);
+    if (kind == 0) k_b_count_cells<0><<<nb, th, 0, st>>>(T, cbase, R, parts, early, out, flags);
+    else k_b_count_cells<1><<<nb, th, 0, st>>>(T, cbase, R, parts, early, out, flags);
     return cudaGetLastError();
 }
 

@@ -250,24 +250,23 @@ __global__ void k_rescale(const double *src, double *dst, int64_t n, Mat9 old_in
 }
 
 // ---------------------------------------------------------------------------------
-// All-pairs recount: one thread per particle (slot order); each unordered pair and
-// periodic image is visited once (candidate index greater than own index).
+// All-pairs recount: one warp per cell (count_cell), or one thread per particle where cells are
+// nearly empty.  Multi-centre bodies count overlapping centre pairs, as the reference's
+// countTotalOverlaps counts them (core/Packing.cpp:468-512).
 // ---------------------------------------------------------------------------------
+constexpr int COUNT_WARPS = 8;
+template <int KIND>
+__global__ void __launch_bounds__(COUNT_WARPS * 32) k_count_cells(DevState s, GridDev g, int parts, int early,
+                                                                  unsigned long long *out, int *flag) {
+    __shared__ CountSmem sm[COUNT_WARPS];
+    const int w = threadIdx.x >> 5, item = blockIdx.x * COUNT_WARPS + w, cell = item / parts;
+    if (cell < g.ncell) count_cell<KIND>(s, g, cell, item - cell * parts, parts, early, out, flag, sm[w]);
+}
+
 template <int KIND>
 __global__ void k_count(DevState s, GridDev g, int early, unsigned long long *out, int *flag) {
     int64_t slot = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (slot < s.n) count_one<KIND>(s, g, slot, early, out, flag);
-}
-
-template __global__ void k_count<0>(DevState, GridDev, int, unsigned long long *, int *);
-template __global__ void k_count<1>(DevState, GridDev, int, unsigned long long *, int *);
-
-// All-pairs recount of polyspheres: one thread per body; every unordered body pair and
-// periodic image once, every pair of their centres (the count of overlapping centre pairs,
-// as the reference's countTotalOverlaps counts them, core/Packing.cpp:468-512).
-__global__ void k_count_poly(DevState s, GridDev g, int early, unsigned long long *out, int *flag) {
-    int64_t slot = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (slot < s.n) count_poly_one(s, g, slot, early, out, flag);
 }
 
 // MODE 1 instantiates the learned-ordering pre-test and the pair-outcome log, MODE 2 the
@@ -428,10 +427,17 @@ __global__ void k_count_deferred(DevState s, int early, unsigned long long *out,
 
 cudaError_t launch_count(const DevState &s, const GridDev &g, int early, unsigned long long *out, int *flag,
                          cudaStream_t st) {
-    unsigned nb = (unsigned)((s.n + 127) / 128);
-    if (s.kind == 0) k_count<0><<<nb, 128, 0, st>>>(s, g, early, out, flag);
-    else if (s.kind == 1) k_count<1><<<nb, 128, 0, st>>>(s, g, early, out, flag);
-    else k_count_poly<<<nb, 128, 0, st>>>(s, g, early, out, flag);
+    if (s.kind != 2 && !count_by_cells(s.n, g.ncell)) {
+        const unsigned nb = (unsigned)((s.n + 127) / 128);
+        if (s.kind == 0) k_count<0><<<nb, 128, 0, st>>>(s, g, early, out, flag);
+        else k_count<1><<<nb, 128, 0, st>>>(s, g, early, out, flag);
+        return cudaGetLastError();
+    }
+    const int parts = count_parts(g.ncell), th = COUNT_WARPS * 32;
+    const unsigned nb = (unsigned)(((int64_t)g.ncell * parts + COUNT_WARPS - 1) / COUNT_WARPS);
+    if (s.kind == 0) k_count_cells<0><<<nb, th, 0, st>>>(s, g, parts, early, out, flag);
+    else if (s.kind == 1) k_count_cells<1><<<nb, th, 0, st>>>(s, g, parts, early, out, flag);
+    else k_count_cells<2><<<nb, th, 0, st>>>(s, g, parts, early, out, flag);
     if (s.kind == 2 && s.cq_buf) {
         int sms = 152, dev = 0;
         cudaGetDevice(&dev);
