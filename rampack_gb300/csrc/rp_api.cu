@@ -403,6 +403,32 @@ double poly_margin(const Handle *h, const GridHost &g, double thr) {
     return 2.0 * (2.0 * d * std::sqrt(3.0) * e + 3.0 * e * e + 4.0 * u32 * thr);
 }
 
+// Margins of the FP32 segment stage of polyspherocylinder centres, as hard_filter_consts forms
+// them for spherocylinders, with l = twice the longest half axis and r the largest radius: the
+// separation of two centres errs by poly_margin's e per component, a half axis by 8 u32 |h|
+// (rounding, the FP32 rotation of the mover's), so an end by dend; g64 bounds the FP64 distance's
+// excess over the minimum from its own parameter error at |ha x hb|^2 = s2_min (D / 16).
+void poly_segment_consts(const Handle *h, const GridHost &g, FilterConsts &fc) {
+    const double u32 = std::ldexp(1.0, -24), u64 = std::ldexp(1.0, -52);
+    double cmax = 0, hmax = 0, r = 0;
+    for (int b = 0; b < h->ncen; b++) {
+        const double *c = h->cbody + 3 * b, *x = h->chax + 3 * b;
+        cmax = std::max(cmax, std::sqrt(c[0] * c[0] + c[1] * c[1] + c[2] * c[2]));
+        hmax = std::max(hmax, std::sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]));
+        r = std::max(r, h->crad[b]);
+    }
+    const double l = 2 * hmax, L = cell_lrow(g);
+    const double e = 32.0 * u32 * (L + 1.0) + 32.0 * u32 * (cmax + L + 1.0);
+    const double dend = std::sqrt(3.0) * (e + 8.0 * u32 * hmax);
+    const double ddp = 4.0 * u32 * std::sqrt(3.0) * (2 * r + 4 * l);
+    const double eval = 2.0 * 1.1 * (2 * r) * ddp + ddp * ddp + 16.0 * u32 * (2 * r) * l + 4.0 * u32 * 4 * r * r;
+    const double noise = 8.0 * u64 * 2.0 * l * l * l * (2 * r + 2 * l), g64 = 2e-6;
+    const double d_min = std::max(4.0 * (2 * r) * l * std::sqrt(2.0) * noise / g64 * 10.0, 1e-9 * l * l * l * l);
+    fc.seg_err = static_cast<float>(2.0 * (2.0 * (2 * r) * 2.0 * dend + 4.0 * dend * dend + eval) + g64);
+    // (FP64's parallel branch, D below 1e-10, is never certified)
+    fc.s2_min = static_cast<float>(std::max(d_min, 4e-10) / 16.0);
+}
+
 DevState dev_state(Handle *h) {
     DevState s{};
     s.n = h->n;
@@ -481,9 +507,16 @@ DevState dev_state(Handle *h) {
         double far = h->range * h->range;
         fc.far_lo = static_cast<float>(far - poly_margin(h, g, far));
         fc.far_hi = static_cast<float>(far + poly_margin(h, g, far));
+        if (h->segs) poly_segment_consts(h, g, fc);
     }
     s.fc = fc;
     return s;
+}
+
+// Candidates a warp stages in `bytes` of shared memory beside its scratch (16-bit queue entries).
+size_t staging_capacity(size_t bytes, int kind, int ncen) {
+    const size_t fixed = sweep_smem_per_warp(kind, 0, false, ncen);
+    return std::min<size_t>((bytes - fixed) * 32 / (sweep_smem_per_warp(kind, 32, false, ncen) - fixed), 65504);
 }
 
 // Chooses the checkerboard grid for a box: cells at least one interaction range high
@@ -573,21 +606,23 @@ int setup_grid(Handle *h, GridHost &G, const double *box, const double *shift) {
         RP_CUDA(h, cudaMalloc(&g.max_occ, sizeof(int32_t)));
         if (h->ncen > 0) {
             RP_CUDA(h, cudaMalloc(&g.mcen, sizeof(float4) * n * h->ncen));
-            RP_CUDA(h, cudaMalloc(&g.cthr, sizeof(float) * 2 * MAX_CEN * MAX_CEN));
+            if (h->segs) RP_CUDA(h, cudaMalloc(&g.mhax, sizeof(float4) * n * h->ncen));
+            RP_CUDA(h, cudaMalloc(&g.cthr, sizeof(float) * 3 * MAX_CEN * MAX_CEN));
         }
     }
     if (h->ncen > 0) {
         // FP32 centre-pair thresholds of this grid: (r_a + r_b)^2 - margin (overlap below) and
         // (r_a + r_b)^2 + margin (none above); for polyspherocylinders the upper one is the
-        // circumspheres' (c_a + c_b)^2 + margin, between the two the segments decide in FP64
+        // circumspheres' (c_a + c_b)^2 + margin, between the two the segments decide
         std::vector<float> &t = G.cthr;
-        t.assign(2 * MAX_CEN * MAX_CEN, 0.0f);
+        t.assign(3 * MAX_CEN * MAX_CEN, 0.0f);
         for (int a = 0; a < h->ncen; a++)
             for (int b = 0; b < h->ncen; b++) {
                 double thr = h->cthr_host[a * MAX_CEN + b];
                 double hi = h->segs ? h->circ_host[a * MAX_CEN + b] : thr;
                 t[a * MAX_CEN + b] = static_cast<float>(thr - poly_margin(h, G, thr));
                 t[MAX_CEN * MAX_CEN + a * MAX_CEN + b] = static_cast<float>(hi + poly_margin(h, G, hi));
+                t[2 * MAX_CEN * MAX_CEN + a * MAX_CEN + b] = static_cast<float>(thr);
             }
         RP_CUDA(h, cudaMemcpyAsync(g.cthr, t.data(), sizeof(float) * t.size(), cudaMemcpyHostToDevice, h->stream));
     }
@@ -645,7 +680,7 @@ int setup_grid(Handle *h, GridHost &G, const double *box, const double *shift) {
     double mean = 27.0 * kept * static_cast<double>(h->n) / static_cast<double>(ncell);
     int cap = static_cast<int>(mean + 6.0 * std::sqrt(mean) + 32.0);
     cap = (cap + 31) / 32 * 32;
-    int maxcap = static_cast<int>(48 * 1024 / (sweep_smem_per_warp(h->shape.kind, 32, false, h->ncen) / 32));
+    int maxcap = static_cast<int>(staging_capacity(48 * 1024, h->shape.kind, h->ncen));
     G.cap = std::min(cap, maxcap / 32 * 32);
     // two cells per warp: 32 lane groups per SM (4 blocks of 8) in 224 KB of shared memory
     // (capacities in multiples of 16); offered while that capacity holds the mean
@@ -804,7 +839,7 @@ static void order_starts(const GridDev &g, int start[27]) {
 // Re-runs the cells of a phase whose neighbourhood did not fit the normal staging
 // capacity, with one large-capacity warp per block (device-side work count).
 int run_overflow(Handle *h, SweepArgs a, bool list) {
-    int cap = static_cast<int>(OVF_SMEM / sweep_smem_per_warp(a.s.kind, 32, false, a.s.ncen) * 32);
+    int cap = static_cast<int>(staging_capacity(OVF_SMEM, a.s.kind, a.s.ncen));
     cap = cap / 32 * 32;
     a.cap = cap;
     a.work = h->overflow;
@@ -1289,6 +1324,7 @@ int rp_destroy(void *handle) {
         if (!h->batch_member) cudaFree(g.bounds);
         cudaFree(g.max_occ);
         cudaFree(g.mcen);
+        cudaFree(g.mhax);
         cudaFree(g.cthr);
     }
     cudaFree(h->rot64);

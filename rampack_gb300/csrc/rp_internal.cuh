@@ -70,7 +70,9 @@ struct GridDev {
     int32_t *order_off;
     // polyspheres
     float4 *mcen;         // [n][ncen] FP32 rotated centre offsets, cell order
-    float *cthr;          // [2][MAX_CEN^2] FP32 centre-pair thresholds (r_a + r_b)^2 -/+ margin
+    float4 *mhax;         // [n][ncen] FP32 rotated half axes (polyspherocylinders), cell order
+    float *cthr;          // [3][MAX_CEN^2] FP32 centre-pair thresholds: (r_a + r_b)^2 - margin, the upper one
+                          // + margin, and (r_a + r_b)^2 itself (the segment stage adds its own margin)
     // staging filter (cells well above the interaction range): a neighbour is staged only
     // if its distance from each face-slab of the home cell, in cell fractions times the
     // cell height stage_h[d], is at most stage_thr (the range plus a margin)
@@ -186,9 +188,10 @@ RP_HD int cell_phase(const int *dims, int cell) {
     return ring_colour(dims[0], cx) + 3 * ring_colour(dims[1], cy) + 9 * ring_colour(dims[2], cz);
 }
 // per-warp polysphere scratch of the sweep (float4 units): the mover's FP32 centres
-// [MAX_CEN], the centre-pair thresholds [2 MAX_CEN^2 floats], the mover's exact centres
-// and absolute centres [2 x 3 MAX_CEN doubles]
-constexpr int SWEEP_POLY_SCRATCH = MAX_CEN + MAX_CEN * MAX_CEN / 2 + 3 * MAX_CEN + 3 * MAX_CEN / 2;
+// [MAX_CEN], the centre-pair thresholds [3 MAX_CEN^2 floats], the mover's exact centres,
+// absolute centres and half axes [3 x 3 MAX_CEN doubles], its FP32 half axes [MAX_CEN], the queue
+// of centre pairs for the segment stage [64 words]
+constexpr int SWEEP_POLY_SCRATCH = MAX_CEN + 3 * MAX_CEN * MAX_CEN / 4 + 9 * MAX_CEN / 2 + MAX_CEN + 16;
 
 constexpr int NUM_COUNTERS = 9;     // sweep statistics words per handle (rp_sweep_stats order)
 constexpr int SWEEP_WARPS = 4;       // warps per block of the sweep kernel

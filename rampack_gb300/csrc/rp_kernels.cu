@@ -181,7 +181,10 @@ __global__ void k_remap(DevState s, GridDev g, GridDev old, int *moved) {
     g.pid_cell[pid] = cell;
     g.mpos[k] = make_float4(loc.x, loc.y, loc.z, __int_as_float(pid));
     g.maxis[k] = old.maxis[k];
-    for (int b = 0; b < s.ncen; b++) g.mcen[k * s.ncen + b] = old.mcen[k * s.ncen + b];
+    for (int b = 0; b < s.ncen; b++) {
+        g.mcen[k * s.ncen + b] = old.mcen[k * s.ncen + b];
+        if (s.segs) g.mhax[k * s.ncen + b] = old.mhax[k * s.ncen + b];
+    }
 }
 
 // Absolute centres of every polysphere (Packing::recalculateAbsoluteInteractionCentres,
@@ -272,7 +275,7 @@ __global__ void k_count(DevState s, GridDev g, int early, unsigned long long *ou
 // MODE 1 instantiates the learned-ordering pre-test and the pair-outcome log, MODE 2 the
 // overlap counting, MODE 3 the plain scan of rototranslations (kept out of the plain
 // kernel, whose registers and branches they would crowd)
-template <int KIND, bool LIST, int MODE, int GW>
+template <int KIND, bool LIST, int MODE, int GW, bool SEG>
 __global__ void __launch_bounds__(SWEEP_WARPS * 32, SWEEP_MIN_BLOCKS) k_sweep(const SweepArgs A) {
     extern __shared__ float4 smem[];
     const Grp<GW> grp;
@@ -323,7 +326,7 @@ __global__ void __launch_bounds__(SWEEP_WARPS * 32, SWEEP_MIN_BLOCKS) k_sweep(co
             item = grp.shfl(it, 0);
         }
         if (item >= nitems) break;
-        sweep_cell<KIND, LIST, MODE, GW>(A, item, -1, A.cap, A.overflow, A.overflow_count, cpos, cax, qseg, qun, nacc,
+        sweep_cell<KIND, LIST, MODE, GW, SEG>(A, item, -1, A.cap, A.overflow, A.overflow_count, cpos, cax, qseg, qun, nacc,
                                           pstage, cslot, wx, ws);
         grp.sync();
         if (ws.abort) break;
@@ -471,13 +474,13 @@ size_t sweep_smem_per_half(int kind, int cap) {
 int sweep_half_blocks_per_sm(int kind, int cap) {
     const size_t smem = sweep_smem_per_half(kind, cap) * (SWEEP_WARPS * 2);
     int n = 0;
-    cudaError_t e = kind == 0 ? cudaFuncSetAttribute(k_sweep<0, false, 0, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = kind == 0 ? cudaFuncSetAttribute(k_sweep<0, false, 0, 16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      (int)smem)
-                              : cudaFuncSetAttribute(k_sweep<1, false, 0, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              : cudaFuncSetAttribute(k_sweep<1, false, 0, 16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      (int)smem);
     if (e != cudaSuccess) return 0;
-    e = kind == 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep<0, false, 0, 16>, SWEEP_WARPS * 32, smem)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep<1, false, 0, 16>, SWEEP_WARPS * 32, smem);
+    e = kind == 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep<0, false, 0, 16, false>, SWEEP_WARPS * 32, smem)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep<1, false, 0, 16, false>, SWEEP_WARPS * 32, smem);
     return e == cudaSuccess ? n : 0;
 }
 
@@ -487,12 +490,12 @@ cudaError_t launch_rot_table(double *out64, float *out32, uint32_t count, uint64
     return cudaGetLastError();
 }
 
-template <int KIND, bool LIST, int MODE, int GW = 32>
+template <int KIND, bool LIST, int MODE, int GW = 32, bool SEG = KIND == 2>
 static cudaError_t launch_sweep_t(const SweepArgs &a, unsigned blocks, int threads, size_t smem, cudaStream_t st) {
-    cudaError_t e = cudaFuncSetAttribute(k_sweep<KIND, LIST, MODE, GW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(k_sweep<KIND, LIST, MODE, GW, SEG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem);
     if (e != cudaSuccess) return e;
-    k_sweep<KIND, LIST, MODE, GW><<<blocks, threads, smem, st>>>(a);
+    k_sweep<KIND, LIST, MODE, GW, SEG><<<blocks, threads, smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -525,7 +528,8 @@ cudaError_t launch_sweep(const SweepArgs &a, bool list, int nwarps, cudaStream_t
         if (list) return launch_sweep_t<2, true, 0>(a, blocks, th, smem, st);
         if (learn) return launch_sweep_t<2, false, 1>(a, blocks, th, smem, st);
         return rt ? launch_sweep_t<2, false, 3>(a, blocks, th, smem, st)
-                  : launch_sweep_t<2, false, 0>(a, blocks, th, smem, st);
+             : a.s.segs ? launch_sweep_t<2, false, 0>(a, blocks, th, smem, st)
+                        : launch_sweep_t<2, false, 0, 32, false>(a, blocks, th, smem, st);
     }
     if (rt) return a.s.kind == 0 ? launch_sweep_t<0, false, 3>(a, blocks, th, smem, st)
                                  : launch_sweep_t<1, false, 3>(a, blocks, th, smem, st);

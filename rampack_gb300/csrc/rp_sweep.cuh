@@ -111,6 +111,25 @@ __device__ __forceinline__ int seg_stage(const FilterConsts &fc, float3 d, float
     return (f + err < fc.core_thr && (par || s2 >= fc.s2_min)) ? 1 : 2;
 }
 
+// The segment stage of two centres of polyspherocylinders: segments b - a = d apart with half axes
+// ha and hb of any lengths (a zero one is a sphere), threshold thr = (r_a + r_b)^2; as seg_stage
+// with lam and mu in [-1, 1], an overlap of segments with |ha x hb|^2 below s2_min left to FP64.
+__device__ __forceinline__ int seg_stage_pair(const FilterConsts &fc, float thr, float3 d, float3 ha, float3 hb) {
+    const float aa = dot3f(ha, ha), bb = dot3f(hb, hb), c = dot3f(ha, hb), A = dot3f(d, ha), B = dot3f(d, hb);
+    const float3 cr = make_float3(fmaf(ha.y, hb.z, -ha.z * hb.y), fmaf(ha.z, hb.x, -ha.x * hb.z), fmaf(ha.x, hb.y, -ha.y * hb.x));
+    const float x = dot3f(cr, cr);
+    float lam = __fdividef(fmaf(A, bb, -c * B), fmaxf(x, 1e-18f));
+    lam = fminf(fmaxf(lam, -1.f), 1.f);
+    const float mu = fminf(fmaxf(__fdividef(fmaf(c, lam, -B), fmaxf(bb, 1e-18f)), -1.f), 1.f);
+    lam = fminf(fmaxf(__fdividef(fmaf(c, mu, A), fmaxf(aa, 1e-18f)), -1.f), 1.f);
+    const float3 dP = make_float3(fmaf(mu, hb.x, fmaf(-lam, ha.x, d.x)), fmaf(mu, hb.y, fmaf(-lam, ha.y, d.y)),
+                                  fmaf(mu, hb.z, fmaf(-lam, ha.z, d.z)));
+    const float f = dot3f(dP, dP), gs = dot3f(dP, ha), gt = dot3f(dP, hb);
+    const float G = 2.f * (fabsf(gs) + fabsf(gt) + fmaf(gt, mu, -gs * lam));
+    if (f - G - fc.seg_err >= thr) return 0;
+    return (f + fc.seg_err < thr && x >= fc.s2_min) ? 1 : 2;
+}
+
 // FP32 classification of one pair: 0 no overlap, 1 overlap, 2 undecided in FP32.
 template <int KIND>
 __device__ __forceinline__ int classify(const FilterConsts &fc, float3 d, float3 ai, float3 aj) {
@@ -237,7 +256,8 @@ constexpr int STAGE_WAIT_LIMIT = 1 << 21;
 // MODE 0: plain sweep; 1: learned-ordering pre-test and pair log; 2: overlap counting
 // (Packing::toggleOverlapCounting, core/Packing.cpp:304-323: the move's energy is the sign of
 // the change of the mover's overlap count).
-template <int KIND, bool LIST, int MODE, int GW = 32>
+// SEG: multi-centre bodies may be polyspherocylinders (false: spheres only, without their code).
+template <int KIND, bool LIST, int MODE, int GW = 32, bool SEG = true>
 __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, const int cell_direct, const int cap,
                                            int32_t *ovf, int32_t *ovf_count, float4 *cpos, float4 *cax,
                                            uint16_t *qseg, uint16_t *qun, uint8_t *nacc, uint16_t *pstage,
@@ -253,6 +273,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
     constexpr bool AXM = GW == 16 && KIND == 1;
     const unsigned lt = (1u << lane) - 1u;
     const DevState &S = A.s;
+    const bool segs = KIND == 2 && SEG && S.segs;
     const GridDev &G = A.g;
 
     // ---- which cell ----
@@ -401,11 +422,13 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
     // polyspheres: the warp's scratch holds the mover's FP32 centres (wx[0..K)), the
     // centre-pair thresholds (lo, hi) and the mover's exact new centres and absolute centres
     float *wthr = reinterpret_cast<float *>(wx + MAX_CEN);
-    double *wabs = reinterpret_cast<double *>(wx + MAX_CEN + MAX_CEN * MAX_CEN / 2);
+    double *wabs = reinterpret_cast<double *>(wx + MAX_CEN + 3 * MAX_CEN * MAX_CEN / 4);
     double *wcen = wabs + 3 * MAX_CEN;
     double *whax = wcen + 3 * MAX_CEN;   // polyspherocylinders: the mover's rotated half axes
+    float4 *wh = reinterpret_cast<float4 *>(whax + 3 * MAX_CEN);   // ... in FP32
+    uint32_t *wpq = reinterpret_cast<uint32_t *>(wh + MAX_CEN);    // centre pairs for the segment stage
     if (KIND == 2)
-        for (int t = lane; t < 2 * MAX_CEN * MAX_CEN; t += GW) wthr[t] = G.cthr[t];
+        for (int t = lane; t < 3 * MAX_CEN * MAX_CEN; t += GW) wthr[t] = G.cthr[t];
     const bool self_images = (G.dims[0] == 1) || (G.dims[1] == 1) || (G.dims[2] == 1);
     // per own-cell particle: FP32 roundings accumulated in its mirror position this sweep
     for (int k = lane; k < occ; k += GW) nacc[k] = 0;
@@ -555,6 +578,12 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 float3 cn = make_float3(c.x, c.y, c.z);
                 if (type != 0) cn = mat32(R32, cn.x, cn.y, cn.z);
                 wx[lane] = make_float4(cn.x, cn.y, cn.z, 0.f);
+                if (segs) {
+                    const float4 h = G.mhax[((size_t)gbase + slot) * S.ncen + lane];
+                    float3 hn = make_float3(h.x, h.y, h.z);
+                    if (type != 0) hn = mat32(R32, hn.x, hn.y, hn.z);
+                    wh[lane] = make_float4(hn.x, hn.y, hn.z, 0.f);
+                }
             }
             grp.sync();
         }
@@ -650,8 +679,64 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             }
         }
         grp.sync();
+        // ---- FP32 pass 2 (polyspherocylinders): the centre pairs of a near body, one body per lane;
+        //      pairs between the insphere and circumsphere thresholds are queued and their segments
+        //      decided 32 to a round (in FP64 those pairs bound the sweep: 25 against 8 ms for five
+        //      cycles of 10^5 bent rods) ----
+        bool unall = false;   // more undecided pairs than the queue holds: every near body in FP64
+        if (!COUNT && !LEARN && KIND == 2 && segs && !overlap) {
+            const int K = S.ncen;
+            int qp = 0;
+            auto segments = [&](int n) {
+                int cls = 0, k = 0;
+                if (lane < n) {
+                    const uint32_t e = wpq[qp - n + lane];
+                    k = (int)(e >> 6);
+                    const int a = (e >> 3) & 7, j = e & 7;
+                    const float4 q = cpos[k], m = wx[a], x = wh[a];
+                    const float4 c = G.mcen[(size_t)cslot[k] * K + j], y = G.mhax[(size_t)cslot[k] * K + j];
+                    cls = seg_stage_pair(S.fc, wthr[2 * MAX_CEN * MAX_CEN + a * MAX_CEN + j],
+                                         make_float3(q.x - pn.x + c.x - m.x, q.y - pn.y + c.y - m.y, q.z - pn.z + c.z - m.z),
+                                         make_float3(x.x, x.y, x.z), make_float3(y.x, y.y, y.z));
+                }
+                qp -= n;
+                if (grp.ballot(cls == 1)) overlap = true;
+                const unsigned b2 = grp.ballot(cls == 2);
+                if (nun + __popc(b2) > cap) unall = true;
+                else {
+                    if (cls == 2) qun[nun + __popc(b2 & lt)] = (uint16_t)k;
+                    nun += __popc(b2);
+                }
+                grp.sync();
+            };
+            for (int base = 0; base < nseg && !overlap; base += GW) {
+                const int i = base + lane;
+                const int k = i < nseg ? qseg[i] : 0;
+                const float4 q = cpos[k];
+                const float3 dq = make_float3(q.x - pn.x, q.y - pn.y, q.z - pn.z);
+                const float4 *cj = G.mcen + (size_t)cslot[k] * K;
+                bool hit = false;
+                for (int j = 0; j < K && !overlap; j++) {
+                    const float4 c = cj[j];
+                    for (int a = 0; a < K && !overlap; a++) {
+                        const float4 m = wx[a];
+                        const float3 d = make_float3(dq.x + c.x - m.x, dq.y + c.y - m.y, dq.z + c.z - m.z);
+                        const float d2 = dot3f(d, d);
+                        hit = hit || (i < nseg && d2 < wthr[a * MAX_CEN + j]);
+                        const bool band = i < nseg && !hit && d2 <= wthr[MAX_CEN * MAX_CEN + a * MAX_CEN + j];
+                        const unsigned bal = grp.ballot(band);
+                        if (band) wpq[qp + __popc(bal & lt)] = (uint32_t)(k << 6 | a << 3 | j);
+                        qp += __popc(bal);
+                        grp.sync();
+                        if (qp >= GW) segments(GW);
+                    }
+                }
+                if (grp.ballot(hit)) overlap = true;
+            }
+            if (!overlap && qp > 0) segments(qp);
+        }
         // ---- FP32 pass 2 (polyspheres): every centre pair of a near body, one body per lane ----
-        if (!COUNT && KIND == 2 && !overlap) {
+        if (!COUNT && KIND == 2 && (LEARN || !segs) && !overlap) {
             const int K = S.ncen;
             for (int base = 0; base < nseg; base += GW) {
                 const int i = base + lane;
@@ -895,7 +980,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                     wabs[3 * lane + 1] = a.y;
                     wabs[3 * lane + 2] = a.z;
                 }
-                if (S.segs) {
+                if (segs) {
                     // orientation * half axis with the mover's new orientation
                     // (PolyspherocylinderTraits.cpp:118-119)
                     const double oe = type != 0 ? onew_own : rot_own;
@@ -911,7 +996,9 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 grp.sync();
             }
             // the guard band: queued pairs re-decided in FP64
-            if (KIND == 2 && code == 0 && nun > 0) {
+            if (KIND == 2 && code == 0 && (nun > 0 || unall)) {
+                const uint16_t *uq = unall ? qseg : qun;
+                const int nu = unall ? nseg : nun;
                 // every centre pair of the queued bodies, one pair per lane: with K^2 <= 16,
                 // 32 / K^2 bodies per pass (the FP64 segment tests of polyspherocylinders
                 // keep the lanes busy), else one body per pass
@@ -919,16 +1006,16 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 const int KK = K * K;
                 const int per = KK <= GW / 2 ? GW / KK : 1;
                 bool ov = false;
-                for (int q0 = 0; q0 < nun && !ov; q0 += per) {
+                for (int q0 = 0; q0 < nu && !ov; q0 += per) {
                     const int qi = q0 + (per > 1 ? lane / KK : 0);
-                    const int k = qun[qi < nun ? qi : q0];
+                    const int k = uq[qi < nu ? qi : q0];
                     const float4 q = cpos[k];
                     const float3 dq = make_float3(q.x - pn.x, q.y - pn.y, q.z - pn.z);
                     const float4 *cj = G.mcen + (size_t)cslot[k] * K;
                     for (int tb = 0; tb < (per > 1 ? 1 : KK); tb += GW) {
                         const int t = per > 1 ? lane % KK : tb + lane;
                         bool hit = false;
-                        if (t < KK && qi < nun && (per == 1 || lane < per * KK)) {
+                        if (t < KK && qi < nu && (per == 1 || lane < per * KK)) {
                             const int a = t / K, j = t % K;
                             const float4 m = wx[a];
                             const float4 c = cj[j];
@@ -943,7 +1030,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                         }
                     }
                 }
-                ws.fp64 += nun;
+                ws.fp64 += nu;
                 if (ov) code = 1;
             }
             if (KIND != 2 && code == 0 && nun > 0) {
@@ -972,7 +1059,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 if (lane == 0)
                     wov = wall_overlap_count(S.walls, S.wall_vec, S.wall_far, S.wall_half, KIND, S.wall_radius,
                                              S.wall_half_len, pnew, anew, KIND == 2 ? wcen : nullptr,
-                                             KIND == 2 ? S.ncen : 0, true, KIND == 2 && S.segs ? whax : nullptr);
+                                             KIND == 2 ? S.ncen : 0, true, KIND == 2 && segs ? whax : nullptr);
                 if (grp.shfl(wov, 0)) code = 1;
             }
         }
@@ -1005,9 +1092,17 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                             const float3 d0 = make_float3((db.x + c.x) - m0.x, (db.y + c.y) - m0.y, (db.z + c.z) - m0.z);
                             const float q0 = dot3f(d0, d0);
                             int cb = exact ? 2 : (q0 < lo ? 1 : (q0 <= hi ? 2 : 0));
+                            const float cthr = wthr[2 * MAX_CEN * MAX_CEN + a * MAX_CEN + j];
+                            float4 hj = make_float4(0.f, 0.f, 0.f, 0.f);
+                            if (segs && !exact) {
+                                hj = G.mhax[(size_t)cslot[k] * K + j];
+                                const float4 x = G.mhax[((size_t)gbase + slot) * K + a];
+                                if (cb == 2)
+                                    cb = seg_stage_pair(S.fc, cthr, d0, make_float3(x.x, x.y, x.z), make_float3(hj.x, hj.y, hj.z));
+                            }
                             if (cb == 2) {
                                 d3 h0{0.0, 0.0, 0.0};
-                                if (S.segs)
+                                if (segs)
                                     h0 = mv3(S.rot64 + 9 * (size_t)pid, d3{S.chax[a][0], S.chax[a][1], S.chax[a][2]});
                                 cb = exact_centre_pair(S, load_d3(S.abs64 + 3 * ((size_t)pid * K + a)), a, pj, j, d0,
                                                        h0) ? 1 : 0;
@@ -1016,6 +1111,10 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                             const float3 d1 = make_float3((da.x + c.x) - m1.x, (da.y + c.y) - m1.y, (da.z + c.z) - m1.z);
                             const float q1 = dot3f(d1, d1);
                             int ca = exact ? 2 : (q1 < lo ? 1 : (q1 <= hi ? 2 : 0));
+                            if (segs && !exact && ca == 2) {
+                                const float4 x = wh[a];
+                                ca = seg_stage_pair(S.fc, cthr, d1, make_float3(x.x, x.y, x.z), make_float3(hj.x, hj.y, hj.z));
+                            }
                             if (ca == 2)
                                 ca = exact_centre_pair(S, d3{wabs[3 * a], wabs[3 * a + 1], wabs[3 * a + 2]}, a, pj, j, d1,
                                                        d3{whax[3 * a], whax[3 * a + 1], whax[3 * a + 2]}) ? 1 : 0;
@@ -1026,16 +1125,16 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 }
                 if (S.walls && lane == 0) {
                     double hcur[3 * MAX_CEN];
-                    if (S.segs)
+                    if (segs)
                         for (int a = 0; a < K; a++) {
                             d3 h = mv3(S.rot64 + 9 * (size_t)pid, d3{S.chax[a][0], S.chax[a][1], S.chax[a][2]});
                             hcur[3 * a] = h.x, hcur[3 * a + 1] = h.y, hcur[3 * a + 2] = h.z;
                         }
                     before += wall_overlap_count(S.walls, S.wall_vec, S.wall_far, S.wall_half, 2, S.wall_radius, 0.0,
                                                  pc64, ac64, S.cen64 + 3 * (size_t)pid * K, K, false,
-                                                 S.segs ? hcur : nullptr);
+                                                 segs ? hcur : nullptr);
                     after += wall_overlap_count(S.walls, S.wall_vec, S.wall_far, S.wall_half, 2, S.wall_radius, 0.0,
-                                                pnew, anew, wcen, K, false, S.segs ? whax : nullptr);
+                                                pnew, anew, wcen, K, false, segs ? whax : nullptr);
                 }
             }
             for (int k = lane; k < (KIND == 2 ? 0 : total); k += GW) {
@@ -1125,6 +1224,9 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                     const float4 c32 = make_float4((float)wcen[3 * lane], (float)wcen[3 * lane + 1],
                                                    (float)wcen[3 * lane + 2], 0.f);
                     G.mcen[gslot * S.ncen + lane] = c32;
+                    if (segs)
+                        G.mhax[gslot * S.ncen + lane] = make_float4((float)whax[3 * lane], (float)whax[3 * lane + 1],
+                                                                    (float)whax[3 * lane + 2], 0.f);
                 }
             }
             if (self_images) {
@@ -1260,6 +1362,11 @@ __device__ __forceinline__ void finish_one(const DevState &s, const GridDev &g, 
             const double *c = s.cen64 + 3 * ((size_t)pid * s.ncen + b);
             g.mcen[(size_t)k * s.ncen + b] =
                 make_float4(static_cast<float>(c[0]), static_cast<float>(c[1]), static_cast<float>(c[2]), 0.f);
+            if (s.segs) {
+                const d3 h = mv3(r, d3{s.chax[b][0], s.chax[b][1], s.chax[b][2]});
+                g.mhax[(size_t)k * s.ncen + b] =
+                    make_float4(static_cast<float>(h.x), static_cast<float>(h.y), static_cast<float>(h.z), 0.f);
+            }
         }
     }
 }
@@ -1383,7 +1490,14 @@ __device__ __forceinline__ int count_pair(const DevState &s, const GridDev &g, i
             const float d2 = dot3f(e, e);
             const bool exact = s.pbc_fold == 2;
             bool ov = !exact && d2 < g.cthr[a * MAX_CEN + j];
-            if (!ov && (exact || d2 <= g.cthr[MAX_CEN * MAX_CEN + a * MAX_CEN + j])) {
+            int cls = ov ? 1 : ((exact || d2 <= g.cthr[MAX_CEN * MAX_CEN + a * MAX_CEN + j]) ? 2 : 0);
+            if (cls == 2 && s.segs && !exact) {
+                const float4 x = g.mhax[(size_t)sa * K + a], y = g.mhax[(size_t)sb * K + j];
+                cls = seg_stage_pair(s.fc, g.cthr[2 * MAX_CEN * MAX_CEN + a * MAX_CEN + j], e, make_float3(x.x, x.y, x.z),
+                                     make_float3(y.x, y.y, y.z));
+                ov = cls == 1;
+            }
+            if (cls == 2) {
                 n64++;
                 if (s.cq_buf) {
                     const int qi = atomicAdd(s.cq_count, 1);

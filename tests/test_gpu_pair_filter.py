@@ -75,3 +75,33 @@ def test_multi_centre_counts(oracle, engine, walls):
     assert counts(W.POLYSPHEROCYLINDER, W.polyspherocylinder_params(W.BENT_ROD), pos, rot, box, walls) > 0
     chain = W.polysphere_params(W.banana_centres(1.16, 2.0, 5), 0.5)
     assert counts(W.POLYSPHERE, chain, pos, rot, box, walls) > 0
+
+
+@pytest.mark.parametrize("counting", [False, True])
+def test_unequal_segments_replay(oracle, engine, counting):
+    """Sweeps of bodies whose segments differ in length and radius (one a sphere), from an aligned
+    lattice on: every logged move replays on the oracle, and so do the counts of random states."""
+    from rampack_gb300.packing import GpuPacking
+    data = ((-0.4, 0.0, 0.0, 0.3, 0.0, 0.2, 0.25), (0.3, 0.0, 0.1, 0.0, 0.0, 0.0, 0.35), (0.0, 0.3, 0.0, 0.0, 0.5, 0.0, 0.15))
+    prm = W.polyspherocylinder_params(data)
+    pos = W.lattice((5, 6, 7), (1.75, 1.6, 1.2))
+    box = W.diag_box(8.75, 9.6, 8.4)
+    rot = W.aligned_rotations(len(pos))
+    if counting:
+        rng = np.random.default_rng(3)
+        rot = rotations(rng, len(pos), None)
+        assert counts(W.POLYSPHEROCYLINDER, prm, pos, rot, box) > 0
+    cpu = po.CpuPacking("oracle", W.POLYSPHEROCYLINDER, prm, pos, rot, box, threads=1)
+    with GpuPacking(W.POLYSPHEROCYLINDER, prm, pos, rot, box) as g:
+        if counting:
+            cpu.set_counting(True)
+            g.set_counting(True)
+        for cycle in range(4):
+            st = g.sweep(0.2, 0.4, seed=5, counter=cycle, log=True)
+            moves, codes = g.sweep_log()
+            want, _ = cpu.replay(moves, g.grid()[2])
+            assert np.array_equal(codes, want), (cycle, np.count_nonzero(codes != want))
+            assert 0 < st["accepted"] < st["moves"]
+        gp, gr, _ = g.state()
+        cp, cr, _ = cpu.state()
+        assert np.array_equal(gp, cp) and np.array_equal(gr, cr)
