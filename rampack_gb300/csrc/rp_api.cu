@@ -509,6 +509,18 @@ DevState dev_state(Handle *h) {
         fc.far_hi = static_cast<float>(far + poly_margin(h, g, far));
         if (h->segs) poly_segment_consts(h, g, fc);
     }
+    if (h->soft) {
+        // FP32 separations err by 32 u32 (L + 1) per component (hard_filter_consts), doubled for safety
+        const double delta = 2.0 * std::sqrt(3.0) * 32.0 * std::ldexp(1.0, -24) * (cell_lrow(g) + 1.0);
+        const double cut = h->soft == RP_SOFT_REPULSIVE_LJ ? h->soft_cut : h->soft_sigma;
+        fc.soft_delta = static_cast<float>(delta);
+        fc.soft_sigma2 = static_cast<float>(h->soft_sigma * h->soft_sigma);
+        fc.soft_cut2 = static_cast<float>(cut * cut);
+        fc.soft_reach2 = static_cast<float>((cut + 2 * delta) * (cut + 2 * delta) * (1.0 + 1e-3));
+        fc.soft_4eps = static_cast<float>(4.0 * h->soft_eps);
+        fc.soft_eps = static_cast<float>(h->soft_eps);
+        fc.soft_floor = static_cast<float>(1e-6 * std::fabs(h->soft_eps));
+    }
     s.fc = fc;
     return s;
 }
@@ -1746,7 +1758,14 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         if (rc2) return rc2;
     }
     h->since_rank++;
-    const bool fp64_sweep = h->soft || h->shape.kind == RP_SHAPE_CONVEX;
+    // spheres with a soft part take the FP32 sweep with an error bound on the energy change, over a
+    // grid where a staged candidate is one image of another particle
+    const bool soft32 = h->soft && h->shape.kind == RP_SHAPE_SPHERE && !h->counting && !(p->flags & RP_SWEEP_FP64_ONLY) &&
+                        !h->grid[h->gcur].no_ng && g.dims[0] >= 3 && g.dims[1] >= 3 && g.dims[2] >= 3 &&
+                        (h->soft_only || !h->walls);
+    const bool fp64_sweep = (h->soft && !soft32) || h->shape.kind == RP_SHAPE_CONVEX;
+    if (soft32 && types == SWEEP_ROTOTRANSLATION)
+        return fail(h, RP_ERR_UNSUPPORTED, "rototranslations with a soft part or a convex body");
     if (fp64_sweep) {
         // a soft part or a generic convex body: every move decided in FP64 (hard part, then the
         // energy change with the Metropolis test at the handle's temperature), one warp per
@@ -1794,8 +1813,13 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     if (ordered) order_starts(g, order_start);
     for (int ph : (fp64_sweep ? std::vector<int>{} : phases)) {
         SweepArgs a = base_args(h);
-        if (h->order_mode != RP_ORDER_OFF) a.partners = h->partners;
-        if (h->pair_cap > 0) {
+        if (h->order_mode != RP_ORDER_OFF && !soft32) a.partners = h->partners;
+        if (soft32) {
+            a.soft32 = 1;
+            a.temperature = h->temperature;
+            a.inv_temp = static_cast<float>(1.0 / h->temperature);
+        }
+        if (h->pair_cap > 0 && !soft32) {
             a.pair_feats = h->pair_feats;
             a.pair_labels = h->pair_labels;
             a.pair_count = h->pair_count;
@@ -1830,7 +1854,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         }
         // two cells per warp for the plain scans of spheres and spherocylinders
         const GridHost &gh = h->grid[h->gcur];
-        const bool half = h->cells_per_warp == 2 && gh.cap_half > 0 && !h->counting && types != SWEEP_ROTOTRANSLATION &&
+        const bool half = h->cells_per_warp == 2 && gh.cap_half > 0 && !h->counting && !soft32 && types != SWEEP_ROTOTRANSLATION &&
                           a.partners == nullptr && a.pair_every == 0;
         if (half && h->half_cap_cached != gh.cap_half) {
             h->half_blocks = sweep_half_blocks_per_sm(h->shape.kind, gh.cap_half);

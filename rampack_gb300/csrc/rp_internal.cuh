@@ -39,6 +39,9 @@ struct FilterConsts {
     float par_err;                // bound on that branch's excess over the true minimum
     float half_len;               // l / 2
     float cell_margin;            // relative in-cell margin of the FP32 ActiveDomain test
+    // soft part: bound of an FP32 separation's error, sigma^2, cut-off^2, the reach^2 of pairs to
+    // evaluate (cut-off^2 and a margin), 4 eps and eps, an energy error floor per move
+    float soft_delta, soft_sigma2, soft_cut2, soft_reach2, soft_4eps, soft_eps, soft_floor;
 };
 
 // One checkerboard cell grid with its cell list and FP32 mirror in cell order.
@@ -232,6 +235,9 @@ struct SweepArgs {
     rp_move *log;                  // [ntypes * n] indexed by ntypes * start[cell] + k
     uint8_t *log_codes;
     int fp64_only;
+    int soft32;                    // spheres with a soft part: energies in FP32 with error bounds, FP64 where unsure
+    double temperature;            // their Metropolis temperature, and its reciprocal
+    float inv_temp;
     int bulk_stage;                // stage neighbourhoods with bulk asynchronous copies (one per cell and array)
     // overflow: cells whose neighbourhood exceeds cap are appended here and rerun
     int32_t *overflow;             // [ncell]

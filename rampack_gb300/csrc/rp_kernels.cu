@@ -531,6 +531,7 @@ cudaError_t launch_sweep(const SweepArgs &a, bool list, int nwarps, cudaStream_t
              : a.s.segs ? launch_sweep_t<2, false, 0>(a, blocks, th, smem, st)
                         : launch_sweep_t<2, false, 0, 32, false>(a, blocks, th, smem, st);
     }
+    if (a.soft32) return launch_sweep_t<0, false, 4>(a, blocks, th, smem, st);
     if (rt) return a.s.kind == 0 ? launch_sweep_t<0, false, 3>(a, blocks, th, smem, st)
                                  : launch_sweep_t<1, false, 3>(a, blocks, th, smem, st);
     if (a.s.kind == 0) {

@@ -74,24 +74,6 @@ __device__ int neighbour_cells(const GridDev &g, const int c[3], int *out) {
     return k;
 }
 
-// CentralInteraction::calculateEnergyForDistance2 of the soft part, in the reference's
-// operation order: RepulsiveLennardJonesInteraction.cpp:9-17, SquareInverseCoreInteraction.cpp:13-15.
-// (cut^2, sigma^2 and 4 eps are the host's products of the same operands, identical roundings).
-__device__ double soft_energy(const DevState &s, double d2) {
-    if (s.soft == 1) {
-        if (d2 >= s.soft_cut2) return 0.0;
-        const double x2 = ddiv(s.soft_sigma2, d2);
-        const double x6 = dmul(dmul(x2, x2), x2);
-        const double x12 = dmul(x6, x6);
-        return dadd(dmul(s.soft_4eps, dsub(x12, x6)), s.soft_eps);
-    }
-    if (s.soft == 2) {
-        const double v = dsub(ddiv(s.soft_sigma2, d2), 1.0);
-        return dmul(s.soft_eps, 0.0 < v ? v : 0.0);  // std::max(0.0, v)
-    }
-    return 0.0;
-}
-
 // Pair test of a sphere, spherocylinder or generic convex mover (position p, axis a,
 // orientation rot) against particle j at translation t (null: no grid in the reference, the
 // periodic boundary conditions' nearest image), SphereTraits.cpp:56-65 /
@@ -631,33 +613,6 @@ __global__ void k_commit_single(DevState s, SingleTry *t, uint8_t *disp_flag, in
 
 // ---- soft sweeps ----------------------------------------------------------------------
 
-// Metropolis acceptance u <= exp(-dE / T) (core/Simulation.cpp:483) for the sweep's own
-// uniforms (multiples of 2^-53 in [0, 1)) and T > 0, without the FP64 exponential where the
-// answer is certain: dE <= 0 accepts (exp >= 1 > u); an exponent below -80 accepts only u = 0
-// (exp < 2e-35 below the smallest positive u); otherwise CUDA's FP32 expf decides wherever u
-// lies more than 1e-4 (relative) away from it, far beyond the FP32 errors of the exponent
-// (< 5e-6 relative at |x| <= 80), of expf (a few ulp) and of u; the band in between, and a NaN,
-// take the FP64 exponential.  The decision is that of the FP64 test in every case.
-__device__ __forceinline__ bool metropolis(double u, double dE, double T) {
-    if (dE <= 0.0) return true;
-    const double x = T == 1.0 ? -dE : -dE / T;   // a division by one is exact
-    if (x < -80.0) return u == 0.0;
-    const float ef = expf(static_cast<float>(x)), uf = static_cast<float>(u);
-    if (uf <= ef * (1.0f - 1e-4f)) return true;
-    if (uf >= ef * (1.0f + 1e-4f)) return false;
-    return u <= exp(x);
-}
-
-// The Metropolis uniform of move mi of a cell: 53 bits of a Philox draw apart from the
-// proposal's words.
-__device__ double soft_uniform(const SoftSweepArgs &A, int cell, int mi) {
-    const u4 q = philox(u4{(uint32_t)mi, (uint32_t)cell, (uint32_t)A.counter, (uint32_t)(A.counter >> 32) ^ 0x2545f491u},
-                        (uint32_t)A.seed ^ 0x9e3779b9u, (uint32_t)(A.seed >> 32));
-    // (a >> 5) * 2^26 + (b >> 6) is an integer below 2^53: formed exactly as one, then scaled
-    const uint64_t k = (static_cast<uint64_t>(q.a >> 5) << 26) | static_cast<uint64_t>(q.b >> 6);
-    return static_cast<double>(k) * (1.0 / 9007199254740992.0);
-}
-
 template <int KIND>
 __global__ void __launch_bounds__(SOFT_WARPS * 32, 4) k_soft_sweep(SoftSweepArgs A) {
     __shared__ Mover movers[SOFT_WARPS];
@@ -713,7 +668,7 @@ __global__ void __launch_bounds__(SOFT_WARPS * 32, 4) k_soft_sweep(SoftSweepArgs
             const int type = ntypes == 2 ? ((r.a >> 31) ? 1 : 0) : ((A.types & 1) ? 0 : 1);
             const int slot = (int)(((uint64_t)(r.a & 0x7fffffffu) * (uint32_t)occ) >> 31);
             const int pid = G.slot_pid[gbase + slot];
-            const double uni = soft_uniform(A, cell, mi);
+            const double uni = static_cast<double>(soft_uniform_bits(A.seed, A.counter, cell, mi)) * (1.0 / 9007199254740992.0);
             if (lane == 0) {
                 // the proposal: a translation uniform in the cube of the step (an FP32 value, exact
                 // as FP64), or a rotation of this sweep's table or its transpose
@@ -781,6 +736,77 @@ __global__ void __launch_bounds__(SOFT_WARPS * 32, 4) k_soft_sweep(SoftSweepArgs
 }
 
 // ---- total soft energy ----------------------------------------------------------------
+
+// Packing::getTotalEnergy of single-centre bodies over a grid of at least three cells a side: a warp
+// takes 32 slots, lane by lane walks the particles of the 27 cells in the FP32 mirror, queues the
+// pairs (j > i) within the soft range plus a margin, and evaluates 32 of them at a time in FP64 at
+// the image of their FP32 separation; one sum per block, in a fixed order.  (One thread per
+// particle over FP64 positions took 0.25 ms for 97,336 spheres, bound by FP64 differences of pairs
+// out of range and by energies on a few lanes.)
+constexpr int ENERGY_WARPS = 4;
+__global__ void __launch_bounds__(ENERGY_WARPS * 32) k_mirror_energies(DevState s, GridDev g, double *out) {
+    __shared__ uint32_t queue[ENERGY_WARPS][64];
+    __shared__ int2 pair[ENERGY_WARPS][64];
+    __shared__ double part[ENERGY_WARPS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int64_t slot = (blockIdx.x * (int64_t)ENERGY_WARPS + w) * 32 + lane;
+    const bool in = slot < s.n;
+    const float4 p = in ? g.mpos[slot] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int pid = __float_as_int(p.w);
+    const int cell = in ? g.pid_cell[pid] : 0;
+    const int cx = cell % g.dims[0], cy = (cell / g.dims[0]) % g.dims[1], cz = cell / (g.dims[0] * g.dims[1]);
+    const float reach = s.fc.soft_reach2;
+    const unsigned lt = (1u << lane) - 1u;
+    double e = 0.0;
+    int qn = 0;
+    auto evaluate = [&](int n) {
+        if (lane < n) {
+            const int2 ij = pair[w][qn - n + lane];
+            const int o = (int)queue[w][qn - n + lane];
+            const float4 a = g.mpos[ij.x], b = g.mpos[ij.y];
+            const float3 off = mat32(g.cellmat, (float)(o % 3 - 1), (float)((o / 3) % 3 - 1), (float)(o / 9 - 1));
+            const d3 pa = load_d3(s.pos64 + 3 * (size_t)__float_as_int(a.w)), pb = load_d3(s.pos64 + 3 * (size_t)__float_as_int(b.w));
+            const int m = image_index(s, make_float3(b.x + off.x - a.x, b.y + off.y - a.y, b.z + off.z - a.z), pa, pb);
+            e = dadd(e, soft_energy(s, norm2(sub3(add3(pb, load_d3(s.trans + 3 * m)), pa))));
+        }
+        qn -= n;
+        __syncwarp();
+    };
+    for (int o = 0; o < 27; o++) {
+        const int ox = o % 3 - 1, oy = (o / 3) % 3 - 1, oz = o / 9 - 1;
+        const int nb = wrap_cell(cx + ox, g.dims[0]) +
+                       g.dims[0] * (wrap_cell(cy + oy, g.dims[1]) + g.dims[1] * wrap_cell(cz + oz, g.dims[2]));
+        const float3 off = mat32(g.cellmat, (float)ox, (float)oy, (float)oz);
+        const int b = g.start[nb], cnt = in ? g.start[nb + 1] - b : 0;
+        const int most = __reduce_max_sync(FULL, cnt);
+        for (int k = 0; k < most; k++) {
+            bool near = false;
+            if (k < cnt) {
+                const float4 q = g.mpos[b + k];
+                const float dx = q.x + off.x - p.x, dy = q.y + off.y - p.y, dz = q.z + off.z - p.z;
+                near = __float_as_int(q.w) > pid && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= reach;
+            }
+            const unsigned bal = __ballot_sync(FULL, near);
+            if (!bal) continue;
+            if (near) {
+                pair[w][qn + __popc(bal & lt)] = make_int2((int)slot, b + k);
+                queue[w][qn + __popc(bal & lt)] = (uint32_t)o;
+            }
+            qn += __popc(bal);
+            __syncwarp();
+            if (qn >= 32) evaluate(32);
+        }
+    }
+    if (qn > 0) evaluate(qn);
+    for (int d = 16; d > 0; d >>= 1) e = dadd(e, __shfl_xor_sync(FULL, e, d));
+    if (lane == 0) part[w] = e;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int k = 0; k < ENERGY_WARPS; k++) t = dadd(t, part[k]);
+        out[blockIdx.x] = t;
+    }
+}
 
 // Per particle i: its pairs with every j > i at every image within reach (each unordered pair
 // once, as Packing::getTotalEnergy sums them); the grid current for every particle.
@@ -921,6 +947,12 @@ cudaError_t launch_count_fp64(const SingleArgs &a, int early, unsigned long long
 // fixed-order sum.
 cudaError_t launch_total_energy(const SingleArgs &a, double *scratch, double *out, cudaStream_t st) {
     const unsigned nb = (unsigned)((a.s.n + 127) / 128);
+    if (a.s.kind != 2 && !a.s.pbc_fold && a.g.dims[0] >= 3 && a.g.dims[1] >= 3 && a.g.dims[2] >= 3) {
+        static_assert(ENERGY_WARPS * 32 == 128, "a block per 128 slots");
+        k_mirror_energies<<<nb, ENERGY_WARPS * 32, 0, st>>>(a.s, a.g, scratch);
+        k_sum_fixed<<<1, 1024, 0, st>>>(scratch, nb, out);
+        return cudaGetLastError();
+    }
     if (a.s.kind == 0) k_pair_energies<0><<<nb, 128, 0, st>>>(a, scratch);
     else if (a.s.kind == 1) k_pair_energies<1><<<nb, 128, 0, st>>>(a, scratch);
     else k_pair_energies<2><<<nb, 128, 0, st>>>(a, scratch);

@@ -230,6 +230,69 @@ __device__ __forceinline__ bool exact_centre_pair(const DevState &s, d3 pa, int 
     return norm2(d) < s.cthr64[a * MAX_CEN + j];
 }
 
+// CentralInteraction::calculateEnergyForDistance2 of the soft part, in the reference's
+// operation order: RepulsiveLennardJonesInteraction.cpp:9-17, SquareInverseCoreInteraction.cpp:13-15.
+// (cut^2, sigma^2 and 4 eps are the host's products of the same operands, identical roundings).
+__device__ __forceinline__ double soft_energy(const DevState &s, double d2) {
+    if (s.soft == 1) {
+        if (d2 >= s.soft_cut2) return 0.0;
+        const double x2 = ddiv(s.soft_sigma2, d2);
+        const double x6 = dmul(dmul(x2, x2), x2);
+        const double x12 = dmul(x6, x6);
+        return dadd(dmul(s.soft_4eps, dsub(x12, x6)), s.soft_eps);
+    }
+    if (s.soft == 2) {
+        const double v = dsub(ddiv(s.soft_sigma2, d2), 1.0);
+        return dmul(s.soft_eps, 0.0 < v ? v : 0.0);  // std::max(0.0, v)
+    }
+    return 0.0;
+}
+
+// Metropolis acceptance u <= exp(-dE / T) (core/Simulation.cpp:483) for the sweep's own
+// uniforms (multiples of 2^-53 in [0, 1)) and T > 0, without the FP64 exponential where the
+// answer is certain: dE <= 0 accepts (exp >= 1 > u); an exponent below -80 accepts only u = 0
+// (exp < 2e-35 below the smallest positive u); otherwise CUDA's FP32 expf decides wherever u
+// lies more than 1e-4 (relative) away from it, far beyond the FP32 errors of the exponent
+// (< 5e-6 relative at |x| <= 80), of expf (a few ulp) and of u; the band in between, and a NaN,
+// take the FP64 exponential.  The decision is that of the FP64 test in every case.
+__device__ __forceinline__ bool metropolis(double u, double dE, double T) {
+    if (dE <= 0.0) return true;
+    const double x = T == 1.0 ? -dE : -dE / T;   // a division by one is exact
+    if (x < -80.0) return u == 0.0;
+    const float ef = expf(static_cast<float>(x)), uf = static_cast<float>(u);
+    if (uf <= ef * (1.0f - 1e-4f)) return true;
+    if (uf >= ef * (1.0f + 1e-4f)) return false;
+    return u <= exp(x);
+}
+
+// The 53 random bits of the Metropolis uniform of move mi of a cell (a Philox draw apart from the
+// proposal's words): (a >> 5) * 2^26 + (b >> 6), an integer below 2^53 to be scaled by 2^-53.
+__device__ __forceinline__ uint64_t soft_uniform_bits(uint64_t seed, uint64_t counter, int cell, int mi) {
+    const u4 q = philox(u4{(uint32_t)mi, (uint32_t)cell, (uint32_t)counter, (uint32_t)(counter >> 32) ^ 0x2545f491u},
+                        (uint32_t)seed ^ 0x9e3779b9u, (uint32_t)(seed >> 32));
+    return (static_cast<uint64_t>(q.a >> 5) << 26) | static_cast<uint64_t>(q.b >> 6);
+}
+
+// The soft energy at FP32 squared distance d2 and a bound of its error against the FP64 value at
+// the true distance: d2 is off by at most a relative 2 delta / d + (delta / d)^2 + 6 u32 (delta =
+// fc.soft_delta bounds the FP32 separation), times the potential's logarithmic slope (at most 6
+// on the repulsive Lennard-Jones' x^6 term, x = sigma^2 / d^2; 1 for the square inverse core), plus
+// the roundings of the evaluation.
+__device__ __forceinline__ void soft_energy32(const FilterConsts &fc, int kind, float d2, float &v, float &err) {
+    v = err = 0.f;
+    if (d2 >= fc.soft_reach2) return;
+    const float inv = __fdividef(1.f, d2), dd = fc.soft_delta * rsqrtf(d2);
+    const float rel = fmaf(dd, dd, fmaf(2.f, dd, 4e-7f)), x = fc.soft_sigma2 * inv;
+    if (kind == 1) {
+        const float x3 = x * x * x, x6 = x3 * x3;
+        if (d2 < fc.soft_cut2) v = fmaf(fc.soft_4eps, x6 - x3, fc.soft_eps);
+        err = fc.soft_4eps * fmaf(6.f * x6, rel, 1e-6f * (x6 + x3));
+    } else {
+        v = fc.soft_eps * fmaxf(x - 1.f, 0.f);
+        err = fabsf(fc.soft_eps) * x * (rel + 1e-6f);
+    }
+}
+
 // ---------------------------------------------------------------------------------
 // Checkerboard sweep: one warp per active cell.
 //
@@ -255,7 +318,8 @@ constexpr int STAGE_WAIT_LIMIT = 1 << 21;
 
 // MODE 0: plain sweep; 1: learned-ordering pre-test and pair log; 2: overlap counting
 // (Packing::toggleOverlapCounting, core/Packing.cpp:304-323: the move's energy is the sign of
-// the change of the mover's overlap count).
+// the change of the mover's overlap count); 3: rototranslations; 4: spheres with a soft part (the
+// energy change in FP32 with an error bound, FP64 where the Metropolis test is not certain).
 // SEG: multi-centre bodies may be polyspherocylinders (false: spheres only, without their code).
 template <int KIND, bool LIST, int MODE, int GW = 32, bool SEG = true>
 __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, const int cell_direct, const int cap,
@@ -264,6 +328,8 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                                            uint32_t *cslot, float4 *wx, WarpStats &ws) {
     constexpr bool LEARN = MODE == 1;
     constexpr bool COUNT = MODE == 2;
+    constexpr bool SOFT = MODE == 4;
+    static_assert(!SOFT || (KIND == 0 && !LIST), "soft sweeps of spheres");
     constexpr bool RT = MODE == 3;  // every move a rototranslation (the plain scan otherwise)
     const Grp<GW> grp;
     const int lane = grp.lane;
@@ -482,6 +548,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
     const int ntypes = sweep_move_types(A.types);
 
     u4 rnd_lane = u4{0u, 0u, 0u, 0u};  // Philox output of move (batch base + lane)
+    uint64_t uni_lane = 0;             // soft sweeps: the bits of its Metropolis uniform
     for (int mi = 0; mi < nmoves; mi++) {
         if (!LIST && (mi & (GW - 1)) == 0) {
             // draw the next GW moves' random words at once, one move per lane (the words
@@ -489,6 +556,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             rnd_lane = philox(u4{(uint32_t)(mi + lane), (uint32_t)cell, (uint32_t)A.counter,
                                  (uint32_t)(A.counter >> 32)},
                               (uint32_t)A.seed, (uint32_t)(A.seed >> 32));
+            if (SOFT) uni_lane = soft_uniform_bits(A.seed, A.counter, cell, mi + lane);
         }
         // ---- the proposal (FP32 view; FP64 inputs kept for the exact path) ----
         int type, slot = -1, out_index = -1;
@@ -528,6 +596,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             const int src = mi & (GW - 1);
             u4 r = u4{grp.shfl(rnd_lane.a, src), grp.shfl(rnd_lane.b, src),
                       grp.shfl(rnd_lane.c, src), grp.shfl(rnd_lane.d, src)};
+            if (SOFT) uni = static_cast<double>(grp.shfl(uni_lane, src)) * (1.0 / 9007199254740992.0);
             const bool rt = RT || (COUNT && A.types == SWEEP_ROTOTRANSLATION);
             if (rt) type = 2;
             else if (ntypes == 2) type = (r.a >> 31) ? 1 : 0;
@@ -641,7 +710,56 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         // ---- FP32 pass 1: centre distances, SWEEP_P1 candidates per lane per round (independent
         //      tests in flight), queued in candidate order ----
         int nseg = 0, nun = 0;
-        if (!COUNT && dom != 1 && !overlap) {
+        int soft = 1;   // soft sweeps: 1 accepted, 0 rejected by the energy, 2 left to FP64
+        if (SOFT && dom != 1) {
+            float de = 0.f, er = 0.f;
+            bool hit = false;
+            for (int base = 0; base < total; base += GW) {
+                const int k = base + lane;
+                int cls = 0;
+                if (k < total) {
+                    const float4 q = cpos[k];
+                    if (__float_as_int(q.w) != pid) {
+                        const float ax = q.x - pn.x, ay = q.y - pn.y, az = q.z - pn.z;
+                        const float a2 = fmaf(ax, ax, fmaf(ay, ay, az * az));
+                        if (!S.soft_only) cls = d2_stage<0>(S.fc, a2);
+                        if (type != 1) {
+                            const float bx = q.x - pcur.x, by = q.y - pcur.y, bz = q.z - pcur.z;
+                            float v0, e0, v1, e1;
+                            soft_energy32(S.fc, S.soft, fmaf(bx, bx, fmaf(by, by, bz * bz)), v0, e0);
+                            soft_energy32(S.fc, S.soft, a2, v1, e1);
+                            de += v1 - v0;
+                            er += (e0 + e1) + 1e-6f * (fabsf(v0) + fabsf(v1));
+                        }
+                    }
+                }
+                hit = hit || cls == 1;
+                if (!S.soft_only) {
+                    const unsigned bu = grp.ballot(cls == 2);
+                    if (cls == 2) qun[nun + __popc(bu & lt)] = (uint16_t)k;
+                    nun += __popc(bu);
+                }
+            }
+            if (lane == 0) ws.pairs += (unsigned)total;
+            overlap = grp.ballot(hit) != 0;
+            if (!overlap && type != 1) {
+#pragma unroll
+                for (int d = GW / 2; d > 0; d >>= 1) {
+                    de += grp.shfl_xor(de, d);
+                    er += grp.shfl_xor(er, d);
+                }
+                er = fmaf(2.f, er, S.fc.soft_floor);
+                // Metropolis (core/Simulation.cpp:483) where [de - er, de + er] leaves one answer,
+                // with a relative 1e-4 for expf and the FP32 uniform; a zero uniform goes to FP64
+                const float uf = static_cast<float>(uni);
+                soft = 2;
+                if (uf > 0.f) {
+                    if (de + er <= 0.f || uf <= expf(-(de + er) * A.inv_temp) * (1.f - 1e-4f)) soft = 1;
+                    else if (uf >= expf(-(de - er) * A.inv_temp) * (1.f + 1e-4f)) soft = 0;
+                }
+            }
+        }
+        if (!COUNT && !SOFT && dom != 1 && !overlap) {
             for (int base = 0; base < total; base += SWEEP_P1 * GW) {
                 int cl[SWEEP_P1];
 #pragma unroll
@@ -863,7 +981,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         // ---- FP64: the exact proposal of a surviving move (or of an accepted u == 0 move) ----
         // (an overlap found near the cell wall still needs the exact ActiveDomain test: the
         // reference rejects a move that leaves the domain before it tests any overlap)
-        const bool need64 = (code == 0) || (uni <= 0.0) || (dom == 2);
+        const bool need64 = (code == 0 && (!SOFT || soft != 0 || nun > 0)) || (uni <= 0.0) || (dom == 2);
         const bool needR = type != 0 && (need64 || A.log != nullptr);
         double rel_own = 0.0, pnew_own = 0.0, onew_own = 0.0, rrow[3] = {0.0, 0.0, 0.0};
         bool exact_rel = false;     // rel_own holds the exact FP64 relative coordinate
@@ -1052,6 +1170,30 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 ws.fp64 += nun;
                 if (ov) code = 1;
             }
+            if (SOFT && code == 0 && soft == 2) {
+                // the energy change in FP64 (core/Packing.cpp:103-108), every candidate within the
+                // soft range at the image of its FP32 separation; a fixed reduction order
+                const d3 p0{grp.shfl(pos_own, 0), grp.shfl(pos_own, 1), grp.shfl(pos_own, 2)};
+                double e0 = 0.0, e1 = 0.0;
+                for (int k = lane; k < total; k += GW) {
+                    const float4 q = cpos[k];
+                    const int pj = __float_as_int(q.w);
+                    if (pj == pid) continue;
+                    const float3 db = make_float3(q.x - pcur.x, q.y - pcur.y, q.z - pcur.z);
+                    const float3 da = make_float3(q.x - pn.x, q.y - pn.y, q.z - pn.z);
+                    const d3 p = load_d3(S.pos64 + 3 * (size_t)pj);
+                    if (dot3f(db, db) < S.fc.soft_reach2)
+                        e0 = dadd(e0, soft_energy(S, norm2(sub3(add3(p, load_d3(S.trans + 3 * image_index(S, db, p0, p))), p0))));
+                    if (dot3f(da, da) < S.fc.soft_reach2)
+                        e1 = dadd(e1, soft_energy(S, norm2(sub3(add3(p, load_d3(S.trans + 3 * image_index(S, da, pnew, p))), pnew))));
+                }
+                for (int d = GW / 2; d > 0; d >>= 1) {
+                    e0 = dadd(e0, grp.shfl_xor(e0, d));
+                    e1 = dadd(e1, grp.shfl_xor(e1, d));
+                }
+                soft = metropolis(uni, dsub(e1, e0), A.temperature) ? 1 : 0;
+                ws.fp64 += total - 1;
+            }
             // hard walls: the mover at its exact new state (Packing::countParticleOverlaps adds
             // the wall overlaps after the pairs, core/Packing.cpp:424-428)
             if (!COUNT && S.walls && code == 0) {
@@ -1171,7 +1313,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         }
 
         // ---- Metropolis (core/Simulation.cpp:483): u <= exp(-dE/T), dE in {-inf, 0, +inf} ----
-        const bool acc = code == 3 ? true : ((code == 0) ? (uni <= 1.0) : (uni <= 0.0));
+        const bool acc = code == 3 ? true : ((code == 0) ? (SOFT ? soft == 1 : uni <= 1.0) : (uni <= 0.0));
         if (acc) {
             const size_t gslot = (size_t)gbase + slot;
             // Packing::acceptMove adds the move's overlap delta in counting mode (core/Packing.cpp:298-300)
