@@ -59,6 +59,9 @@ cudaError_t launch_score_partners(const DevState &s, const GridDev &g, const flo
                                   int mode, float inv_range, int32_t *partners, cudaStream_t st);
 cudaError_t launch_rot_table(double *out64, float *out32, uint32_t count, uint64_t seed, uint64_t counter, float step,
                              cudaStream_t st);
+int cluster_blocks();
+int cluster_warps(const SweepArgs &a, int blocks, int active);
+cudaError_t launch_cluster_sweep(const SweepArgs &a, const int *phases, int nphases, int blocks, int warps, cudaStream_t st);
 cudaError_t launch_sweep_half(const SweepArgs &a, int ncells, cudaStream_t st);
 size_t sweep_smem_per_half(int kind, int cap);
 int sweep_half_blocks_per_sm(int kind, int cap);
@@ -75,6 +78,8 @@ namespace {
 
 constexpr int OVF_WARPS = 152;          // overflow rerun: one warp per block, grid-stride over cells
 constexpr size_t OVF_SMEM = 200 * 1024; // shared memory of one overflow warp
+constexpr int64_t CLUSTER_MAX_N = 32768;     // particles and cells of a cluster sweep's rebuild (16 blocks)
+constexpr int CLUSTER_MAX_CELLS = 16384;
 
 struct GridHost {
     GridDev d{};
@@ -176,6 +181,7 @@ struct Handle {
     float *rtab32 = nullptr;
     int32_t *item_counters = nullptr;  // work counters of persistent sweep launches
     int num_sms = 0;
+    int cl_blocks = -1;                // blocks of a cluster sweep on this device (-1: not asked yet)
     unsigned long long *count_out = nullptr;
     int *flag = nullptr;
     DeferredPair *cq_buf = nullptr;   // multi-centre recounts: deferred FP64 centre pairs
@@ -710,6 +716,8 @@ int setup_grid(Handle *h, GridHost &G, const double *box, const double *shift) {
     return RP_OK;
 }
 
+int rebuilt(Handle *h);
+
 int rebuild(Handle *h, int gi, int pi) {
     int saved_g = h->gcur, saved_p = h->pcur;
     h->gcur = gi;
@@ -721,6 +729,11 @@ int rebuild(Handle *h, int gi, int pi) {
         Group grp(h, RP_KERNEL_REBUILD, 6);
         RP_CUDA(h, launch_rebuild(s, h->grid[gi].d, h->block_sums, h->stream));
     }
+    return rebuilt(h);
+}
+
+// The grid of the current positions was (re)built on the stream.
+int rebuilt(Handle *h) {
     h->grid_rebuilds++;
     // a grid built from the current positions lists every particle where it is
     if (!h->disp_host.empty()) {
@@ -1724,17 +1737,56 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
                        (r.c >> 8) * (1.0 / 16777216.0)};
     int rc = setup_grid(h, h->grid[h->gcur], h->box, shift);
     if (rc) return rc;
-    rc = rebuild(h, h->gcur, h->pcur);
+    const GridDev &g = h->grid[h->gcur].d;
+    // spheres with a soft part take the FP32 sweep with an error bound on the energy change, over a
+    // grid where a staged candidate is one image of another particle
+    const bool soft32 = h->soft && h->shape.kind == RP_SHAPE_SPHERE && !h->counting && !(p->flags & RP_SWEEP_FP64_ONLY) &&
+                        !h->grid[h->gcur].no_ng && g.dims[0] >= 3 && g.dims[1] >= 3 && g.dims[2] >= 3 &&
+                        (h->soft_only || !h->walls);
+    const bool fp64_sweep = (h->soft && !soft32) || h->shape.kind == RP_SHAPE_CONVEX;
+    if ((soft32 || fp64_sweep) && types == SWEEP_ROTOTRANSLATION)
+        return fail(h, RP_ERR_UNSUPPORTED, "rototranslations with a soft part or a convex body");
+    std::vector<int> phases;
+    grid_phases(g, r.d, phases);
+    // the arguments every phase shares
+    auto sweep_args = [&](double tstep) {
+        SweepArgs a = base_args(h);
+        if (soft32) {
+            a.soft32 = 1;
+            a.temperature = h->temperature;
+            a.inv_temp = static_cast<float>(1.0 / h->temperature);
+        }
+        a.inv_range = static_cast<float>(1.0 / h->range);
+        a.seed = p->seed;
+        a.counter = p->counter;
+        a.tstep = static_cast<float>(tstep);
+        a.rstep = static_cast<float>(p->rotation_step);
+        a.types = types;
+        a.rtab64 = h->rtab64;
+        a.rtab32 = h->rtab32;
+        a.rtab_mask = ROT_TABLE - 1;
+        if (p->flags & RP_SWEEP_FP64_ONLY) a.fp64_only = 1;
+        return a;
+    };
+    // small systems: the rebuild and every phase in one launch of a thread-block cluster, where each
+    // active cell of a phase gets a warp there (1000 spheres: 180 -> 45 us a sweep; with more cells
+    // than that the whole chip's warps are worth the launches)
+    int cl_warps = 0;
+    if (!fp64_sweep && !h->bulk_stage && h->cells_per_warp == 1 && h->order_mode == RP_ORDER_OFF && h->pair_cap == 0 &&
+        h->n <= CLUSTER_MAX_N && g.ncell <= CLUSTER_MAX_CELLS) {
+        if (h->cl_blocks < 0) h->cl_blocks = cluster_blocks();
+        int most = 0, act[3];
+        for (int ph : phases) most = std::max(most, phase_cells(g, ph, act));
+        cl_warps = cluster_warps(sweep_args(0.0), h->cl_blocks, most);
+    }
+    rc = cl_warps ? rebuilt(h) : rebuild(h, h->gcur, h->pcur);
     if (rc) return rc;
     h->grid_stale = false;
     h->stale_unshifted = false;
-    const GridDev &g = h->grid[h->gcur].d;
     // translation step limited to half the smallest box height (TranslationSampler.cpp:39-46)
     double hgt[3];
     heights_of(h->box, hgt);
     double tstep = std::min(p->translation_step, std::min({hgt[0], hgt[1], hgt[2]}) / 2);
-    std::vector<int> phases;
-    grid_phases(g, r.d, phases);
     int ntypes = sweep_move_types(types);
     bool log = (p->flags & RP_SWEEP_LOG) != 0;
     if (log) {
@@ -1758,20 +1810,10 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         if (rc2) return rc2;
     }
     h->since_rank++;
-    // spheres with a soft part take the FP32 sweep with an error bound on the energy change, over a
-    // grid where a staged candidate is one image of another particle
-    const bool soft32 = h->soft && h->shape.kind == RP_SHAPE_SPHERE && !h->counting && !(p->flags & RP_SWEEP_FP64_ONLY) &&
-                        !h->grid[h->gcur].no_ng && g.dims[0] >= 3 && g.dims[1] >= 3 && g.dims[2] >= 3 &&
-                        (h->soft_only || !h->walls);
-    const bool fp64_sweep = (h->soft && !soft32) || h->shape.kind == RP_SHAPE_CONVEX;
-    if (soft32 && types == SWEEP_ROTOTRANSLATION)
-        return fail(h, RP_ERR_UNSUPPORTED, "rototranslations with a soft part or a convex body");
     if (fp64_sweep) {
         // a soft part or a generic convex body: every move decided in FP64 (hard part, then the
         // energy change with the Metropolis test at the handle's temperature), one warp per
         // active cell
-        if (types == SWEEP_ROTOTRANSLATION)
-            return fail(h, RP_ERR_UNSUPPORTED, "rototranslations with a soft part or a convex body");
         SoftSweepArgs sa{};
         sa.c.s = dev_state(h);
         sa.c.g = g;
@@ -1811,14 +1853,19 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     int order_start[27] = {0};
     const bool ordered = h->cell_order && !fp64_sweep && g.order;
     if (ordered) order_starts(g, order_start);
-    for (int ph : (fp64_sweep ? std::vector<int>{} : phases)) {
-        SweepArgs a = base_args(h);
-        if (h->order_mode != RP_ORDER_OFF && !soft32) a.partners = h->partners;
-        if (soft32) {
-            a.soft32 = 1;
-            a.temperature = h->temperature;
-            a.inv_temp = static_cast<float>(1.0 / h->temperature);
+    if (cl_warps) {
+        SweepArgs a = sweep_args(tstep);
+        if (log) {
+            a.log = h->d_log;
+            a.log_codes = h->d_log_codes;
         }
+        h->last_cells_per_warp = 1;
+        Group grp(h, RP_KERNEL_SWEEP, 1);
+        RP_CUDA(h, launch_cluster_sweep(a, phases.data(), static_cast<int>(phases.size()), h->cl_blocks, cl_warps, h->stream));
+    }
+    for (int ph : (fp64_sweep || cl_warps ? std::vector<int>{} : phases)) {
+        SweepArgs a = sweep_args(tstep);
+        if (h->order_mode != RP_ORDER_OFF && !soft32) a.partners = h->partners;
         if (h->pair_cap > 0 && !soft32) {
             a.pair_feats = h->pair_feats;
             a.pair_labels = h->pair_labels;
@@ -1826,7 +1873,6 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
             a.pair_cap = static_cast<unsigned long long>(h->pair_cap);
             a.pair_every = h->pair_every;
         }
-        a.inv_range = static_cast<float>(1.0 / h->range);
         a.next_item = h->item_counters + phase_no++;
         int act[3];
         a.num_active = phase_cells(g, ph, act);
@@ -1839,15 +1885,6 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
             a.work_count = nullptr;
             a.num_work = a.num_active;
         }
-        a.seed = p->seed;
-        a.counter = p->counter;
-        a.tstep = static_cast<float>(tstep);
-        a.rstep = static_cast<float>(p->rotation_step);
-        a.types = types;
-        a.rtab64 = h->rtab64;
-        a.rtab32 = h->rtab32;
-        a.rtab_mask = ROT_TABLE - 1;
-        if (p->flags & RP_SWEEP_FP64_ONLY) a.fp64_only = 1;
         if (log) {
             a.log = h->d_log;
             a.log_codes = h->d_log_codes;
