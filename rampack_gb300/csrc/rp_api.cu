@@ -1,5 +1,7 @@
 // C-ABI of the engine (include/rampack_gb300.h): handle lifetime, state transfer,
 // cell-grid set-up, move lists, device-driven sweeps and box moves.
+#include <atomic>
+#include <cstddef>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -182,7 +184,15 @@ struct Handle {
     int32_t *item_counters = nullptr;  // work counters of persistent sweep launches
     int num_sms = 0;
     int cl_blocks = -1;                // blocks of a cluster sweep on this device (-1: not asked yet)
+    // the answers of recounts and box moves in one device block, so that one copy brings them to the
+    // page-locked `answers` (their order here): overlaps, early-exit flag, particles that changed cell
     unsigned long long *count_out = nullptr;
+    struct Answers {
+        unsigned long long count;
+        int flag, moved;
+        uint32_t status, pad;
+    } *answers = nullptr;
+    int *moved = nullptr;
     int *flag = nullptr;
     DeferredPair *cq_buf = nullptr;   // multi-centre recounts: deferred FP64 centre pairs
     int *cq_count = nullptr;
@@ -272,6 +282,8 @@ struct Handle {
     // grid is then current for every other particle: grid_patched)
     SingleTry *d_try = nullptr;
     bool try_valid = false;
+    SingleResult *try_result = nullptr;   // page-locked: the kernel's answer to the last rp_try_move
+    unsigned long long try_seq = 0;
     int32_t try_particle = -1;
     int32_t *d_disp_list = nullptr;
     uint8_t *d_disp_flag = nullptr;
@@ -745,29 +757,38 @@ int rebuilt(Handle *h) {
     return RP_OK;
 }
 
+// The device's answers (count_out and the status word) on the host; waits for the stream.
+int fetch_answers(Handle *h) {
+    RP_CUDA(h, cudaMemcpyAsync(h->answers, h->count_out, offsetof(Handle::Answers, status), cudaMemcpyDeviceToHost, h->stream));
+    RP_CUDA(h, cudaMemcpyAsync(&h->answers->status, h->status, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->stream));
+    RP_CUDA(h, cudaStreamSynchronize(h->stream));
+    return RP_OK;
+}
+
 // The grid of a rescaled state (rp_try_scaling; h->gcur / h->pcur already name grid `ng` and
 // the rescaled positions): when its divisions and origin are the old grid's and the old grid
 // lists every particle where it is, the old cells are kept and only the FP32 cell-local
 // positions recomputed (k_remap, one pass, the grid a rebuild would build); a particle that
 // changed cell through rounding falls back to the full rebuild.
-int remap_or_rebuild(Handle *h, int old_g, int ng, int np) {
+// `then` enqueues work on the kept grid (a recount) before the one wait for the answers; kept
+// tells whether the grid, and so that work, stands.
+template <class Then>
+int remap_or_rebuild(Handle *h, int old_g, int ng, int np, Then then, bool &kept) {
     const GridDev &o = h->grid[old_g].d, &g = h->grid[ng].d;
     bool same = !h->grid_patched && !h->grid_stale && h->disp_host.empty() && o.ncell == g.ncell && o.slot_pid;
     for (int d = 0; d < 3; d++) same = same && o.dims[d] == g.dims[d] && o.shift[d] == g.shift[d];
     if (same) {
-        RP_CUDA(h, cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
+        // (the cells' occupancy order is not carried over: sweeps rebuild the grid)
+        RP_CUDA(h, cudaMemsetAsync(h->count_out, 0, sizeof(Handle::Answers), h->stream));
         {
             Group grp(h, RP_KERNEL_RESCALE, 1);
-            RP_CUDA(h, launch_remap(dev_state(h), g, o, h->flag, h->stream));
+            RP_CUDA(h, launch_remap(dev_state(h), g, o, h->moved, h->stream));
         }
-        int moved = 0;
-        RP_CUDA(h, cudaMemcpyAsync(&moved, h->flag, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-        RP_CUDA(h, cudaStreamSynchronize(h->stream));
-        if (!moved) {
-            // the kept cells keep their occupancy order
-            if (g.order && o.order)
-                RP_CUDA(h, cudaMemcpyAsync(g.order, o.order, sizeof(int32_t) * g.ncell, cudaMemcpyDeviceToDevice,
-                                           h->stream));
+        int ra = then();
+        if (ra == RP_OK) ra = fetch_answers(h);
+        if (ra) return ra;
+        if (!h->answers->moved) {
+            kept = true;
             h->grid_remaps++;
             return RP_OK;
         }
@@ -1119,8 +1140,10 @@ static int create_common(Handle *h, int64_t n, int device, void **handle) {
         cudaMemset(h->status, 0, sizeof(uint32_t));
         cudaMemset(h->counters, 0, sizeof(unsigned long long) * NUM_COUNTERS);
     }
-    if ((e = cudaMalloc(&h->count_out, sizeof(unsigned long long))) != cudaSuccess) return bail(e);
-    if ((e = cudaMalloc(&h->flag, sizeof(int))) != cudaSuccess) return bail(e);
+    if ((e = cudaMalloc(&h->count_out, sizeof(Handle::Answers))) != cudaSuccess) return bail(e);
+    h->flag = reinterpret_cast<int *>(h->count_out + 1);
+    h->moved = h->flag + 1;
+    if ((e = cudaMallocHost(&h->answers, sizeof(Handle::Answers))) != cudaSuccess) return bail(e);
     if ((e = cudaMalloc(&h->overflow_count, sizeof(int32_t))) != cudaSuccess) return bail(e);
     if ((e = cudaMalloc(&h->d_overlaps, sizeof(unsigned long long))) != cudaSuccess) return bail(e);
     cudaMemset(h->d_overlaps, 0, sizeof(unsigned long long));
@@ -1376,7 +1399,8 @@ int rp_destroy(void *handle) {
     cudaFree(h->d_energy);
     cudaFree(h->d_disp_list);
     cudaFree(h->d_disp_flag);
-    cudaFree(h->flag);
+    cudaFreeHost(h->answers);
+    cudaFreeHost(h->try_result);
     cudaFree(h->overflow);
     cudaFree(h->overflow_count);
     cudaFree(h->d_overlaps);
@@ -1500,6 +1524,8 @@ SingleArgs single_args(Handle *h) {
     return a;
 }
 
+static int enqueue_count(Handle *h, int early_exit);
+
 int rp_count_overlaps(void *handle, int early_exit, int64_t *out_count) {
     Handle *h = static_cast<Handle *>(handle);
     if (!h || !out_count) return fail(h, RP_ERR_ARG, "null argument");
@@ -1513,8 +1539,17 @@ int rp_count_overlaps(void *handle, int early_exit, int64_t *out_count) {
         int rg = ensure_grid(h);  // an upload defers the grid
         if (rg) return rg;
     }
-    RP_CUDA(h, cudaMemsetAsync(h->count_out, 0, sizeof(unsigned long long), h->stream));
-    RP_CUDA(h, cudaMemsetAsync(h->flag, 0, sizeof(int), h->stream));
+    RP_CUDA(h, cudaMemsetAsync(h->count_out, 0, sizeof(Handle::Answers), h->stream));
+    int rc = enqueue_count(h, early_exit);
+    if (rc == RP_OK) rc = fetch_answers(h);
+    if (rc) return rc;
+    const unsigned long long c = h->answers->count;
+    *out_count = early_exit ? (c > 0 ? 1 : 0) : static_cast<int64_t>(c);
+    return h->answers->status ? check_status(h) : RP_OK;
+}
+
+// The recount's kernels on the current grid (count_out zeroed).
+static int enqueue_count(Handle *h, int early_exit) {
     // polyspherocylinders: the FP64 segment tests of the recount go to a second, lane-dense
     // kernel (polyspheres' centre tests are cheap enough inline)
     const bool defer = h->ncen > 0 && h->segs;
@@ -1540,11 +1575,7 @@ int rp_count_overlaps(void *handle, int early_exit, int64_t *out_count) {
         Group grp(h, RP_KERNEL_COUNT, defer ? 2 : 1);
         RP_CUDA(h, launch_count(s, h->grid[h->gcur].d, early_exit ? 1 : 0, h->count_out, h->flag, h->stream));
     }
-    unsigned long long c = 0;
-    RP_CUDA(h, cudaMemcpyAsync(&c, h->count_out, sizeof(c), cudaMemcpyDeviceToHost, h->stream));
-    RP_CUDA(h, cudaStreamSynchronize(h->stream));
-    *out_count = early_exit ? (c > 0 ? 1 : 0) : static_cast<int64_t>(c);
-    return check_status(h);
+    return RP_OK;
 }
 
 static int fill_info(Handle *h, rp_grid_info *info) {
@@ -1799,7 +1830,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         }
     }
     if (stats) RP_CUDA(h, cudaMemsetAsync(h->counters, 0, sizeof(unsigned long long) * NUM_COUNTERS, h->stream));
-    RP_CUDA(h, cudaMemsetAsync(h->item_counters, 0, sizeof(int32_t) * 64, h->stream));
+    if (!cl_warps) RP_CUDA(h, cudaMemsetAsync(h->item_counters, 0, sizeof(int32_t) * 64, h->stream));
     if (types & (2 | SWEEP_ROTOTRANSLATION)) {
         Group grp(h, RP_KERNEL_SWEEP, 1);
         RP_CUDA(h, launch_rot_table(h->rtab64, h->rtab32, ROT_TABLE, p->seed, p->counter,
@@ -2043,14 +2074,27 @@ int rp_try_scaling(void *handle, const double *new_box9, double *dE) {
     h->pcur = np;
     h->gcur = ng;
     double shift[3] = {h->grid[old_g].d.shift[0], h->grid[old_g].d.shift[1], h->grid[old_g].d.shift[2]};
-    int rc = setup_grid(h, h->grid[ng], h->box, shift);
-    if (rc == RP_OK) rc = remap_or_rebuild(h, old_g, ng, np);
-    if (rc == RP_OK && h->ncen > 0) {
+    // A convex shape in a box that only grew cannot overlap (core/Packing.cpp:199-200);
+    // polyspheres are not convex (PolysphereTraits.h:133).
+    const bool grew = h->shape.kind != RP_SHAPE_POLYSPHERE && box_upscaled(h->saved_box, h->box);
+    // the plain recount goes with the kept grid, ahead of the wait that tells whether it is kept
+    const bool plain = !h->soft_only && !h->counting && !grew;
+    auto centres = [&]() -> int {
         // Packing::tryScaling recalculates the absolute centres (core/Packing.cpp:186-187)
+        if (h->ncen == 0) return RP_OK;
         Group grp(h, RP_KERNEL_RESCALE, 1);
-        cudaError_t e = launch_abs_centres(dev_state(h), h->stream);
-        if (e != cudaSuccess) rc = fail(h, RP_ERR_CUDA, cudaGetErrorString(e));
-    }
+        RP_CUDA(h, launch_abs_centres(dev_state(h), h->stream));
+        return RP_OK;
+    };
+    bool kept = false;
+    int rc = setup_grid(h, h->grid[ng], h->box, shift);
+    if (rc == RP_OK)
+        rc = remap_or_rebuild(h, old_g, ng, np, [&]() -> int {
+            const int e = centres();
+            return e == RP_OK && plain ? enqueue_count(h, 1) : e;
+        }, kept);
+    if (rc == RP_OK && !kept) rc = centres();
+    if (rc == RP_OK && kept && h->answers->status) rc = check_status(h);
     if (rc) {
         std::memcpy(h->box, h->saved_box, sizeof(h->box));
         std::memcpy(h->inv, h->saved_inv, sizeof(h->inv));
@@ -2089,16 +2133,18 @@ int rp_try_scaling(void *handle, const double *new_box9, double *dE) {
                         : (delta > 0 ? std::numeric_limits<double>::infinity() : 0.0);
         return soft_change(dE);
     }
-    // A convex shape in a box that only grew cannot overlap (core/Packing.cpp:199-200);
-    // polyspheres are not convex (PolysphereTraits.h:133).
-    if (h->shape.kind != RP_SHAPE_POLYSPHERE && box_upscaled(h->saved_box, h->box)) {
+    if (grew) {
         *dE = 0;
-        RP_CUDA(h, cudaStreamSynchronize(h->stream));
+        if (!kept) RP_CUDA(h, cudaStreamSynchronize(h->stream));
         return soft_change(dE);
     }
     int64_t cnt = 0;
-    rc = rp_count_overlaps(h, 1, &cnt);
-    if (rc) return rc;
+    if (kept) {
+        cnt = h->answers->count > 0 ? 1 : 0;
+    } else {
+        rc = rp_count_overlaps(h, 1, &cnt);
+        if (rc) return rc;
+    }
     *dE = cnt > 0 ? std::numeric_limits<double>::infinity() : 0.0;
     return soft_change(dE);
 }
@@ -2135,6 +2181,8 @@ int rp_try_move(void *handle, const rp_move *move, const double *domain6, double
     h->try_valid = false;
     if (!h->d_try) {
         RP_CUDA(h, cudaMalloc(&h->d_try, sizeof(SingleTry)));
+        RP_CUDA(h, cudaMallocHost(&h->try_result, sizeof(SingleResult)));
+        *h->try_result = SingleResult{};
         RP_CUDA(h, cudaMalloc(&h->d_disp_list, sizeof(int32_t) * Handle::DISP_CAP));
         RP_CUDA(h, cudaMalloc(&h->d_disp_flag, static_cast<size_t>(h->n)));
         RP_CUDA(h, cudaMemsetAsync(h->d_disp_flag, 0, static_cast<size_t>(h->n), h->stream));
@@ -2153,6 +2201,8 @@ int rp_try_move(void *handle, const rp_move *move, const double *domain6, double
     a.g = h->grid[h->gcur].d;
     a.m = *move;
     a.out = h->d_try;
+    a.result = h->try_result;
+    a.seq = ++h->try_seq;
     a.disp_list = h->d_disp_list;
     a.disp_flag = h->d_disp_flag;
     a.ndisp = static_cast<int>(h->disp_host.size());
@@ -2168,11 +2218,22 @@ int rp_try_move(void *handle, const rp_move *move, const double *domain6, double
         Group grp(h, RP_KERNEL_SINGLE, 1);
         RP_CUDA(h, launch_try_single(a, h->stream));
     }
-    double e = 0;
-    RP_CUDA(h, cudaMemcpyAsync(&e, &h->d_try->dE, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    int rc = check_status(h);  // synchronises
-    if (rc) return rc;
-    *dE = e;
+    // the answer is in page-locked memory once the kernel has written the call's number there; the
+    // stream is asked now and then, so that a failed launch ends the wait
+    const volatile SingleResult *res = h->try_result;
+    for (unsigned spins = 1; res->seq != a.seq; spins++)
+        if (spins % 4096 == 0) {
+            const cudaError_t q = cudaStreamQuery(h->stream);
+            if (q == cudaErrorNotReady) continue;
+            RP_CUDA(h, q);
+            if (res->seq != a.seq) return fail(h, RP_ERR_DEVICE, "a single move's kernel left no answer");
+        }
+    std::atomic_thread_fence(std::memory_order_acquire);
+    if (res->status) {
+        const int rc = check_status(h);
+        if (rc) return rc;
+    }
+    *dE = res->dE;
     h->try_valid = true;
     h->try_particle = move->particle;
     return RP_OK;

@@ -268,6 +268,14 @@ struct SingleTry {
     int32_t outside, pad;   // rejected by the ActiveDomain before any overlap test
 };
 
+// What a single-move test tells the host, in page-locked memory that the kernel writes: the
+// energy, the device status word, and last the call's number (the host waits for it).
+struct SingleResult {
+    double dE;
+    uint32_t status, pad;
+    unsigned long long seq;
+};
+
 // Arguments of one single-move test: the mover's candidates are the particles listed in the
 // 27 grid cells around its position (the grid is current except for the particles moved by
 // single moves since it was built, which are skipped there and tested from `disp_list`).
@@ -276,6 +284,8 @@ struct SingleArgs {
     GridDev g;
     rp_move m;
     SingleTry *out;
+    SingleResult *result;
+    unsigned long long seq;
     double temperature;   // soft sweeps: the Metropolis temperature
     const int32_t *disp_list;
     const uint8_t *disp_flag;

@@ -261,7 +261,10 @@ __device__ __forceinline__ int candidate_at(const SingleArgs &A, const Mover &mv
 // pairs between insphere and circumsphere distance are queued and their refinements run packed
 // 32 to a warp pass, so the lanes of a pass all refine (instead of a few lanes per candidate
 // round).  Same pairs and decisions as the per-candidate loop; the count, or 0 / 1 with `early`.
-__device__ int warp_overlaps_convex(const SingleArgs &A, const Mover &mv, int which, bool early, int pid) {
+// Of `step` / 32 warps that share the candidates the one starting at `first` (a multiple of 32);
+// xq: its queue.  The walls are the first one's.
+__device__ int warp_overlaps_convex(const SingleArgs &A, const Mover &mv, int which, bool early, int pid, int first,
+                                    int step, int *xq) {
     const DevState &s = A.s;
     const int lane = threadIdx.x & 31;
     const int in_cells = mv.cstart[which][mv.ncells[which]];
@@ -276,7 +279,7 @@ __device__ int warp_overlaps_convex(const SingleArgs &A, const Mover &mv, int wh
         for (int b = 0; b < nq; b += 32) {
             int c = 0;
             if (b + lane < nq) {
-                const int e = mv.xq[b + lane];
+                const int e = xq[b + lane];
                 const int j = e / 28, m = e % 28;
                 const d3 pj = load_d3(s.pos64 + 3 * (size_t)j);
                 const d3 t = m == 27 ? pbc_translation(s.box, s.inv, p, pj)
@@ -293,7 +296,7 @@ __device__ int warp_overlaps_convex(const SingleArgs &A, const Mover &mv, int wh
         nq = 0;
         return false;
     };
-    for (int base = 0; base < total; base += 32) {
+    for (int base = first; base < total; base += step) {
         const int k = base + lane;
         int certain = 0;
         int near_e[4];
@@ -340,14 +343,14 @@ __device__ int warp_overlaps_convex(const SingleArgs &A, const Mover &mv, int wh
             const bool has = r < nnear;
             const unsigned bal = __ballot_sync(FULL, has);
             if (!bal) break;
-            if (has) mv.xq[nq + __popc(bal & ((1u << lane) - 1))] = near_e[r];
+            if (has) xq[nq + __popc(bal & ((1u << lane) - 1))] = near_e[r];
             nq += __popc(bal);
         }
         __syncwarp();
     }
     if (drain()) return 1;
     for (int d = 16; d > 0; d >>= 1) cnt += __shfl_xor_sync(FULL, cnt, d);
-    if (s.walls && !(early && cnt)) {
+    if (s.walls && first == 0 && !(early && cnt)) {
         // hard walls after the pairs (core/Packing.cpp:424-428)
         int w = 0;
         if (lane == 0) w = xc_wall_count(*s.xc, s.walls, s.wall_vec, s.wall_far, s.wall_half, p, rot, early);
@@ -359,8 +362,8 @@ __device__ int warp_overlaps_convex(const SingleArgs &A, const Mover &mv, int wh
 // Overlaps of mover state `which` with every candidate, then the walls (the count, or 0 / 1
 // with `early`: Packing::countParticleOverlaps, core/Packing.cpp:373-429); the whole warp.
 template <int KIND>
-__device__ int warp_overlaps(const SingleArgs &A, const Mover &mv, int which, bool early, int pid) {
-    if constexpr (KIND == 3) return warp_overlaps_convex(A, mv, which, early, pid);
+__device__ int warp_overlaps(const SingleArgs &A, const Mover &mv, int which, bool early, int pid, int first, int step, int *xq) {
+    if constexpr (KIND == 3) return warp_overlaps_convex(A, mv, which, early, pid, first, step, xq);
     const DevState &s = A.s;
     const int lane = threadIdx.x & 31;
     const int in_cells = mv.cstart[which][mv.ncells[which]];
@@ -368,7 +371,7 @@ __device__ int warp_overlaps(const SingleArgs &A, const Mover &mv, int which, bo
     const d3 a{mv.rot[which][2], mv.rot[which][5], mv.rot[which][8]};
     const double *hax = (KIND == 2 && s.segs) ? mv.hax[which] : nullptr;
     int cnt = 0;
-    for (int base = 0; base < total; base += 32) {
+    for (int base = first; base < total; base += step) {
         const int k = base + lane;
         int c = 0;
         if (k < total) {
@@ -381,7 +384,7 @@ __device__ int warp_overlaps(const SingleArgs &A, const Mover &mv, int which, bo
         cnt += c;
     }
     for (int d = 16; d > 0; d >>= 1) cnt += __shfl_xor_sync(FULL, cnt, d);
-    if (s.walls) {
+    if (s.walls && first == 0) {
         // hard walls after the pairs (core/Packing.cpp:424-428)
         int w = 0;
         if (lane == 0) {
@@ -398,12 +401,12 @@ __device__ int warp_overlaps(const SingleArgs &A, const Mover &mv, int which, bo
 // Soft energy of mover state `which` with every candidate (Packing::calculateParticleEnergy,
 // core/Packing.cpp:649-687); the whole warp, a fixed reduction order.
 template <int KIND>
-__device__ double warp_energy(const SingleArgs &A, const Mover &mv, int which, int pid) {
+__device__ double warp_energy(const SingleArgs &A, const Mover &mv, int which, int pid, int first, int step) {
     const int lane = threadIdx.x & 31;
     const int in_cells = mv.cstart[which][mv.ncells[which]];
     const int total = in_cells + A.ndisp;
     double e = 0.0;
-    for (int k = lane; k < total; k += 32) {
+    for (int k = first + lane; k < total; k += step) {
         const int j = candidate_at(A, mv, which, k, in_cells);
         if (j >= 0 && j != pid) e = dadd(e, candidate_energy<KIND>(A, mv.pos[which], mv.abs[which], j));
     }
@@ -547,29 +550,68 @@ __device__ double move_energy(const SingleArgs &A, const Mover &mv, int pid, int
     if (mv.outside) return CUDART_INF;
     if (!s.soft_only) {
         if (s.counting) {
-            const int after = warp_overlaps<KIND>(A, mv, 0, false, pid);
-            const int before = warp_overlaps<KIND>(A, mv, 1, false, pid);
+            const int after = warp_overlaps<KIND>(A, mv, 0, false, pid, 0, 32, mv.xq);
+            const int before = warp_overlaps<KIND>(A, mv, 1, false, pid, 0, 32, mv.xq);
             delta = after - before;
             if (delta < 0) return -CUDART_INF;
             if (delta > 0) return CUDART_INF;
-        } else if (warp_overlaps<KIND>(A, mv, 0, true, pid)) {
+        } else if (warp_overlaps<KIND>(A, mv, 0, true, pid, 0, 32, mv.xq)) {
             return CUDART_INF;
         }
     }
     if (!s.soft) return 0.0;
-    const double initial = warp_energy<KIND>(A, mv, 1, pid);
-    const double final_ = warp_energy<KIND>(A, mv, 0, pid);
+    const double initial = warp_energy<KIND>(A, mv, 1, pid, 0, 32);
+    const double final_ = warp_energy<KIND>(A, mv, 0, pid, 0, 32);
     return dsub(final_, initial);
 }
 
+// One single move: the first warp builds the mover, TRY_WARPS warps share its candidates (a warp
+// alone walked a rod's 200 candidates in seven dependent rounds: 19 against 8 us a move), and the
+// host reads the answer from page-locked memory.
+constexpr int TRY_WARPS = 8;
 template <int KIND>
-__global__ void __launch_bounds__(32) k_try_single(SingleArgs A) {
+__global__ void __launch_bounds__(TRY_WARPS * 32) k_try_single(const __grid_constant__ SingleArgs A) {
     __shared__ Mover mv;
-    const int pid = A.m.particle;
-    build_mover<KIND>(A, mv, A.m, pid, A.s.counting || A.s.soft, A.has_domain ? A.dom_lo : nullptr,
-                      A.has_domain ? A.dom_hi : nullptr, nullptr);
+    __shared__ int xq[KIND == 3 ? TRY_WARPS : 1][XC_QUEUE];
+    __shared__ int count[2];
+    __shared__ double part[2][TRY_WARPS];
+    const DevState &s = A.s;
+    const int pid = A.m.particle, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x < 2) count[threadIdx.x] = 0;
+    if (w == 0)
+        build_mover<KIND>(A, mv, A.m, pid, s.counting || s.soft, A.has_domain ? A.dom_lo : nullptr,
+                          A.has_domain ? A.dom_hi : nullptr, nullptr);
+    __syncthreads();
+    // move_energy with the candidates shared (every branch is the whole block's)
+    const int first = 32 * w, step = 32 * TRY_WARPS;
+    int *q = xq[KIND == 3 ? w : 0];
     int delta = 0;
-    const double dE = move_energy<KIND>(A, mv, pid, delta);
+    double dE = mv.outside ? CUDART_INF : 0.0;
+    if (!mv.outside && !s.soft_only) {
+        if (s.counting) {
+            for (int which = 0; which < 2; which++) {
+                const int n = warp_overlaps<KIND>(A, mv, which, false, pid, first, step, q);
+                if (lane == 0 && n) atomicAdd(&count[which], n);
+            }
+            __syncthreads();
+            delta = count[0] - count[1];
+            if (delta != 0) dE = delta < 0 ? -CUDART_INF : CUDART_INF;
+        } else if (__syncthreads_or(warp_overlaps<KIND>(A, mv, 0, true, pid, first, step, q))) {
+            dE = CUDART_INF;
+        }
+    }
+    if (s.soft && dE == 0.0) {
+        for (int which = 0; which < 2; which++) {
+            const double e = warp_energy<KIND>(A, mv, which, pid, first, step);
+            if (lane == 0) part[which][w] = e;
+        }
+        __syncthreads();
+        double e[2] = {0.0, 0.0};
+        for (int which = 0; which < 2; which++)
+            for (int k = 0; k < TRY_WARPS; k++) e[which] = dadd(e[which], part[which][k]);
+        dE = dsub(e[0], e[1]);
+    }
+    __syncthreads();   // every thread's status bits are raised
     if (threadIdx.x == 0) {
         SingleTry *o = A.out;
         for (int d = 0; d < 3; d++) o->pos[d] = mv.pos[0][d];
@@ -585,6 +627,11 @@ __global__ void __launch_bounds__(32) k_try_single(SingleArgs A) {
         o->type = A.m.type;
         o->delta = delta;
         o->valid = 1;
+        volatile SingleResult *r = A.result;
+        r->dE = dE;
+        r->status = atomicOr(s.status, 0u);
+        __threadfence_system();
+        r->seq = A.seq;
     }
 }
 
@@ -905,10 +952,10 @@ __global__ void k_sum_fixed(const double *v, int64_t n, double *out) {
 }  // namespace
 
 cudaError_t launch_try_single(const SingleArgs &a, cudaStream_t st) {
-    if (a.s.kind == 0) k_try_single<0><<<1, 32, 0, st>>>(a);
-    else if (a.s.kind == 1) k_try_single<1><<<1, 32, 0, st>>>(a);
-    else if (a.s.kind == 2) k_try_single<2><<<1, 32, 0, st>>>(a);
-    else k_try_single<3><<<1, 32, 0, st>>>(a);
+    if (a.s.kind == 0) k_try_single<0><<<1, TRY_WARPS * 32, 0, st>>>(a);
+    else if (a.s.kind == 1) k_try_single<1><<<1, TRY_WARPS * 32, 0, st>>>(a);
+    else if (a.s.kind == 2) k_try_single<2><<<1, TRY_WARPS * 32, 0, st>>>(a);
+    else k_try_single<3><<<1, TRY_WARPS * 32, 0, st>>>(a);
     return cudaGetLastError();
 }
 

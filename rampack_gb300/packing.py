@@ -44,6 +44,16 @@ def cell_phase(dims, cell: int) -> int:
     return ring_colour(dims[0], cx) + 3 * ring_colour(dims[1], cy) + 9 * ring_colour(dims[2], cz)
 
 
+class MoveRecord(C.Structure):
+    """rp_move (the layout of MOVE_DTYPE)."""
+    _fields_ = [("particle", C.c_int32), ("type", C.c_int32), ("domain", C.c_int32), ("reserved", C.c_int32),
+                ("translation", C.c_double * 3), ("rotation", C.c_double * 9), ("uniform", C.c_double)]
+
+
+assert C.sizeof(MoveRecord) == MOVE_DTYPE.itemsize
+IDENTITY = (1.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 1.0)
+
+
 class GpuPacking:
     def __init__(self, kind: int, params, pos, rot, box, device: int = 0):
         self.lib = _lib.load()
@@ -192,15 +202,15 @@ class GpuPacking:
         """Packing::tryTranslation / tryRotation / tryMove (rp_try_move), with no ActiveDomain or
         with `domain` = its relative bounds (lo[3], hi[3]): the move's energy (0 or +inf; -inf,
         0 or +inf in overlap counting); the tried state waits for accept_move."""
-        m = np.zeros(1, dtype=MOVE_DTYPE)
-        m["particle"] = particle
-        m["type"] = type_
-        m["domain"] = -1
-        m["translation"] = np.asarray(translation, dtype=np.float64).reshape(3)
-        m["rotation"] = np.eye(3).reshape(9) if rotation is None else np.asarray(rotation, dtype=np.float64).reshape(9)
+        particle, type_ = int(particle), int(type_)
+        if not -0x80000000 <= particle <= 0x7fffffff or not -0x80000000 <= type_ <= 0x7fffffff:
+            raise OverflowError("a particle index or move type beyond 32 bits")
+        m = MoveRecord(particle=particle, type=type_, domain=-1)
+        m.translation[:] = np.asarray(translation, dtype=np.float64).reshape(3).tolist()
+        m.rotation[:] = IDENTITY if rotation is None else np.asarray(rotation, dtype=np.float64).reshape(9).tolist()
         de = C.c_double()
         dom = None if domain is None else np.ascontiguousarray(domain, dtype=np.float64).reshape(6)
-        self._check(self.lib.rp_try_move(self.h, m.ctypes.data_as(C.c_void_p), None if dom is None else dptr(dom),
+        self._check(self.lib.rp_try_move(self.h, C.byref(m), None if dom is None else dptr(dom),
                                          C.byref(de)))
         return de.value
 
