@@ -174,7 +174,26 @@ __device__ int candidate_overlaps(const SingleArgs &A, const double *p, d3 a, co
         const float3 sep = separation32(s.pos64 + 3 * (size_t)j, p);
         for_each_image(A, sep, [&](int mx, int my, int mz) {
             const d3 t = image_translation(s, mx, my, mz);
-            if (!body_overlap<KIND>(s, pp, a, rot, j, &t)) return false;
+            if constexpr (KIND != 3) {
+                // the FP32 filter on the rounded FP64 separation (its margins cover coarser ones);
+                // FP64 only inside the guard band: its dependent chain is most of a try's time
+                float3 d = sep;
+                if (mx | my | mz) {
+                    const d3 q = sub3(add3(load_d3(s.pos64 + 3 * (size_t)j), t), pp);
+                    d = make_float3(static_cast<float>(q.x), static_cast<float>(q.y), static_cast<float>(q.z));
+                }
+                const double *rj = s.rot64 + 9 * (size_t)j;
+                float3 ai = make_float3(0.f, 0.f, 0.f), aj = ai;
+                if (KIND == 1) {
+                    ai = make_float3(static_cast<float>(a.x), static_cast<float>(a.y), static_cast<float>(a.z));
+                    aj = make_float3(static_cast<float>(rj[2]), static_cast<float>(rj[5]), static_cast<float>(rj[8]));
+                }
+                const int cls = classify<KIND>(s.fc, d, ai, aj);
+                if (cls == 0) return false;
+                if (cls == 2 && !body_overlap<KIND>(s, pp, a, rot, j, &t)) return false;
+            } else if (!body_overlap<KIND>(s, pp, a, rot, j, &t)) {
+                return false;
+            }
             cnt++;
             return early;
         });
@@ -566,7 +585,7 @@ __device__ double move_energy(const SingleArgs &A, const Mover &mv, int pid, int
 }
 
 // One single move: the first warp builds the mover, TRY_WARPS warps share its candidates (a warp
-// alone walked a rod's 200 candidates in seven dependent rounds: 19 against 8 us a move), and the
+// alone walked a rod's 200 candidates in seven dependent rounds), and the
 // host reads the answer from page-locked memory.
 constexpr int TRY_WARPS = 8;
 template <int KIND>
