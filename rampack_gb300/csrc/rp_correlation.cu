@@ -71,6 +71,11 @@ struct CorrGeom {
     float hm32[3], tau32, kn32[3], bin_abs_lw;
     float edge32;    // no FP32 rejection when a folded relative separation is this near 1/2
     int fp64_only;   // RP_CORR_FP64_ONLY: no FP32 pre-filter
+    // radial pairs over three or more cells a side (k_corr_rows): the cell matrix (box column k / nc[k])
+    // in FP64 for the points' row coordinates and in FP32 for the row offsets, the squared reach and
+    // the bin margin with their error
+    double cell[9];
+    float cell32[9], row_thr2, row_margin;
 };
 
 struct SortedPoints {
@@ -80,6 +85,8 @@ struct SortedPoints {
     double *f64;      // [slot][3] focal point
     double *r64;      // [slot][3] relative focal point (inverse box x focal point)
     double *ax64;     // [slot][3] correlated axis (averaged correlations)
+    float4 *row32;    // position from the corner of the cell's row: cell matrix * (c0 + f0, f1, f2), c
+                      // and f the cell and in-cell coordinates
 };
 
 RP_HD double dsqrt(double x) {
@@ -155,6 +162,15 @@ __global__ void k_corr_scatter(CorrGeom G, const double *pos64, const double *ro
     double *fo = S.f64 + 3 * (int64_t)slot, *ro = S.r64 + 3 * (int64_t)slot;
     fo[0] = f.x, fo[1] = f.y, fo[2] = f.z;
     ro[0] = r.x, ro[1] = r.y, ro[2] = r.z;
+    if (S.row32) {
+        const double w[3] = {r.x - floor(r.x), r.y - floor(r.y), r.z - floor(r.z)};
+        const int c1 = (c / G.nc[0]) % G.nc[1], c2 = c / (G.nc[0] * G.nc[1]);
+        const double u0 = w[0] * G.nc[0], u1 = w[1] * G.nc[1] - c1, u2 = w[2] * G.nc[2] - c2;
+        float p[3];
+        for (int k = 0; k < 3; k++)
+            p[k] = static_cast<float>(G.cell[3 * k] * u0 + G.cell[3 * k + 1] * u1 + G.cell[3 * k + 2] * u2);
+        S.row32[slot] = make_float4(p[0], p[1], p[2], 0.f);
+    }
     if (want_axes) {
         d3 a = shape_axis(G, rot64 + 9 * i);
         double *ao = S.ax64 + 3 * (int64_t)slot;
@@ -406,6 +422,180 @@ __global__ void __launch_bounds__(CORR_THREADS, 2) k_corr_pairs(CorrGeom G, Sort
     }
 }
 
+// Radial pairs over a grid of three or more cells a side: one warp per focal point walks the rows of
+// its neighbourhood.  The cells of a row (same y and z) are consecutive slots, so a row is one
+// contiguous run of candidates (two where it wraps around the box), and their positions from the
+// row's corner differ from the focal point's by one offset per run: a pair costs one load, three
+// subtractions and a squared norm, where the general kernel folds relative coordinates and multiplies
+// by the box for each pair and looks up each candidate's cell (182 instructions per 32 pairs against
+// about 30; 6.9 against 1.5 ms for 10^9 pairs of 10^6 points).  In range, the bin is the integer part
+// of d / step unless d / step lies within `row_margin` of an integer or of the last bin's end; those
+// pairs are queued for decide_pair, and so are, for the averaged correlations, all in-range pairs
+// (with their bin), so that the FP64 axis functions run on full warps.  Counts are 32 bits wide per
+// block (`n` points in at most 2^32 pairs a block, else the general kernel).
+template <int F>
+__global__ void __launch_bounds__(CORR_THREADS) k_corr_rows(CorrGeom G, SortedPoints S, const int32_t *start, int64_t n,
+                                                            unsigned long long *hist, double *hsum,
+                                                            unsigned long long *tested) {
+    extern __shared__ unsigned long long sh[];
+    constexpr bool AVG = F != RP_CORR_DENSITY;
+    double *hs = reinterpret_cast<double *>(sh);                        // averaged correlations: value sums
+    uint32_t *hc = reinterpret_cast<uint32_t *>(sh + (AVG ? G.nb : 0));
+    for (int b = threadIdx.x; b < G.nb; b += blockDim.x) {
+        hc[b] = 0;
+        if (AVG) hs[b] = 0;
+    }
+    __shared__ int2 queue[CORR_THREADS / 32][64];
+    __shared__ int2 vqueue[AVG ? CORR_THREADS / 32 : 1][64];
+    __shared__ int vbin[AVG ? CORR_THREADS / 32 : 1][64];
+    __syncthreads();
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const unsigned lt = (1u << lane) - 1u;
+    int2 *q = queue[wib];
+    int qn = 0, vn = 0;
+    unsigned long long my_tested = 0;
+    // pairs for the FP64 decision: straight to the global histogram (few)
+    auto decide = [&](int cnt) {
+        if (lane < cnt) {
+            const int2 p = q[qn - cnt + lane];
+            const bool first = S.idx[p.x] <= S.idx[p.y];
+            decide_pair<RP_PAIRS_RADIAL, F>(G, S, first ? p.x : p.y, first ? p.y : p.x, hist, hsum);
+        }
+        qn -= cnt;
+        __syncwarp();
+    };
+    auto values = [&](int cnt) {   // averaged correlations: the binned pairs' values
+        if (lane < cnt) {
+            const int2 p = vqueue[AVG ? wib : 0][vn - cnt + lane];
+            const bool first = S.idx[p.x] <= S.idx[p.y];
+            const d3 x = load3(S.ax64, p.x), y = load3(S.ax64, p.y);
+            atomicAdd(hs + vbin[AVG ? wib : 0][vn - cnt + lane], axis_function<F>(first ? x : y, first ? y : x, d3{0.0, 0.0, 0.0}));
+        }
+        vn -= cnt;
+        __syncwarp();
+    };
+    const int wy = 2 * G.span[1] + 1, rows = wy * (2 * G.span[2] + 1);   // at most 25
+    const float inv = G.inv_step32, thr = G.row_thr2, half = 0.5f - G.row_margin, last = G.nb - G.row_margin;
+    const int64_t warps = (int64_t)gridDim.x * (CORR_THREADS / 32);
+    for (int64_t a = blockIdx.x * (int64_t)(CORR_THREADS / 32) + wib; a < n; a += warps) {
+        const int ca = S.cell[a];
+        const float4 pa = S.row32[a];
+        if (AVG) {   // the averaged correlations also take the pair (i, i)
+            if (lane == 0) q[qn] = make_int2(static_cast<int>(a), static_cast<int>(a));
+            qn++;
+            my_tested += lane == 0;
+            __syncwarp();
+            if (qn >= 32) decide(32);
+        }
+        const int cx = ca % G.nc[0], cy = (ca / G.nc[0]) % G.nc[1], cz = ca / (G.nc[0] * G.nc[1]);
+        // lane r holds row r: the run of cells cx - span .. cx + span inside the box and the wrapped rest
+        int b0[2] = {0, 0}, len[2] = {0, 0}, sx = 0;
+        if (lane < rows) {
+            const int oy = lane % wy - G.span[1], oz = lane / wy - G.span[2];
+            int y = cy + oy, z = cz + oz;
+            y += y < 0 ? G.nc[1] : (y >= G.nc[1] ? -G.nc[1] : 0);
+            z += z < 0 ? G.nc[2] : (z >= G.nc[2] ? -G.nc[2] : 0);
+            const int row = (z * G.nc[1] + y) * G.nc[0];
+            const int lo = cx - G.span[0], hi = cx + G.span[0];
+            int c0[2] = {max(lo, 0), 0}, c1[2] = {min(hi, G.nc[0] - 1), -1};
+            if (lo < 0) {
+                c0[1] = lo + G.nc[0], c1[1] = G.nc[0] - 1, sx = -1;
+            } else if (hi >= G.nc[0]) {
+                c0[1] = 0, c1[1] = hi - G.nc[0], sx = 1;
+            }
+            for (int u = 0; u < 2; u++)
+                if (c1[u] >= c0[u]) {
+                    b0[u] = max(start[row + c0[u]], static_cast<int>(a) + 1);
+                    len[u] = max(start[row + c1[u] + 1] - b0[u], 0);
+                }
+        }
+        unsigned todo = __ballot_sync(full, len[0] + len[1] > 0);
+        for (; todo; todo &= todo - 1) {
+            const int r = __ffs(todo) - 1;
+            const float oy = (float)(r % wy - G.span[1]), oz = (float)(r / wy - G.span[2]);
+#pragma unroll 1
+            for (int u = 0; u < 2; u++) {
+                const int cnt = __shfl_sync(full, len[u], r);
+                if (cnt == 0) continue;
+                const int first = __shfl_sync(full, b0[u], r);
+                const float ox = u == 0 ? 0.f : (float)(__shfl_sync(full, sx, r) * G.nc[0]);
+                const float ax = pa.x - (G.cell32[0] * ox + G.cell32[1] * oy + G.cell32[2] * oz);
+                const float ay = pa.y - (G.cell32[3] * ox + G.cell32[4] * oy + G.cell32[5] * oz);
+                const float az = pa.z - (G.cell32[6] * ox + G.cell32[7] * oy + G.cell32[8] * oz);
+#pragma unroll 2
+                for (int k = lane; k - lane < cnt; k += 32) {
+                    bool need = false, in = false;
+                    int bin = 0;
+                    if (k < cnt) {
+                        const float4 pb = S.row32[first + k];
+                        const float dx = pb.x - ax, dy = pb.y - ay, dz = pb.z - az;
+                        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                        if (d2 <= thr) {
+                            const float t = __fsqrt_rn(d2) * inv, fl = floorf(t);
+                            bin = (int)fl;
+                            need = !(fabsf(t - fl - 0.5f) < half && t < last);
+                            in = !need;
+                            if (in) atomicAdd(hc + bin, 1u);
+                        }
+                    }
+                    const unsigned bal = __ballot_sync(full, need);
+                    if (bal) {
+                        if (need) {
+                            q[qn + __popc(bal & lt)] = make_int2(static_cast<int>(a), first + k);
+                            my_tested++;
+                        }
+                        qn += __popc(bal);
+                        __syncwarp();
+                        if (qn >= 32) decide(32);
+                    }
+                    if (AVG) {
+                        const unsigned vb = __ballot_sync(full, in);
+                        if (in) {
+                            vqueue[wib][vn + __popc(vb & lt)] = make_int2(static_cast<int>(a), first + k);
+                            vbin[wib][vn + __popc(vb & lt)] = bin;
+                        }
+                        vn += __popc(vb);
+                        __syncwarp();
+                        if (vn >= 32) values(32);
+                    }
+                }
+            }
+        }
+    }
+    if (qn > 0) decide(qn);
+    if (AVG && vn > 0) values(vn);
+    for (int o = 16; o > 0; o >>= 1) my_tested += __shfl_xor_sync(full, my_tested, o);
+    if (lane == 0 && my_tested) atomicAdd(tested, my_tested);
+    __syncthreads();
+    for (int b = threadIdx.x; b < G.nb; b += blockDim.x) {
+        if (hc[b]) atomicAdd(hist + b, (unsigned long long)hc[b]);
+        if (AVG && hs[b] != 0.0) atomicAdd(hsum + b, hs[b]);
+    }
+}
+
+template <int F>
+cudaError_t launch_rows_t(const CorrGeom &G, const SortedPoints &S, const int32_t *start, int64_t n, int grid,
+                          unsigned long long *hist, double *hsum, unsigned long long *tested, cudaStream_t st) {
+    const size_t smem = size_t(G.nb) * (F != RP_CORR_DENSITY ? 12 : 4);
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(k_corr_rows<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        if (e != cudaSuccess) return e;
+    }
+    k_corr_rows<F><<<grid, CORR_THREADS, smem, st>>>(G, S, start, n, hist, hsum, tested);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_rows(int f, const CorrGeom &G, const SortedPoints &S, const int32_t *start, int64_t n, int grid,
+                        unsigned long long *hist, double *hsum, unsigned long long *tested, cudaStream_t st) {
+    switch (f) {
+        case RP_CORR_DENSITY: return launch_rows_t<RP_CORR_DENSITY>(G, S, start, n, grid, hist, hsum, tested, st);
+        case RP_CORR_S110: return launch_rows_t<RP_CORR_S110>(G, S, start, n, grid, hist, hsum, tested, st);
+        case RP_CORR_S220: return launch_rows_t<RP_CORR_S220>(G, S, start, n, grid, hist, hsum, tested, st);
+        default: return launch_rows_t<RP_CORR_AXES_ANGLE>(G, S, start, n, grid, hist, hsum, tested, st);
+    }
+}
+
 template <int E, int F>
 cudaError_t launch_pairs_t(const CorrGeom &G, const SortedPoints &S, const int32_t *start, int64_t n, int grid,
                            int use_smem, size_t smem, unsigned long long *hist, double *hsum,
@@ -466,7 +656,7 @@ struct Corr {
     }
     void free_points() {
         for (void *p : {(void *)cell_of, (void *)S.idx, (void *)S.cell, (void *)S.rel32, (void *)S.f64,
-                        (void *)S.r64, (void *)S.ax64, (void *)focal_out})
+                        (void *)S.r64, (void *)S.ax64, (void *)S.row32, (void *)focal_out})
             if (p) cudaFree(p);
         cell_of = nullptr;
         S = SortedPoints{};
@@ -576,6 +766,7 @@ int ensure_buffers(Corr *c, const PackingView &v, int64_t ncell, bool axes) {
         CORR_CUDA(c, cudaMalloc(&c->S.idx, sizeof(int32_t) * m));
         CORR_CUDA(c, cudaMalloc(&c->S.cell, sizeof(int32_t) * m));
         CORR_CUDA(c, cudaMalloc(&c->S.rel32, sizeof(float4) * m));
+        CORR_CUDA(c, cudaMalloc(&c->S.row32, sizeof(float4) * m));
         CORR_CUDA(c, cudaMalloc(&c->S.f64, sizeof(double) * 3 * m));
         CORR_CUDA(c, cudaMalloc(&c->S.r64, sizeof(double) * 3 * m));
         CORR_CUDA(c, cudaMalloc(&c->focal_out, sizeof(double) * 3 * m));
@@ -717,6 +908,27 @@ int add_snapshot(Corr *c, void *handle) {
         }
     }
     G.ncell = static_cast<int>(ncell);
+    // the row kernel's coordinates: a point's row position, at most M_i in component i, and a row
+    // offset, at most O_i, are rounded to FP32, the offset's sums (3), the shifted position (M + O)
+    // and the difference (2 M) round again: in all 2^-24 (4 M_i + 5 O_i), taken 1.5 times
+    bool by_rows = d.enumerator == RP_PAIRS_RADIAL && d.function != RP_CORR_S221 && !G.fp64_only && d.num_bins <= SMEM_BINS &&
+                   G.span[0] > 0 && G.span[1] > 0 && G.span[2] > 0;
+    {
+        double e2 = 0;
+        for (int i = 0; i < 3; i++) {
+            for (int k = 0; k < 3; k++) {
+                G.cell[3 * i + k] = v.box[3 * i + k] / G.nc[k];
+                G.cell32[3 * i + k] = static_cast<float>(G.cell[3 * i + k]);
+            }
+            const double row = std::abs(v.box[3 * i]), across = std::abs(G.cell[3 * i + 1]) + std::abs(G.cell[3 * i + 2]);
+            const double e = std::ldexp(4 * (row + across) + 5 * (row + 2 * across), -24);
+            e2 += e * e;
+        }
+        const double m_row = 1.5 * std::sqrt(e2), reach_row = d.max_r * (1 + 1e-6) + m_row;
+        G.row_thr2 = static_cast<float>(reach_row * reach_row * (1 + 1e-6));
+        G.row_margin = static_cast<float>(m_row / G.step * (1 + 1e-6) + 1e-6 * d.num_bins);
+        by_rows = by_rows && G.row_margin < 0.25f;
+    }
 
     rc = ensure_buffers(c, v, ncell, axes);
     if (rc != RP_OK) return rc;
@@ -762,7 +974,14 @@ int add_snapshot(Corr *c, void *handle) {
         const int use_smem = nb <= SMEM_BINS ? 1 : 0;
         const size_t smem = use_smem ? size_t(nb) * (axes ? 16 : 8) : 0;
         cudaError_t le;
-        if (d.enumerator == RP_PAIRS_RADIAL)
+        if (by_rows) {
+            // a block's pairs fit its 32-bit counts
+            int64_t blocks = std::min<int64_t>(wblk, int64_t(dev_sms) * 8);
+            const int64_t wpb = CORR_THREADS / 32;
+            while (blocks < wblk && (v.n + blocks * wpb - 1) / (blocks * wpb) * wpb > (int64_t(1) << 32) / v.n) blocks *= 2;
+            le = launch_rows(d.function, G, c->S, c->start, v.n, static_cast<int>(std::min(blocks, wblk)), c->hist, c->hsum,
+                             c->tested, st);
+        } else if (d.enumerator == RP_PAIRS_RADIAL)
             le = launch_pairs_e<RP_PAIRS_RADIAL>(d.function, G, c->S, c->start, v.n, grid, use_smem, smem, c->hist,
                                                  c->hsum, c->tested, st);
         else if (d.enumerator == RP_PAIRS_LINEAR)
