@@ -422,19 +422,21 @@ __global__ void __launch_bounds__(CORR_THREADS, 2) k_corr_pairs(CorrGeom G, Sort
     }
 }
 
-// Radial pairs over a grid of three or more cells a side: one warp per focal point walks the rows of
-// its neighbourhood.  The cells of a row (same y and z) are consecutive slots, so a row is one
-// contiguous run of candidates (two where it wraps around the box), and their positions from the
-// row's corner differ from the focal point's by one offset per run: a pair costs one load, three
-// subtractions and a squared norm, where the general kernel folds relative coordinates and multiplies
-// by the box for each pair and looks up each candidate's cell (182 instructions per 32 pairs against
-// about 30; 6.9 against 1.5 ms for 10^9 pairs of 10^6 points).  In range, the bin is the integer part
-// of d / step unless d / step lies within `row_margin` of an integer or of the last bin's end; those
-// pairs are queued for decide_pair, and so are, for the averaged correlations, all in-range pairs
+// Radial pairs over a grid of three or more cells a side: one warp per cell walks the rows of its
+// neighbourhood, ROW_POINTS of its points at a time.  The cells of a row (same y and z) are consecutive
+// slots, so a row is one contiguous run of candidates (two where it wraps around the box), and their
+// positions from the row's corner differ from the cell's points' by one offset per run: a pair costs
+// three subtractions, a squared norm and the bin, and a load is shared by ROW_POINTS pairs, where the
+// general kernel folds relative coordinates and multiplies by the box for each pair and looks up each
+// candidate's cell (182 instructions per 32 pairs).  The kernel is bound by issue slots; the snapshot of
+// 10^6 points with 10^9 candidate pairs went from 7.28 to 2.54 ms.  In range, the bin is the integer
+// part of d / step unless d / step lies within `row_margin` of an integer or of the last bin's end;
+// those pairs are queued for decide_pair, and so are, for the averaged correlations, all in-range pairs
 // (with their bin), so that the FP64 axis functions run on full warps.  Counts are 32 bits wide per
-// block (`n` points in at most 2^32 pairs a block, else the general kernel).
+// block; the host gives every block at most 2^32 pairs.
+constexpr int ROW_POINTS = 4;   // 2.87, 2.54 and 2.55 ms a snapshot of 10^6 points for 2, 4 and 8
 template <int F>
-__global__ void __launch_bounds__(CORR_THREADS) k_corr_rows(CorrGeom G, SortedPoints S, const int32_t *start, int64_t n,
+__global__ void __launch_bounds__(CORR_THREADS) k_corr_rows(CorrGeom G, SortedPoints S, const int32_t *start,
                                                             unsigned long long *hist, double *hsum,
                                                             unsigned long long *tested) {
     extern __shared__ unsigned long long sh[];
@@ -477,20 +479,15 @@ __global__ void __launch_bounds__(CORR_THREADS) k_corr_rows(CorrGeom G, SortedPo
     };
     const int wy = 2 * G.span[1] + 1, rows = wy * (2 * G.span[2] + 1);   // at most 25
     const float inv = G.inv_step32, thr = G.row_thr2, half = 0.5f - G.row_margin, last = G.nb - G.row_margin;
-    const int64_t warps = (int64_t)gridDim.x * (CORR_THREADS / 32);
-    for (int64_t a = blockIdx.x * (int64_t)(CORR_THREADS / 32) + wib; a < n; a += warps) {
-        const int ca = S.cell[a];
-        const float4 pa = S.row32[a];
-        if (AVG) {   // the averaged correlations also take the pair (i, i)
-            if (lane == 0) q[qn] = make_int2(static_cast<int>(a), static_cast<int>(a));
-            qn++;
-            my_tested += lane == 0;
-            __syncwarp();
-            if (qn >= 32) decide(32);
-        }
-        const int cx = ca % G.nc[0], cy = (ca / G.nc[0]) % G.nc[1], cz = ca / (G.nc[0] * G.nc[1]);
-        // lane r holds row r: the run of cells cx - span .. cx + span inside the box and the wrapped rest
-        int b0[2] = {0, 0}, len[2] = {0, 0}, sx = 0;
+    const int warps = gridDim.x * (CORR_THREADS / 32);
+    for (int cell = blockIdx.x * (CORR_THREADS / 32) + wib; cell < G.ncell; cell += warps) {
+        const int s0 = start[cell], occ = start[cell + 1] - s0;
+        if (occ == 0) continue;
+        const int cx = cell % G.nc[0], cy = (cell / G.nc[0]) % G.nc[1], cz = cell / (G.nc[0] * G.nc[1]);
+        // lane r holds row r: the run of cells cx - span .. cx + span inside the box, the wrapped rest
+        // (both cut to the slots above the cell's first), and the row's offset
+        int first0 = 0, end0 = 0, first1 = 0, end1 = 0, sx = 0;
+        float offx = 0.f, offy = 0.f, offz = 0.f;
         if (lane < rows) {
             const int oy = lane % wy - G.span[1], oz = lane / wy - G.span[2];
             int y = cy + oy, z = cz + oz;
@@ -498,67 +495,106 @@ __global__ void __launch_bounds__(CORR_THREADS) k_corr_rows(CorrGeom G, SortedPo
             z += z < 0 ? G.nc[2] : (z >= G.nc[2] ? -G.nc[2] : 0);
             const int row = (z * G.nc[1] + y) * G.nc[0];
             const int lo = cx - G.span[0], hi = cx + G.span[0];
-            int c0[2] = {max(lo, 0), 0}, c1[2] = {min(hi, G.nc[0] - 1), -1};
+            auto run = [&](int c0, int c1, int &from, int &to) {
+                from = max(start[row + c0], s0 + 1);
+                to = start[row + c1 + 1];
+            };
+            run(max(lo, 0), min(hi, G.nc[0] - 1), first0, end0);
             if (lo < 0) {
-                c0[1] = lo + G.nc[0], c1[1] = G.nc[0] - 1, sx = -1;
+                run(lo + G.nc[0], G.nc[0] - 1, first1, end1);
+                sx = -1;
             } else if (hi >= G.nc[0]) {
-                c0[1] = 0, c1[1] = hi - G.nc[0], sx = 1;
+                run(0, hi - G.nc[0], first1, end1);
+                sx = 1;
             }
-            for (int u = 0; u < 2; u++)
-                if (c1[u] >= c0[u]) {
-                    b0[u] = max(start[row + c0[u]], static_cast<int>(a) + 1);
-                    len[u] = max(start[row + c1[u] + 1] - b0[u], 0);
-                }
+            offx = G.cell32[1] * oy + G.cell32[2] * oz;
+            offy = G.cell32[4] * oy + G.cell32[5] * oz;
+            offz = G.cell32[7] * oy + G.cell32[8] * oz;
         }
-        unsigned todo = __ballot_sync(full, len[0] + len[1] > 0);
-        for (; todo; todo &= todo - 1) {
-            const int r = __ffs(todo) - 1;
-            const float oy = (float)(r % wy - G.span[1]), oz = (float)(r / wy - G.span[2]);
+        const unsigned any = __ballot_sync(full, end0 > first0 || end1 > first1);
+        // the cell's points, ROW_POINTS at a time: a candidate is loaded once for all of them
+        for (int i = 0; i < occ; i += ROW_POINTS) {
+            const int a0 = s0 + i, np = min(ROW_POINTS, occ - i);
+            float4 pa[ROW_POINTS];
+#pragma unroll
+            for (int p = 0; p < ROW_POINTS; p++) pa[p] = S.row32[a0 + min(p, np - 1)];
+            if (AVG) {   // the averaged correlations also take the pairs (i, i)
+                if (lane < np) {
+                    q[qn + lane] = make_int2(a0 + lane, a0 + lane);
+                    my_tested++;
+                }
+                qn += np;
+                __syncwarp();
+                if (qn >= 32) decide(32);
+            }
+            for (unsigned todo = any; todo; todo &= todo - 1) {
+                const int r = __ffs(todo) - 1;
+                int first = max(__shfl_sync(full, first0, r), a0 + 1), end = __shfl_sync(full, end0, r);
+                float x = __shfl_sync(full, offx, r), y = __shfl_sync(full, offy, r), z = __shfl_sync(full, offz, r);
+                for (bool wrapped = false;; wrapped = true) {
 #pragma unroll 1
-            for (int u = 0; u < 2; u++) {
-                const int cnt = __shfl_sync(full, len[u], r);
-                if (cnt == 0) continue;
-                const int first = __shfl_sync(full, b0[u], r);
-                const float ox = u == 0 ? 0.f : (float)(__shfl_sync(full, sx, r) * G.nc[0]);
-                const float ax = pa.x - (G.cell32[0] * ox + G.cell32[1] * oy + G.cell32[2] * oz);
-                const float ay = pa.y - (G.cell32[3] * ox + G.cell32[4] * oy + G.cell32[5] * oz);
-                const float az = pa.z - (G.cell32[6] * ox + G.cell32[7] * oy + G.cell32[8] * oz);
-#pragma unroll 2
-                for (int k = lane; k - lane < cnt; k += 32) {
-                    bool need = false, in = false;
-                    int bin = 0;
-                    if (k < cnt) {
-                        const float4 pb = S.row32[first + k];
-                        const float dx = pb.x - ax, dy = pb.y - ay, dz = pb.z - az;
-                        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                        if (d2 <= thr) {
-                            const float t = __fsqrt_rn(d2) * inv, fl = floorf(t);
-                            bin = (int)fl;
-                            need = !(fabsf(t - fl - 0.5f) < half && t < last);
-                            in = !need;
-                            if (in) atomicAdd(hc + bin, 1u);
+                    for (int base = first; base < end; base += 32) {
+                        const int b = min(base + lane, end - 1);
+                        float4 pb = S.row32[b];
+                        pb.x += x;
+                        pb.y += y;
+                        pb.z += z;
+                        // a point takes candidates above its own slot (none for a point that is not there)
+                        const int ahead = base + lane < end ? b - a0 : 0;
+                        unsigned need = 0, in = 0;
+                        int bin[ROW_POINTS];
+#pragma unroll
+                        for (int p = 0; p < ROW_POINTS; p++) {
+                            const float dx = pb.x - pa[p].x, dy = pb.y - pa[p].y, dz = pb.z - pa[p].z;
+                            const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                            const bool near = d2 <= thr && ahead > p && p < np;
+                            // the bin by a sum that rounds to the nearest integer (NaN at d2 = 0: FP64)
+                            const float t = d2 * rsqrtf(d2) * inv - 0.5f;
+                            const float kf = t + 12582912.f;
+                            bin[p] = __float_as_int(kf) - 0x4b400000;
+                            const bool sure = t < last - 0.5f && fabsf(t - (kf - 12582912.f)) < half;
+                            if (near && sure) {
+                                atomicAdd(hc + bin[p], 1u);
+                                if (AVG) in |= 1u << p;
+                            }
+                            if (near && !sure) need |= 1u << p;
+                        }
+                        if (__any_sync(full, need)) {
+                            for (int p = 0; p < ROW_POINTS; p++) {
+                                const bool me = (need >> p) & 1u;
+                                const unsigned bal = __ballot_sync(full, me);
+                                if (me) {
+                                    q[qn + __popc(bal & lt)] = make_int2(a0 + p, b);
+                                    my_tested++;
+                                }
+                                qn += __popc(bal);
+                                __syncwarp();
+                                if (qn >= 32) decide(32);
+                            }
+                        }
+                        if (AVG) {
+#pragma unroll
+                            for (int p = 0; p < ROW_POINTS; p++) {
+                                const bool me = (in >> p) & 1u;
+                                const unsigned bal = __ballot_sync(full, me);
+                                if (me) {
+                                    vqueue[wib][vn + __popc(bal & lt)] = make_int2(a0 + p, b);
+                                    vbin[wib][vn + __popc(bal & lt)] = bin[p];
+                                }
+                                vn += __popc(bal);
+                                __syncwarp();
+                                if (vn >= 32) values(32);
+                            }
                         }
                     }
-                    const unsigned bal = __ballot_sync(full, need);
-                    if (bal) {
-                        if (need) {
-                            q[qn + __popc(bal & lt)] = make_int2(static_cast<int>(a), first + k);
-                            my_tested++;
-                        }
-                        qn += __popc(bal);
-                        __syncwarp();
-                        if (qn >= 32) decide(32);
-                    }
-                    if (AVG) {
-                        const unsigned vb = __ballot_sync(full, in);
-                        if (in) {
-                            vqueue[wib][vn + __popc(vb & lt)] = make_int2(static_cast<int>(a), first + k);
-                            vbin[wib][vn + __popc(vb & lt)] = bin;
-                        }
-                        vn += __popc(vb);
-                        __syncwarp();
-                        if (vn >= 32) values(32);
-                    }
+                    if (wrapped) break;
+                    first = max(__shfl_sync(full, first1, r), a0 + 1);
+                    end = __shfl_sync(full, end1, r);
+                    if (end <= first) break;
+                    const float ox = (float)(__shfl_sync(full, sx, r) * G.nc[0]);
+                    x += G.cell32[0] * ox;
+                    y += G.cell32[3] * ox;
+                    z += G.cell32[6] * ox;
                 }
             }
         }
@@ -575,24 +611,24 @@ __global__ void __launch_bounds__(CORR_THREADS) k_corr_rows(CorrGeom G, SortedPo
 }
 
 template <int F>
-cudaError_t launch_rows_t(const CorrGeom &G, const SortedPoints &S, const int32_t *start, int64_t n, int grid,
+cudaError_t launch_rows_t(const CorrGeom &G, const SortedPoints &S, const int32_t *start, int grid,
                           unsigned long long *hist, double *hsum, unsigned long long *tested, cudaStream_t st) {
     const size_t smem = size_t(G.nb) * (F != RP_CORR_DENSITY ? 12 : 4);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(k_corr_rows<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         if (e != cudaSuccess) return e;
     }
-    k_corr_rows<F><<<grid, CORR_THREADS, smem, st>>>(G, S, start, n, hist, hsum, tested);
+    k_corr_rows<F><<<grid, CORR_THREADS, smem, st>>>(G, S, start, hist, hsum, tested);
     return cudaGetLastError();
 }
 
-cudaError_t launch_rows(int f, const CorrGeom &G, const SortedPoints &S, const int32_t *start, int64_t n, int grid,
+cudaError_t launch_rows(int f, const CorrGeom &G, const SortedPoints &S, const int32_t *start, int grid,
                         unsigned long long *hist, double *hsum, unsigned long long *tested, cudaStream_t st) {
     switch (f) {
-        case RP_CORR_DENSITY: return launch_rows_t<RP_CORR_DENSITY>(G, S, start, n, grid, hist, hsum, tested, st);
-        case RP_CORR_S110: return launch_rows_t<RP_CORR_S110>(G, S, start, n, grid, hist, hsum, tested, st);
-        case RP_CORR_S220: return launch_rows_t<RP_CORR_S220>(G, S, start, n, grid, hist, hsum, tested, st);
-        default: return launch_rows_t<RP_CORR_AXES_ANGLE>(G, S, start, n, grid, hist, hsum, tested, st);
+        case RP_CORR_DENSITY: return launch_rows_t<RP_CORR_DENSITY>(G, S, start, grid, hist, hsum, tested, st);
+        case RP_CORR_S110: return launch_rows_t<RP_CORR_S110>(G, S, start, grid, hist, hsum, tested, st);
+        case RP_CORR_S220: return launch_rows_t<RP_CORR_S220>(G, S, start, grid, hist, hsum, tested, st);
+        default: return launch_rows_t<RP_CORR_AXES_ANGLE>(G, S, start, grid, hist, hsum, tested, st);
     }
 }
 
@@ -973,14 +1009,23 @@ int add_snapshot(Corr *c, void *handle) {
         const int grid = static_cast<int>(std::min<int64_t>(wblk, int64_t(dev_sms) * 6));
         const int use_smem = nb <= SMEM_BINS ? 1 : 0;
         const size_t smem = use_smem ? size_t(nb) * (axes ? 16 : 8) : 0;
-        cudaError_t le;
+        cudaError_t le = cudaSuccess;
+        int32_t occ = 0;
         if (by_rows) {
-            // a block's pairs fit its 32-bit counts
-            int64_t blocks = std::min<int64_t>(wblk, int64_t(dev_sms) * 8);
-            const int64_t wpb = CORR_THREADS / 32;
-            while (blocks < wblk && (v.n + blocks * wpb - 1) / (blocks * wpb) * wpb > (int64_t(1) << 32) / v.n) blocks *= 2;
-            le = launch_rows(d.function, G, c->S, c->start, v.n, static_cast<int>(std::min(blocks, wblk)), c->hist, c->hsum,
-                             c->tested, st);
+            // a block's pairs fit its 32-bit counts: at most max_occ points of each of its cells, each
+            // with every point of 125 cells
+            CORR_CUDA(c, cudaMemcpyAsync(&occ, c->max_occ, sizeof(occ), cudaMemcpyDeviceToHost, st));
+            CORR_CUDA(c, cudaStreamSynchronize(st));
+            const int64_t wpb = CORR_THREADS / 32, cblk = (ncell + wpb - 1) / wpb;
+            int64_t blocks = std::min<int64_t>(cblk, int64_t(dev_sms) * 8);
+            const double most = 125.0 * occ * occ;   // pairs of one cell
+            while (blocks < cblk && static_cast<double>((cblk + blocks - 1) / blocks * wpb) * most > 4.2e9) blocks *= 2;
+            by_rows = wpb * most <= 4.2e9;
+            if (by_rows)
+                le = launch_rows(d.function, G, c->S, c->start, static_cast<int>(std::min(blocks, cblk)), c->hist, c->hsum,
+                                 c->tested, st);
+        }
+        if (by_rows) {
         } else if (d.enumerator == RP_PAIRS_RADIAL)
             le = launch_pairs_e<RP_PAIRS_RADIAL>(d.function, G, c->S, c->start, v.n, grid, use_smem, smem, c->hist,
                                                  c->hsum, c->tested, st);
