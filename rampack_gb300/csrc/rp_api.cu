@@ -250,6 +250,9 @@ struct Handle {
     double *cthr64 = nullptr;
     double *cbody_dev = nullptr;    // body-frame centres on the device
     XcShape *d_xc = nullptr;        // generic convex bodies: the geometry on the device
+    double xc_insphere = 0;
+    bool xc_flat = false;           // the body takes the sweep's FP32 pair test
+    bool xc_parts = false;
     // batched replicas: the batch owns the rotation table, counters, status word and the
     // device copy of the ActiveDomain bounds (setup_grid leaves the bounds in bounds_host)
     bool batch_member = false;
@@ -452,6 +455,7 @@ DevState dev_state(Handle *h) {
     s.n = h->n;
     s.kind = h->shape.kind;
     s.xc = h->d_xc;
+    s.xc_parts = h->xc_parts ? 1 : 0;
     std::memcpy(s.box, h->box, sizeof(s.box));
     std::memcpy(s.inv, h->inv, sizeof(s.inv));
     for (int i = 0; i < 3; i++) {
@@ -518,7 +522,9 @@ DevState dev_state(Handle *h) {
     }
     // ---- FP32 filter margins for the current grid ----
     const GridHost &g = h->grid[h->gcur];
-    FilterConsts fc = hard_filter_consts(h->shape.kind, h->shape.radius, h->shape.length, cell_lrow(g), h->box);
+    FilterConsts fc = hard_filter_consts(h->shape.kind, h->shape.radius,
+                                         h->shape.kind == RP_SHAPE_CONVEX ? h->xc_insphere : h->shape.length,
+                                         cell_lrow(g), h->box);
     if (h->shape.kind == RP_SHAPE_POLYSPHERE) {
         // bodies whose centres are farther apart than twice the largest centre reach
         // (|c| + r) cannot touch; the centre-pair thresholds live in the grid (setup_grid)
@@ -634,6 +640,7 @@ int setup_grid(Handle *h, GridHost &G, const double *box, const double *shift) {
         RP_CUDA(h, cudaMalloc(&g.maxis, sizeof(float4) * n));
         RP_CUDA(h, cudaMalloc(&g.plocal, sizeof(float4) * n));
         RP_CUDA(h, cudaMalloc(&g.max_occ, sizeof(int32_t)));
+        if (h->xc_flat) RP_CUDA(h, cudaMalloc(&g.mrot, sizeof(float4) * 3 * n));
         if (h->ncen > 0) {
             RP_CUDA(h, cudaMalloc(&g.mcen, sizeof(float4) * n * h->ncen));
             if (h->segs) RP_CUDA(h, cudaMalloc(&g.mhax, sizeof(float4) * n * h->ncen));
@@ -717,7 +724,7 @@ int setup_grid(Handle *h, GridHost &G, const double *box, const double *shift) {
     // neighbourhood plus four standard deviations (the rare larger neighbourhood reruns in the
     // overflow pass; larger neighbourhoods keep a warp per cell)
     G.cap_half = 0;
-    if (h->shape.kind != RP_SHAPE_POLYSPHERE) {
+    if (h->shape.kind == RP_SHAPE_SPHERE || h->shape.kind == RP_SHAPE_SPHEROCYLINDER) {
         const int half_max = static_cast<int>(224 * 1024 / (SWEEP_WARPS * 2 * 4) /
                                               (sweep_smem_per_half(h->shape.kind, 16) / 16)) / 16 * 16;
         if (mean + 4.0 * std::sqrt(mean) + 16.0 <= half_max) G.cap_half = std::min(G.cap, half_max);
@@ -1295,6 +1302,9 @@ int rp_create_convex(const char *script, int64_t n, int device, void **handle) {
     h->range = 2 * xs->circ;
     h->ref_range = h->range;
     h->total_range = h->range;
+    h->xc_insphere = xs->insph;
+    h->xc_flat = xs->flat && xs->f32_sound;
+    h->xc_parts = xs->flat32.nent > 0;
     int rc = create_common(h, n, device, handle);
     if (rc) {
         delete xs;
@@ -1372,6 +1382,7 @@ int rp_destroy(void *handle) {
         if (!h->batch_member) cudaFree(g.bounds);
         cudaFree(g.max_occ);
         cudaFree(g.mcen);
+        cudaFree(g.mrot);
         cudaFree(g.mhax);
         cudaFree(g.cthr);
     }
@@ -1774,8 +1785,12 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     const bool soft32 = h->soft && h->shape.kind == RP_SHAPE_SPHERE && !h->counting && !(p->flags & RP_SWEEP_FP64_ONLY) &&
                         !h->grid[h->gcur].no_ng && g.dims[0] >= 3 && g.dims[1] >= 3 && g.dims[2] >= 3 &&
                         (h->soft_only || !h->walls);
-    const bool fp64_sweep = (h->soft && !soft32) || h->shape.kind == RP_SHAPE_CONVEX;
-    if ((soft32 || fp64_sweep) && types == SWEEP_ROTOTRANSLATION)
+    // flat convex bodies take the FP32 sweep over such a grid too, with the pairs near contact in FP64
+    const bool convex = h->shape.kind == RP_SHAPE_CONVEX;
+    const bool convex32 = convex && h->xc_flat && !h->counting && !h->walls && !(p->flags & RP_SWEEP_FP64_ONLY) &&
+                          !h->grid[h->gcur].no_ng && g.dims[0] >= 3 && g.dims[1] >= 3 && g.dims[2] >= 3;
+    const bool fp64_sweep = (h->soft && !soft32) || (convex && !convex32);
+    if ((soft32 || convex || fp64_sweep) && types == SWEEP_ROTOTRANSLATION)
         return fail(h, RP_ERR_UNSUPPORTED, "rototranslations with a soft part or a convex body");
     std::vector<int> phases;
     grid_phases(g, r.d, phases);
@@ -1803,7 +1818,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     // active cell of a phase gets a warp there (1000 spheres: 180 -> 45 us a sweep; with more cells
     // than that the whole chip's warps are worth the launches)
     int cl_warps = 0;
-    if (!fp64_sweep && !h->bulk_stage && h->cells_per_warp == 1 && h->order_mode == RP_ORDER_OFF && h->pair_cap == 0 &&
+    if (!fp64_sweep && !convex && !h->bulk_stage && h->cells_per_warp == 1 && h->order_mode == RP_ORDER_OFF && h->pair_cap == 0 &&
         h->n <= CLUSTER_MAX_N && g.ncell <= CLUSTER_MAX_CELLS) {
         if (h->cl_blocks < 0) h->cl_blocks = cluster_blocks();
         int most = 0, act[3];
@@ -1922,7 +1937,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         }
         // two cells per warp for the plain scans of spheres and spherocylinders
         const GridHost &gh = h->grid[h->gcur];
-        const bool half = h->cells_per_warp == 2 && gh.cap_half > 0 && !h->counting && !soft32 && types != SWEEP_ROTOTRANSLATION &&
+        const bool half = h->cells_per_warp == 2 && gh.cap_half > 0 && !convex && !h->counting && !soft32 && types != SWEEP_ROTOTRANSLATION &&
                           a.partners == nullptr && a.pair_every == 0;
         if (half && h->half_cap_cached != gh.cap_half) {
             h->half_blocks = sweep_half_blocks_per_sm(h->shape.kind, gh.cap_half);

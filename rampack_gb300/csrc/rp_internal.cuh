@@ -30,14 +30,15 @@ enum : uint32_t {
 // re-decided in FP64 (the guard band).
 struct FilterConsts {
     float sphere_lo, sphere_hi;   // spheres: (2r)^2 -/+ margin
-    float core_lo, core_hi;       // spherocylinders: 4 r^2 -/+ margin
-    float far_lo, far_hi;         // spherocylinders: (2r + l)^2 -/+ margin
+    float core_lo, core_hi;       // spherocylinders: 4 r^2 -/+ margin; convex bodies: (2 insphere)^2
+    float far_lo, far_hi;         // spherocylinders: (2r + l)^2 -/+ margin; convex bodies: (2 circumsphere)^2
     float core_thr;               // 4 r^2
     float seg_err;                // bound on |f32 - f| of the segment distance^2
     float s2_min;                 // sin^2 of the axes' angle below which FP64 decides
     float s2_par;                 // sin^2 below which FP64 certainly takes its parallel branch
     float par_err;                // bound on that branch's excess over the true minimum
     float half_len;               // l / 2
+    float xc_scale, xc_err;       // convex bodies: two circumsphere radii; a bound on the separation's error
     float cell_margin;            // relative in-cell margin of the FP32 ActiveDomain test
     // soft part: bound of an FP32 separation's error, sigma^2, cut-off^2, the reach^2 of pairs to
     // evaluate (cut-off^2 and a margin), 4 eps and eps, an energy error floor per move
@@ -74,6 +75,7 @@ struct GridDev {
     // polyspheres
     float4 *mcen;         // [n][ncen] FP32 rotated centre offsets, cell order
     float4 *mhax;         // [n][ncen] FP32 rotated half axes (polyspherocylinders), cell order
+    float4 *mrot;         // [n][3] FP32 orientation rows, cell order (convex bodies)
     float *cthr;          // [3][MAX_CEN^2] FP32 centre-pair thresholds: (r_a + r_b)^2 - margin, the upper one
                           // + margin, and (r_a + r_b)^2 itself (the segment stage adds its own margin)
     // staging filter (cells well above the interaction range): a neighbour is staged only
@@ -95,6 +97,7 @@ struct DevState {
     int64_t n;
     int kind;
     const XcShape *xc;    // generic convex bodies (kind 3): the body's geometry, device memory
+    int xc_parts;         // ... and whether its flat form has entries beside the rounded box
     double box[9], inv[9];
     double box_zero[3];   // box * (0, 0, 0) row by row (Matrix * Vector from zero): a no-wrap correction
     double *pos64;        // [n][3]
@@ -195,6 +198,8 @@ RP_HD int cell_phase(const int *dims, int cell) {
 // absolute centres and half axes [3 x 3 MAX_CEN doubles], its FP32 half axes [MAX_CEN], the queue
 // of centre pairs for the segment stage [64 words]
 constexpr int SWEEP_POLY_SCRATCH = MAX_CEN + 3 * MAX_CEN * MAX_CEN / 4 + 9 * MAX_CEN / 2 + MAX_CEN + 16;
+
+constexpr int SWEEP_CONVEX_SCRATCH = 5;  // convex bodies: the mover's FP64 orientation
 
 constexpr int NUM_COUNTERS = 9;     // sweep statistics words per handle (rp_sweep_stats order)
 constexpr int SWEEP_WARPS = 4;       // warps per block of the sweep kernel

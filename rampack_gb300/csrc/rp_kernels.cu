@@ -272,11 +272,13 @@ __global__ void k_count(DevState s, GridDev g, int early, unsigned long long *ou
     if (slot < s.n) count_one<KIND>(s, g, slot, early, out, flag);
 }
 
+// (Convex bodies: the portal loop beside the calls of the exact test needs the registers of three
+// resident blocks, 4.2 against 4.4 ms for two sweeps' moves of 262,144 bodies.)
 // MODE 1 instantiates the learned-ordering pre-test and the pair-outcome log, MODE 2 the
 // overlap counting, MODE 3 the plain scan of rototranslations (kept out of the plain
 // kernel, whose registers and branches they would crowd)
 template <int KIND, bool LIST, int MODE, int GW, bool SEG>
-__global__ void __launch_bounds__(SWEEP_WARPS * 32, SWEEP_MIN_BLOCKS) k_sweep(const SweepArgs A) {
+__global__ void __launch_bounds__(SWEEP_WARPS * 32, KIND == 3 ? 3 : SWEEP_MIN_BLOCKS) k_sweep(const SweepArgs A) {
     extern __shared__ float4 smem[];
     const Grp<GW> grp;
     const int lane = grp.lane;
@@ -288,10 +290,16 @@ __global__ void __launch_bounds__(SWEEP_WARPS * 32, SWEEP_MIN_BLOCKS) k_sweep(co
     // mirror slots [cap uint32], two uint16 queues and a byte counter per slot [5 cap bytes],
     // partner slots [LEARN], polysphere scratch [SWEEP_POLY_SCRATCH]
     constexpr bool AXM = GW == 16 && KIND == 1;
-    const int extra = KIND == 1 ? (AXM ? A.cap / 4 : A.cap) : (KIND == 2 ? A.cap / 4 : 0);
+    const int extra = KIND == 1 ? (AXM ? A.cap / 4 : A.cap) : (KIND >= 2 ? A.cap / 4 : 0);
     constexpr bool LEARN = MODE == 1;
     const int per_group = A.cap + extra + A.cap / 4 + A.cap / 16 + (LEARN ? A.cap / 4 : 0) +
-                          (KIND == 2 ? SWEEP_POLY_SCRATCH : 0);
+                          (KIND == 2 ? SWEEP_POLY_SCRATCH : (KIND == 3 ? SWEEP_CONVEX_SCRATCH : 0));
+    __shared__ XcFlat flat;
+    if (KIND == 3) {
+        const int *from = reinterpret_cast<const int *>(&A.s.xc->flat32);
+        for (int k = threadIdx.x; k < (int)(sizeof(XcFlat) / 4); k += blockDim.x) reinterpret_cast<int *>(&flat)[k] = from[k];
+        __syncthreads();
+    }
     float4 *cpos = smem + (size_t)gib * per_group;
     float4 *cax = cpos + A.cap;                                  // spherocylinders
     uint32_t *cslot = reinterpret_cast<uint32_t *>(cpos + A.cap); // mirror slot of each candidate
@@ -327,7 +335,7 @@ __global__ void __launch_bounds__(SWEEP_WARPS * 32, SWEEP_MIN_BLOCKS) k_sweep(co
         }
         if (item >= nitems) break;
         sweep_cell<KIND, LIST, MODE, GW, SEG>(A, item, -1, A.cap, A.overflow, A.overflow_count, cpos, cax, qseg, qun, nacc,
-                                          pstage, cslot, wx, ws);
+                                          pstage, cslot, wx, ws, KIND == 3 ? &flat : nullptr);
         grp.sync();
         if (ws.abort) break;
         item += stride;
@@ -458,8 +466,9 @@ cudaError_t launch_abs_centres(const DevState &s, cudaStream_t st) {
 }
 
 size_t sweep_smem_per_warp(int kind, int cap, bool learn, int ncen) {
-    const int extra = kind == 1 ? cap : (kind == 2 ? cap / 4 : 0);
-    return (size_t)(cap + extra + cap / 4 + cap / 16 + (learn ? cap / 4 : 0) + (kind == 2 ? SWEEP_POLY_SCRATCH : 0)) *
+    const int extra = kind == 1 ? cap : (kind >= 2 ? cap / 4 : 0);
+    return (size_t)(cap + extra + cap / 4 + cap / 16 + (learn ? cap / 4 : 0) +
+                    (kind == 2 ? SWEEP_POLY_SCRATCH : (kind == 3 ? SWEEP_CONVEX_SCRATCH : 0))) *
            sizeof(float4);
 }
 
@@ -531,6 +540,8 @@ cudaError_t launch_sweep(const SweepArgs &a, bool list, int nwarps, cudaStream_t
              : a.s.segs ? launch_sweep_t<2, false, 0>(a, blocks, th, smem, st)
                         : launch_sweep_t<2, false, 0, 32, false>(a, blocks, th, smem, st);
     }
+    if (a.s.kind == 3) return a.s.xc_parts ? launch_sweep_t<3, false, 0, 32, true>(a, blocks, th, smem, st)
+                                           : launch_sweep_t<3, false, 0>(a, blocks, th, smem, st);
     if (a.soft32) return launch_sweep_t<0, false, 4>(a, blocks, th, smem, st);
     if (rt) return a.s.kind == 0 ? launch_sweep_t<0, false, 3>(a, blocks, th, smem, st)
                                  : launch_sweep_t<1, false, 3>(a, blocks, th, smem, st);

@@ -14,8 +14,8 @@
 
 namespace rp {
 
-// Thresholds for a sphere (kind RP_SHAPE_SPHERE, radius r) or spherocylinder (radius r,
-// cylinder length l) whose FP32 coordinates are cell-local: lrow is the largest row norm of
+// Thresholds for a sphere (kind RP_SHAPE_SPHERE, radius r), spherocylinder (radius r,
+// cylinder length l) or convex body (circumsphere radius r, insphere radius l) whose FP32 coordinates are cell-local: lrow is the largest row norm of
 // the cell matrix (box / dims), box the row-major box.  Polysphere thresholds depend on the
 // centres and are formed by the caller.
 inline FilterConsts hard_filter_consts(int kind, double r, double l, double lrow, const double *box) {
@@ -36,7 +36,16 @@ inline FilterConsts hard_filter_consts(int kind, double r, double l, double lrow
         double d = std::sqrt(thr);
         return safety * (2.0 * d * std::sqrt(3.0) * e_sep + 3.0 * e_sep * e_sep + 4.0 * u32 * thr);
     };
-    if (kind == RP_SHAPE_SPHERE) {
+    if (kind == RP_SHAPE_CONVEX) {
+        // r the circumsphere's radius, l the insphere's
+        const double core = std::pow(l + l, 2), far = std::pow(r + r, 2);
+        fc.core_lo = static_cast<float>(core - margin(core));
+        fc.core_hi = static_cast<float>(core + margin(core));
+        fc.far_lo = static_cast<float>(far - margin(far));
+        fc.far_hi = static_cast<float>(far + margin(far));
+        fc.xc_scale = static_cast<float>(2 * r);
+        fc.xc_err = static_cast<float>(2.0 * safety * std::sqrt(3.0) * e_sep);
+    } else if (kind == RP_SHAPE_SPHERE) {
         double thr = std::pow(2 * r, 2);
         fc.sphere_lo = static_cast<float>(thr - margin(thr));
         fc.sphere_hi = static_cast<float>(thr + margin(thr));

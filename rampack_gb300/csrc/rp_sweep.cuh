@@ -200,6 +200,24 @@ __device__ __forceinline__ bool exact_pair(const DevState &s, d3 pi, d3 ai, int 
 }
 
 
+// The same of a convex mover (position pi, orientation ri).
+__device__ __forceinline__ bool exact_convex_pair(const DevState &s, d3 pi, const double *ri, int pid_j, float3 dsep) {
+    const d3 pj = load_d3(s.pos64 + 3 * (size_t)pid_j);
+    bool stuck = false;
+    const bool hit = xc_overlap_filtered(*s.xc, pi, ri, add3(pj, load_d3(s.trans + 3 * image_index(s, dsep, pi, pj))),
+                                         s.rot64 + 9 * (size_t)pid_j, stuck);
+    if (stuck) atomicOr(s.status, ST_PORTAL_STUCK);
+    return hit;
+}
+
+// FP32 orientation of the particle in slot k (convex bodies).
+__device__ __forceinline__ void load_mrot(const GridDev &g, size_t k, float *m) {
+    for (int a = 0; a < 3; a++) {
+        const float4 r = g.mrot[3 * k + a];
+        m[3 * a] = r.x, m[3 * a + 1] = r.y, m[3 * a + 2] = r.z;
+    }
+}
+
 // Exact FP64 test of centre a of a body, at absolute position pa, against centre j of
 // body pid_j seen at FP32 separation dsep (candidate minus mover): the reference's
 // (pos2 + t - pos1).norm2() < (r_a + r_j)^2 (core/Packing.cpp:40-42,
@@ -320,12 +338,15 @@ constexpr int STAGE_WAIT_LIMIT = 1 << 21;
 // (Packing::toggleOverlapCounting, core/Packing.cpp:304-323: the move's energy is the sign of
 // the change of the mover's overlap count); 3: rototranslations; 4: spheres with a soft part (the
 // energy change in FP32 with an error bound, FP64 where the Metropolis test is not certain).
-// SEG: multi-centre bodies may be polyspherocylinders (false: spheres only, without their code).
+// SEG: multi-centre bodies may be polyspherocylinders (false: spheres only, without their code); convex
+// bodies may have parts beside the rounded box.
 template <int KIND, bool LIST, int MODE, int GW = 32, bool SEG = true>
 __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, const int cell_direct, const int cap,
                                            int32_t *ovf, int32_t *ovf_count, float4 *cpos, float4 *cax,
                                            uint16_t *qseg, uint16_t *qun, uint8_t *nacc, uint16_t *pstage,
-                                           uint32_t *cslot, float4 *wx, WarpStats &ws) {
+                                           uint32_t *cslot, float4 *wx, WarpStats &ws,
+                                           const XcFlat *flat = nullptr) {
+    static_assert(KIND != 3 || (!LIST && MODE == 0), "convex bodies: the plain sweep");
     constexpr bool LEARN = MODE == 1;
     constexpr bool COUNT = MODE == 2;
     constexpr bool SOFT = MODE == 4;
@@ -436,7 +457,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             bulk_g2s(cpos + pre[0], G.mpos + st[0], (uint32_t)cnt[0] * 16u, ws.bar);
             if (WITH_AX) bulk_g2s(cax + pre[0], G.maxis + st[0], (uint32_t)cnt[0] * 16u, ws.bar);
         }
-        if (KIND == 2 || AXM)
+        if (KIND >= 2 || AXM)
             for (int k = 0; k < cnt[0]; k++) cslot[pre[0] + k] = (uint32_t)(st[0] + k);
         const bool landed = mbar_wait(ws.bar, ws.bphase, STAGE_WAIT_LIMIT);
         if (grp.ballot(!landed)) {
@@ -468,7 +489,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 p.z += off[r].z;
                 cpos[base + k] = p;
                 if (KIND == 1 && !AXM) cax[base + k] = G.maxis[st[r] + k];
-                if (KIND == 2 || AXM) cslot[base + k] = (uint32_t)(st[r] + k);  // its centres stay in the L2-resident mirror
+                if (KIND >= 2 || AXM) cslot[base + k] = (uint32_t)(st[r] + k);  // its centres stay in the L2-resident mirror
             }
         } else {
             int j = pre[r];
@@ -480,7 +501,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 p.z += off[r].z;
                 cpos[j] = p;
                 if (KIND == 1 && !AXM) cax[j] = G.maxis[st[r] + k];
-                if (KIND == 2 || AXM) cslot[j] = (uint32_t)(st[r] + k);
+                if (KIND >= 2 || AXM) cslot[j] = (uint32_t)(st[r] + k);
                 j++;
             }
         }
@@ -625,6 +646,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 }
             }
         }
+        if (KIND == 3 && A.log) uni = static_cast<double>(soft_uniform_bits(A.seed, A.counter, cell, mi)) * (1.0 / 9007199254740992.0);
         const float4 pcur = cpos[slot];
         const int pid = __float_as_int(pcur.w);
         // the mover's FP64 state, loaded now and first used after the FP32 filter:
@@ -977,6 +999,38 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             grp.sync();
         }
 
+        // ---- FP32 pass 2 (convex bodies): the near pairs' portals, one per lane ----
+        if (KIND == 3 && !overlap && nseg > 0) {
+            float O[9], P[9];
+            load_mrot(G, (size_t)gbase + slot, O);
+            for (int e = 0; e < 9; e++) P[e] = O[e];
+            if (type != 0)
+                for (int e = 0; e < 9; e++)
+                    P[e] = fmaf(R32[3 * (e / 3)], O[e % 3], fmaf(R32[3 * (e / 3) + 1], O[3 + e % 3], R32[3 * (e / 3) + 2] * O[6 + e % 3]));
+            for (int base = 0; base < nseg; base += GW) {
+                const int i = base + lane;
+                int cls = 0, k = 0;
+                if (i < nseg) {
+                    k = qseg[i];
+                    const float4 q = cpos[k];
+                    const f3v d{q.x - pn.x, q.y - pn.y, q.z - pn.z};
+                    float Q[9], rel[9];
+                    load_mrot(G, cslot[k], Q);
+                    for (int e = 0; e < 9; e++)
+                        rel[e] = fmaf(P[e / 3], Q[e % 3], fmaf(P[3 + e / 3], Q[3 + e % 3], P[6 + e / 3] * Q[6 + e % 3]));
+                    cls = xc_flat_pair<SEG>(*flat, rel, fmtv(P, d), 3e-5f * (sqrtf(fdot(d, d)) + S.fc.xc_scale) + S.fc.xc_err);
+                }
+                if (grp.ballot(cls == 1)) {
+                    overlap = true;
+                    break;
+                }
+                const unsigned b2 = grp.ballot(cls == 2);
+                if (cls == 2) qun[nun + __popc(b2 & lt)] = (uint16_t)k;
+                nun += __popc(b2);
+            }
+            grp.sync();
+        }
+
         uint8_t code = dom == 1 ? 2 : (overlap ? 1 : 0);
         // ---- FP64: the exact proposal of a surviving move (or of an accepted u == 0 move) ----
         // (an overlap found near the cell wall still needs the exact ActiveDomain test: the
@@ -1153,14 +1207,20 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             }
             if (KIND != 2 && code == 0 && nun > 0) {
                 bool ov = false;
+                double *wrot = reinterpret_cast<double *>(wx);   // convex bodies: the mover's new orientation
+                if (KIND == 3) {
+                    if (lane < 9) wrot[lane] = type != 0 ? onew_own : rot_own;
+                    grp.sync();
+                }
                 for (int qb = 0; qb < nun; qb += GW) {
                     int qi = qb + lane;
                     bool hit = false;
                     if (qi < nun) {
                         int k = qun[qi];
                         float4 q = cpos[k];
-                        hit = exact_pair(S, pnew, anew, __float_as_int(q.w),
-                                         make_float3(q.x - pn.x, q.y - pn.y, q.z - pn.z));
+                        const float3 dq = make_float3(q.x - pn.x, q.y - pn.y, q.z - pn.z);
+                        hit = KIND == 3 ? exact_convex_pair(S, pnew, wrot, __float_as_int(q.w), dq)
+                                        : exact_pair(S, pnew, anew, __float_as_int(q.w), dq);
                     }
                     if (grp.ballot(hit)) {
                         ov = true;
@@ -1347,6 +1407,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             if (type != 0) {
                 if (lane < 9) S.rot64[9 * (size_t)pid + lane] = onew_own;
                 const float of = (float)onew_own;
+                if (KIND == 3 && lane < 9) reinterpret_cast<float *>(G.mrot + 3 * gslot)[4 * ei + ej] = of;
                 na = make_float4(grp.shfl(of, 2), grp.shfl(of, 5), grp.shfl(of, 8), 0.f);
             }
             if (lane == 0) {
@@ -1500,6 +1561,10 @@ __device__ __forceinline__ void finish_one(const DevState &s, const GridDev &g, 
         g.mpos[k] = make_float4(l.x, l.y, l.z, __int_as_float(pid));
         const double *r = s.rot64 + 9 * (size_t)pid;
         g.maxis[k] = make_float4(static_cast<float>(r[2]), static_cast<float>(r[5]), static_cast<float>(r[8]), 0.f);
+        if (g.mrot)
+            for (int a = 0; a < 3; a++)
+                g.mrot[3 * (size_t)k + a] = make_float4(static_cast<float>(r[3 * a]), static_cast<float>(r[3 * a + 1]),
+                                                        static_cast<float>(r[3 * a + 2]), 0.f);
         for (int b = 0; b < s.ncen; b++) {
             const double *c = s.cen64 + 3 * ((size_t)pid * s.ncen + b);
             g.mcen[(size_t)k * s.ncen + b] =

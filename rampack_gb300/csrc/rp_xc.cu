@@ -287,6 +287,58 @@ struct Builder {
         return fail("Unknown XCBodyBuilder command: " + name);
     }
 
+    // the largest length of an FP32 evaluation of the node's support: displacements, radii of curvature
+    double span(int node) const {
+        const XcNode &g = out.node[node];
+        if (g.type == XC_POINT) return norm3(ld3(g.p));
+        if (g.type == XC_FOOTBALL || g.type == XC_SAUCER) return g.circ + curvature(g);
+        double s = g.type < XC_SUM ? g.circ : 0.0;
+        for (int i = 0; i < g.nent; i++) {
+            const double e = norm3(ld3(g.epos[i])) + span(g.ent[i]);
+            s = g.type == XC_MAX ? std::max(s, e) : s + e;
+        }
+        return s;
+    }
+
+    static double curvature(const XcNode &g) { return 0.5 * (g.p[0] * g.p[0] / g.p[1] + g.p[1]); }
+
+    // the entries of a flat root in FP32
+    void flatten(XcFlat &F) const {
+        const XcNode &r = out.node[out.root];
+        const bool single = r.type < XC_SUM;
+        F.op = single ? XC_SUM : r.type;
+        F.nent = single ? 1 : r.nent;
+        for (int k = 0; k < 3; k++) F.centre[k] = out.fcentre[k];
+        int kept = 0;
+        for (int i = 0; i < F.nent; i++) {
+            const XcNode &g = single ? r : out.node[r.ent[i]];
+            XcFlat::Entry e{};
+            e.type = g.type;
+            for (int k = 0; k < 3; k++) {
+                e.p[k] = static_cast<float>(g.p[k]);
+                e.pos[k] = single ? 0.f : static_cast<float>(r.epos[i][k]);
+                e.moved |= e.pos[k] != 0.f;
+            }
+            for (int k = 0; k < 9; k++) {
+                e.rot[k] = single ? (k % 4 == 0 ? 1.f : 0.f) : static_cast<float>(r.erot[i][k]);
+                e.turned |= e.rot[k] != (k % 4 == 0 ? 1.f : 0.f);
+            }
+            if (g.type == XC_FOOTBALL || g.type == XC_SAUCER) e.r2 = static_cast<float>(curvature(g));
+            const bool sphere = g.type == XC_SPHERE, box = g.type <= XC_CUBOID && !e.turned;
+            if (F.op == XC_SUM && (sphere || box)) {
+                F.folded = 1;
+                for (int k = 0; k < 3; k++) F.pos[k] += e.pos[k];
+                if (sphere) F.radius += e.p[0];
+                else if (g.type == XC_SEGMENT) F.half[2] += e.p[0];
+                else
+                    for (int k = 0; k < 3; k++) (g.type == XC_POINT ? F.pos : F.half)[k] += e.p[k];
+            } else {
+                F.ent[kept++] = e;
+            }
+        }
+        F.nent = kept;
+    }
+
     int depth(int node) const {
         const XcNode &g = out.node[node];
         if (g.type < XC_SUM) return 1;
@@ -346,6 +398,8 @@ bool xc_build(const std::string &script, XcShape &out, std::string &error) {
     if (r.type >= XC_SUM)
         for (int i = 0; i < r.nent; i++) out.flat = out.flat && out.node[r.ent[i]].type < XC_SUM;
     out.circ = r.circ;
+    out.f32_sound = b.span(out.root) <= 4 * r.circ && r.circ >= 1e-4 && r.circ <= 1e6;
+    if (out.flat) b.flatten(out.flat32);
     out.insph = r.insph;
     for (int k = 0; k < 3; k++) out.centre[k] = r.centre[k];
     return true;

@@ -64,9 +64,28 @@ struct XcNodeF {
     float p[3];
 };
 
+// A flat body (a primitive, or one operation over primitives) for the sweep's FP32 pair test: its
+// entries alone, with a note of the placements that change nothing.
+struct XcFlat {
+    int32_t op, nent;
+    float centre[3];
+    // a sum's unturned boxes (points, segments, rectangles) and its spheres, folded into one rounded
+    // box; the entries are the rest
+    int32_t folded;
+    float half[3], radius, pos[3];
+    struct Entry {
+        int32_t type, turned, moved;   // turned: rot is not the identity; moved: pos is not zero
+        float rot[9], pos[3], p[3];
+        float r2;                      // football, saucer: the radius of curvature
+    } ent[XC_MAX_ENTRIES];
+};
+
 struct XcShape {
     XcNode node[XC_MAX_NODES];
     XcNodeF fnode[XC_MAX_NODES];
+    XcFlat flat32;
+    int32_t f32_sound;   // FP32 support points err by a few roundings of the circumsphere radius: no
+                         // part is displaced or curved on a far larger scale, and no product overflows
     float fcentre[3];
     int32_t nnodes;
     int32_t root;
@@ -720,7 +739,7 @@ RP_XC_FN int xc_filter(const XcShape &s, d3 pos1, const double *rot1, d3 pos2bc,
     // a miss certified in FP32 alone: the support projection of the Minkowski difference is a
     // sum, or a maximum, of the parts' projections, each computed to a few FP32 roundings of
     // terms no larger than the scale, so an FP32 projection below -1e-4 scale is negative
-    if (hint == 0 && h32 < static_cast<float>(-(1e-4 * scale + 1e-6))) return 0;
+    if (hint == 0 && s.f32_sound && h32 < static_cast<float>(-(1e-4 * scale + 1e-6))) return 0;
     const double margin = 1e-7 * scale + 1e-9;
     if (hint == 0) {
         const d3 nd{n.x, n.y, n.z};
@@ -756,6 +775,141 @@ RP_HD bool xc_overlap_filtered(const XcShape &s, d3 pos1, const double *rot1, d3
     if (f >= 0) return f == 1;
     return xc_intersect(s, rot1, pos1, rot2, pos2bc, 1.0e-12, stuck);
 }
+
+#ifdef __CUDACC__
+// ---- the sweep's FP32 pair test (flat bodies with f32_sound) --------------------------------
+//
+// The portal refinement of xcf_refine with its certificates in FP32 too, so that FP64 is left to the
+// pairs near contact.  It runs in the first body's frame, where that body's support takes no rotation,
+// and as one loop around one support evaluation whatever the stage a pair is in, so the lanes of a
+// warp stay together (separate loops per stage left 6.6 of 32 lanes active).
+
+template <bool PARTS>
+__device__ __forceinline__ f3v xc_flat_support(const XcFlat &F, f3v n, float inv_n) {
+    f3v acc{0.f, 0.f, 0.f};
+    if (!PARTS || F.folded)
+        acc = {fmaf(n.x, F.radius * inv_n, F.pos[0] + copysignf(F.half[0], n.x)),
+               fmaf(n.y, F.radius * inv_n, F.pos[1] + copysignf(F.half[1], n.y)),
+               fmaf(n.z, F.radius * inv_n, F.pos[2] + copysignf(F.half[2], n.z))};
+    if (!PARTS) return acc;
+    float best = -INFINITY;
+    #pragma unroll 1
+    for (int i = 0; i < F.nent; i++) {
+        const XcFlat::Entry &e = F.ent[i];
+        const f3v dir = F.op == XC_DIFF && i == 1 ? fneg(n) : n;
+        f3v d = e.turned ? fmtv(e.rot, dir) : dir, r;
+        switch (e.type) {
+            case XC_POINT: r = {e.p[0], e.p[1], e.p[2]}; break;
+            case XC_SEGMENT: r = {0.f, 0.f, copysignf(e.p[0], d.z)}; break;
+            case XC_RECTANGLE:
+            case XC_CUBOID: r = {copysignf(e.p[0], d.x), copysignf(e.p[1], d.y), copysignf(e.p[2], d.z)}; break;
+            case XC_DISK: d.z = 0.f; [[fallthrough]];
+            case XC_SPHERE: r = fscale(d, e.p[0] * rsqrtf(fmaxf(fdot(d, d), 1e-37f))); break;
+            case XC_ELLIPSE:
+            case XC_ELLIPSOID: {   // an ellipse's third semi-axis is 0
+                const f3v u{d.x * e.p[0], d.y * e.p[1], d.z * e.p[2]};
+                const float k = rsqrtf(fmaxf(fdot(u, u), 1e-37f));
+                r = {u.x * k * e.p[0], u.y * k * e.p[1], u.z * k * e.p[2]};
+                break;
+            }
+            default: {   // football: a circle's arc turned about z; saucer: two caps
+                const f3v u = fscale(d, inv_n);
+                const float s2 = u.x * u.x + u.y * u.y, k = rsqrtf(fmaxf(s2, 1e-37f)), h = e.p[0];
+                if (e.type == XC_FOOTBALL) {
+                    const float c = e.r2 - e.p[1];
+                    r = fabsf(u.z) * e.r2 > h ? f3v{0.f, 0.f, copysignf(h, u.z)}
+                                              : f3v{u.x * (e.r2 - c * k), u.y * (e.r2 - c * k), u.z * e.r2};
+                } else {
+                    r = s2 * e.r2 * e.r2 > h * h ? f3v{u.x * k * h, u.y * k * h, 0.f}
+                                                 : f3v{u.x * e.r2, u.y * e.r2, u.z * e.r2 - copysignf(e.r2 - e.p[1], u.z)};
+                }
+            }
+        }
+        f3v w = e.turned ? fmv(e.rot, r) : r;
+        if (e.moved) w = fadd(w, f3v{e.pos[0], e.pos[1], e.pos[2]});
+        if (F.op == XC_MAX) {
+            const float pr = fdot(w, n);
+            if (pr > best) {
+                acc = w;
+                best = pr;
+            }
+        } else {
+            acc = F.op == XC_DIFF && i == 1 ? fsub(acc, w) : fadd(acc, w);
+        }
+    }
+    return acc;
+}
+
+// Body 2 (orientation rel, row-major, centre offset at d) against body 1 at the origin: 0 separated, 1
+// overlapping, 2 undecided.  `margin` bounds how far the FP32 difference body lies from the real one,
+// many times over: inputs (separation, axes), the support points and their projections.  A miss needs a
+// projection below -margin; a hit the origin farther than margin inside the tetrahedron of the centre
+// difference and three support points, where a face's normal m errs by up to 28 roundings of l^2 (l the
+// farthest vertex), hence the second term.
+// PARTS: the body has entries beside the rounded box (their code kept out of the plain kernel).
+template <bool PARTS>
+__device__ __forceinline__ int xc_flat_pair(const XcFlat &F, const float *rel, f3v d, float margin) {
+    const f3v c{F.centre[0], F.centre[1], F.centre[2]};
+    const f3v v0 = fsub(fadd(fmv(rel, c), d), c);
+    f3v n = fneg(v0), v1 = v0, v2 = v0, v3 = v0;
+    bool portal = false;   // v1, v2, v3 a portal that the ray from v0 through the origin passes
+    int it = 0;
+next:
+    bool hit = false;
+    #pragma unroll 1
+    for (; it < 32; it++) {
+        const float n2 = fdot(n, n), inv_n = rsqrtf(n2);
+        const f3v v = fsub(fadd(fmv(rel, xc_flat_support<PARTS>(F, fmtv(rel, n), inv_n)), d), xc_flat_support<PARTS>(F, fneg(n), inv_n));
+        const float pv = fdot(v, n);
+        if (!(n2 > 1e-30f)) return 2;
+        // a miss too close to call goes on as if the origin were inside: a later direction or
+        // tetrahedron may be clear
+        if (pv * inv_n < -margin) return 0;
+        if (it == 0) {
+            v1 = v;
+            n = fcross(v1, v0);
+        } else if (it == 1) {
+            v2 = v;
+            n = fcross(fsub(v1, v0), fsub(v2, v0));
+            if (fdot(n, v0) > 0.f) {
+                const f3v t = v1;
+                v1 = v2;
+                v2 = t;
+                n = fneg(n);
+            }
+        } else {
+            // no progress beyond FP32: the origin lies next to the surface
+            if (portal && !(fdot(fsub(v, v3), n) > 1e-6f * fabsf(pv))) return 2;
+            // the vertex that v replaces: looking for a portal, v2 or v1 by the side of the ray that v
+            // leaves uncovered (neither: v completes one); refining one, as the reference splits it
+            const f3v cr = fcross(v, v0);
+            const float s1 = fdot(v1, cr), s2 = fdot(v2, cr), s3 = fdot(v3, cr);
+            const int w = portal ? (s1 > 0.f ? (s2 > 0.f ? 1 : 3) : (s3 > 0.f ? 2 : 1))
+                                 : (s1 < 0.f ? 2 : (s2 > 0.f ? 1 : 3));
+            portal = portal || w == 3;
+            v1 = w == 1 ? v : v1;
+            v2 = w == 2 ? v : v2;
+            v3 = w == 3 ? v : v3;
+            const f3v o = portal ? v1 : v0;
+            n = fcross(fsub(portal ? v2 : v1, o), fsub(portal ? v3 : v2, o));
+            hit = portal && fdot(n, v1) >= 0.f;
+            if (hit) break;
+        }
+    }
+    if (!hit) return 2;
+    it++;
+    const f3v m = n, m1 = fcross(fsub(v2, v0), fsub(v3, v0)),
+              m2 = fcross(fsub(v1, v0), fsub(v3, v0)), m3 = fcross(fsub(v1, v0), fsub(v2, v0));
+    const float l2 = fmaxf(fmaxf(fdot(v0, v0), fdot(v1, v1)), fmaxf(fdot(v2, v2), fdot(v3, v3)));
+    const float slack = 6e-6f * l2 * sqrtf(l2);
+    auto inside = [&](f3v q, f3v a, f3v e) {   // the origin beyond the plane (q, a), on e's side
+        const float se = fdot(q, fsub(e, a)), so = -fdot(q, a), t = margin * sqrtf(fdot(q, q)) + slack;
+        return (se > t && so > t) || (se < -t && so < -t);
+    };
+    if (inside(m, v1, v0) && inside(m1, v0, v1) && inside(m2, v0, v2) && inside(m3, v0, v3)) return 1;
+    goto next;   // the next portal lies farther out
+}
+#endif
 
 // XenoCollideTraits::overlapWithWall (core/shapes/XenoCollideTraits.h:170-186): the wall normal w
 // taken into the body frame, the body's support point against it, and the wall plane through o.
