@@ -352,7 +352,8 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
     constexpr bool COUNT = MODE == 2;
     constexpr bool SOFT = MODE == 4;
     static_assert(!SOFT || (KIND == 0 && !LIST), "soft sweeps of spheres");
-    constexpr bool NEAR = KIND >= 1 && !COUNT && !LEARN;   // pass 1 queues, pass 2 classifies
+    constexpr bool ROWS = KIND >= 1 && !LEARN;     // candidates queued by reach, then classified
+    constexpr bool NEAR = ROWS && !COUNT;          // ... as pass 1 and pass 2
     constexpr bool RT = MODE == 3;  // every move a rototranslation (the plain scan otherwise)
     const Grp<GW> grp;
     const int lane = grp.lane;
@@ -520,7 +521,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         for (int t = lane; t < 3 * MAX_CEN * MAX_CEN; t += GW) wthr[t] = G.cthr[t];
     // pass 1 reads whole rows of the group: candidates out of everyone's reach up to the row's end
     const int padded = (total + GW - 1) / GW * GW;
-    if (NEAR && total + lane < padded) cpos[total + lane] = make_float4(1e18f, 1e18f, 1e18f, __int_as_float(-1));
+    if (ROWS && total + lane < padded) cpos[total + lane] = make_float4(1e18f, 1e18f, 1e18f, __int_as_float(-1));
     const bool self_images = (G.dims[0] == 1) || (G.dims[1] == 1) || (G.dims[2] == 1);
     // per own-cell particle: FP32 roundings accumulated in its mirror position this sweep
     for (int k = lane; k < occ; k += GW) nacc[k] = 0;
@@ -1313,13 +1314,30 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             const d3 pc64{grp.shfl(pos_own, 0), grp.shfl(pos_own, 1), grp.shfl(pos_own, 2)};
             const d3 ac64{grp.shfl(rot_own, 2), grp.shfl(rot_own, 5), grp.shfl(rot_own, 8)};
             int before = 0, after = 0;
+            if (ROWS) {
+                // the candidates within reach of either state, classified below on full warps (a
+                // classification on the spot ran the segment stage for a few lanes of every row)
+                const float far = A.fp64_only ? CUDART_INF_F : S.fc.far_hi;
+                for (int k = lane; k < padded; k += GW) {
+                    const float4 q = cpos[k];
+                    const float ax = q.x - pn.x, ay = q.y - pn.y, az = q.z - pn.z;
+                    const float bx = q.x - pcur.x, by = q.y - pcur.y, bz = q.z - pcur.z;
+                    const float d2 = fminf(fmaf(ax, ax, fmaf(ay, ay, az * az)), fmaf(bx, bx, fmaf(by, by, bz * bz)));
+                    const bool near = d2 <= far && __float_as_int(q.w) >= 0;
+                    const unsigned b = grp.ballot(near);
+                    if (near) qseg[nseg + __popc(b & lt)] = (uint16_t)k;
+                    nseg += __popc(b);
+                }
+                grp.sync();
+            }
             if (KIND == 2) {
                 // multi-centre bodies: every centre pair of every candidate body, the mover's
                 // current centres (FP32 mirror, FP64 absolute centres) and its new ones
                 const int K = S.ncen;
                 const float4 *mcur = G.mcen + ((size_t)gbase + slot) * K;
                 const bool exact = A.fp64_only || S.pbc_fold == 2;
-                for (int k = lane; k < total; k += GW) {
+                for (int i = lane; i < nseg; i += GW) {
+                    const int k = qseg[i];
                     const float4 q = cpos[k];
                     const int pj = __float_as_int(q.w);
                     if (pj == pid) continue;
@@ -1379,7 +1397,8 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                                                 pnew, anew, wcen, K, false, segs ? whax : nullptr);
                 }
             }
-            for (int k = lane; k < (KIND == 2 ? 0 : total); k += GW) {
+            for (int i = lane; i < (KIND == 2 ? 0 : (ROWS ? nseg : total)); i += GW) {
+                const int k = ROWS ? qseg[i] : i;
                 const float4 q = cpos[k];
                 const int pj = __float_as_int(q.w);
                 if (pj == pid) continue;
