@@ -160,8 +160,8 @@ __device__ __forceinline__ void flush_stats(const SweepArgs &A, WarpStats &ws) {
         atomicAdd(C + 6, (unsigned long long)ws.trans);
         atomicAdd(C + 7, (unsigned long long)ws.rots);
         atomicAdd(C + 8, (unsigned long long)ws.acc_trans);
+        ws = WarpStats{};
     }
-    ws = WarpStats{};
 }
 
 // Phase k of every replica: persistent warps take checkerboard cells of the whole batch
@@ -181,7 +181,10 @@ __global__ void __launch_bounds__(WPB * 32, 16 / WPB)
     uint16_t *qun = qseg + cap;
     uint8_t *nacc = reinterpret_cast<uint8_t *>(qun + cap);
     const int total = item_base[R];
-    WarpStats ws{};
+    __shared__ WarpStats stats[WPB];
+    WarpStats &ws = stats[wib];
+    if (lane == 0) ws = WarpStats{};
+    __syncwarp();
     for (;;) {
         int it = 0;
         if (lane == 0) it = atomicAdd(next_item, 1);
@@ -229,7 +232,9 @@ __global__ void __launch_bounds__(32) k_b_overflow(const BatchRep *T, int k, int
     uint16_t *qseg = reinterpret_cast<uint16_t *>(cpos + cap * (KIND == 1 ? 2 : 1));
     uint16_t *qun = qseg + cap;
     uint8_t *nacc = reinterpret_cast<uint8_t *>(qun + cap);
-    WarpStats ws{};
+    __shared__ WarpStats ws;
+    if (threadIdx.x == 0) ws = WarpStats{};
+    __syncwarp();
     for (int q = 0; q < count; q++) {
         sweep_cell<KIND, false, MODE>(A, q, A.overflow[q], cap, nullptr, nullptr, cpos, cax, qseg, qun, nacc,
                                           nullptr, nullptr, nullptr, ws);

@@ -87,7 +87,10 @@ __global__ void __launch_bounds__(CL_MAX_WARPS * 32, 1)
     const int rank = cl.block_rank(), nb = cl.num_blocks();
     const GridDev &G = A.g;
     cluster_rebuild(A.s, G, cl);
-    WarpStats ws{};
+    __shared__ WarpStats stats[CL_MAX_WARPS];
+    WarpStats &ws = stats[w];
+    if (lane == 0) ws = WarpStats{};
+    __syncwarp();
     for (int p = 0; p < P.nphases; p++) {
         const int ph = P.phase[p];
         int act[3];

@@ -310,7 +310,9 @@ __global__ void __launch_bounds__(SWEEP_WARPS * 32, KIND == 3 ? 3 : SWEEP_MIN_BL
     // polyspheres: after the partner slots when the learned ordering is on
     float4 *wx = reinterpret_cast<float4 *>(nacc + A.cap) + (LEARN ? A.cap / 4 : 0);
     int nitems = A.work ? (A.work_count ? *A.work_count : A.num_work) : (LIST ? A.num_list : A.num_active);
-    WarpStats ws{};
+    __shared__ WarpStats stats[SWEEP_WARPS * 32 / GW];
+    WarpStats &ws = stats[gib];
+    if (lane == 0) ws = WarpStats{};
     __shared__ uint64_t stage_bar[SWEEP_WARPS];
     if (GW == 32 && A.bulk_stage) {
         // the group's staging barrier: one arrival (lane 0's expected bytes) per phase
@@ -320,9 +322,9 @@ __global__ void __launch_bounds__(SWEEP_WARPS * 32, KIND == 3 ? 3 : SWEEP_MIN_BL
             fence_mbar_init();
             fence_proxy_async_smem();
         }
-        grp.sync();
-        ws.bar = bar;
+        if (lane == 0) ws.bar = bar;
     }
+    grp.sync();
     // persistent launches (next_item set) take cells from a shared counter until none are
     // left; otherwise groups stride over the cells
     const int stride = gridDim.x * groups_per_block;

@@ -57,6 +57,36 @@ struct Grp {
     __device__ __forceinline__ void sync() const { __syncwarp(mask); }
 };
 
+// Queues the staged candidates for which `in_reach` holds, in order, four rows of the group at a
+// time: tests, votes and counts of the four are independent of one another.
+template <int GW, class F>
+__device__ __forceinline__ void queue_rows(const Grp<GW> &grp, const float4 *cpos, int padded, int lane, unsigned lt,
+                                           uint16_t *queue, int &n, F in_reach) {
+    int k = lane;
+    for (; k + 3 * GW < padded; k += 4 * GW) {
+        bool near[4];
+        unsigned b[4];
+        int at[5];
+#pragma unroll
+        for (int u = 0; u < 4; u++) near[u] = in_reach(cpos[k + u * GW]);
+#pragma unroll
+        for (int u = 0; u < 4; u++) b[u] = grp.ballot(near[u]);
+        at[0] = n;
+#pragma unroll
+        for (int u = 0; u < 4; u++) at[u + 1] = at[u] + __popc(b[u]);
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+            if (near[u]) queue[at[u] + __popc(b[u] & lt)] = (uint16_t)(k + u * GW);
+        n = at[4];
+    }
+    for (; k < padded; k += GW) {
+        const bool near = in_reach(cpos[k]);
+        const unsigned b = grp.ballot(near);
+        if (near) queue[n + __popc(b & lt)] = (uint16_t)k;
+        n += __popc(b);
+    }
+}
+
 // ---------------------------------------------------------------------------------
 // FP32 classification of one pair.  0: no overlap, 1: overlap, 2: undecided in FP32
 // (re-decided in FP64).  d = p_j - p_i (candidate minus mover), a_i/a_j unit axes.
@@ -323,6 +353,7 @@ __device__ __forceinline__ void soft_energy32(const FilterConsts &fc, int kind, 
 // survives the FP32 filter builds its exact FP64 state (one box row per lane, one matrix
 // entry per lane), re-decides the queued pairs in FP64 and, when accepted, writes back.
 // ---------------------------------------------------------------------------------
+// (One per group, in shared memory: registers are what the move loop is short of.)
 struct WarpStats {
     unsigned moves, accepted, rej_overlap, rej_domain, pairs, fp64, trans, rots, acc_trans;
     // bulk staging (whole warps): the group's barrier (null: per-lane loads), the parity of
@@ -462,15 +493,17 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         }
         if (KIND >= 2 || AXM)
             for (int k = 0; k < cnt[0]; k++) cslot[pre[0] + k] = (uint32_t)(st[0] + k);
-        const bool landed = mbar_wait(ws.bar, ws.bphase, STAGE_WAIT_LIMIT);
+        const unsigned bphase = ws.bphase;
+        const bool landed = mbar_wait(ws.bar, bphase, STAGE_WAIT_LIMIT);
         if (grp.ballot(!landed)) {
             // lost copies: flag, give those in flight a last bounded wait, stop the group
             if (lane == 0) atomicOr(S.status, ST_STAGE_TIMEOUT);
-            mbar_wait(ws.bar, ws.bphase, STAGE_WAIT_LIMIT);
-            ws.abort = 1;
+            mbar_wait(ws.bar, bphase, STAGE_WAIT_LIMIT);
+            if (lane == 0) ws.abort = 1;
+            grp.sync();
             return;
         }
-        ws.bphase ^= 1u;
+        if (lane == 0) ws.bphase = bphase ^ 1u;
         if (lane < 27)
             for (int k = 0; k < cnt[0]; k++) {
                 float4 &p = cpos[pre[0] + k];
@@ -554,9 +587,6 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
     const int c_ld = ld == 0 ? c[0] : (ld == 1 ? c[1] : c[2]);
     const int dims_ld = ld == 0 ? G.dims[0] : (ld == 1 ? G.dims[1] : G.dims[2]);
     const int boff_ld = ld == 0 ? G.boundsoff[0] : (ld == 1 ? G.boundsoff[1] : G.boundsoff[2]);
-    const double shift_ld = ld == 0 ? G.shift[0] : (ld == 1 ? G.shift[1] : G.shift[2]);
-    const double lo_d = G.bounds[boff_ld + 2 * c_ld];
-    const double hi_d = G.bounds[boff_ld + 2 * c_ld + 1];
     // this lane's matrix entry (lanes 0-8)
     const int ei = lane < 9 ? lane / 3 : 0, ej = lane < 9 ? lane % 3 : 0;
 
@@ -574,6 +604,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
     }
     const int ntypes = sweep_move_types(A.types);
 
+    unsigned n_listed = 0, n_acc = 0, n_rej = 0, n_trans = 0, n_pairs = 0, n_fp64 = 0;
     u4 rnd_lane = u4{0u, 0u, 0u, 0u};  // Philox output of move (batch base + lane)
     uint64_t uni_lane = 0;             // soft sweeps: the bits of its Metropolis uniform
     for (int mi = 0; mi < nmoves; mi++) {
@@ -688,9 +719,8 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         // ---- FP32 ActiveDomain test (translations): 0 inside, 1 outside, 2 undecided;
         //      and whether the PBC correction may move the particle through the box ----
         int dom = 0;
-        float3 fnew = make_float3(0.f, 0.f, 0.f);
         if (type != 1) {
-            fnew = mat32(G.cellinv, pn.x, pn.y, pn.z);
+            const float3 fnew = mat32(G.cellinv, pn.x, pn.y, pn.z);
             float fm[3] = {fnew.x, fnew.y, fnew.z};
             const float mg = S.fc.cell_margin;
             for (int d = 0; d < 3; d++) {
@@ -731,7 +761,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 }
             }
             const unsigned nt = __popc(grp.ballot(tested));
-            if (lane == 0) ws.pairs += nt;
+            n_pairs += nt;
             if (grp.ballot(cls == 1)) overlap = true;
         }
 
@@ -768,7 +798,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                     nun += __popc(bu);
                 }
             }
-            if (lane == 0) ws.pairs += (unsigned)total;
+            n_pairs += (unsigned)total;
             overlap = grp.ballot(hit) != 0;
             if (!overlap && type != 1) {
 #pragma unroll
@@ -793,23 +823,12 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         // of 10^6 rods: 9.0 against 11.7 ms; of 64,000 longer ones with 481 candidates: 6.0 against 9.7 ms)
         if (NEAR && dom != 1) {
             const float far = A.fp64_only ? CUDART_INF_F : S.fc.far_hi;
-            auto slot1 = [&](const float4 &q, int k) {
+            auto in_reach = [&](const float4 &q) {
                 const float dx = q.x - pn.x, dy = q.y - pn.y, dz = q.z - pn.z;
-                const bool near = fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= far;
-                const unsigned b = grp.ballot(near);
-                if (near) qseg[nseg + __popc(b & lt)] = (uint16_t)k;
-                nseg += __popc(b);
+                return fmaf(dx, dx, fmaf(dy, dy, dz * dz)) <= far;
             };
-            int k = lane;
-            for (; k + 3 * GW < padded; k += 4 * GW) {
-                const float4 q0 = cpos[k], q1 = cpos[k + GW], q2 = cpos[k + 2 * GW], q3 = cpos[k + 3 * GW];
-                slot1(q0, k);
-                slot1(q1, k + GW);
-                slot1(q2, k + 2 * GW);
-                slot1(q3, k + 3 * GW);
-            }
-            for (; k < padded; k += GW) slot1(cpos[k], k);
-            if (lane == 0) ws.pairs += (unsigned)total;
+            queue_rows<GW>(grp, cpos, padded, lane, lt, qseg, nseg, in_reach);
+            n_pairs += (unsigned)total;
             grp.sync();
             if (A.fp64_only) {
                 for (int b = 0; b < nseg; b += GW) {
@@ -837,7 +856,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                         }
                     }
                 }
-                if (lane == 0) ws.pairs += (unsigned)min(SWEEP_P1 * GW, total - base);
+                n_pairs += (unsigned)min(SWEEP_P1 * GW, total - base);
                 bool hit = false;
 #pragma unroll
                 for (int u = 0; u < SWEEP_P1; u++) hit = hit || cl[u] == 1;
@@ -917,8 +936,53 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             }
             if (!overlap && qp > 0) segments(qp);
         }
-        // ---- FP32 pass 2 (polyspheres): every centre pair of a near body, one body per lane ----
-        if (!COUNT && KIND == 2 && (LEARN || !segs) && !overlap) {
+        // ---- FP32 pass 2 (polyspheres): one centre of a near body per lane against the mover's centres
+        //      (a body per lane left a third of the lanes idle and waited for its centres one after
+        //      another, 3/5 of the time of a sweep of chains) ----
+        if (!COUNT && !LEARN && KIND == 2 && !segs && !overlap) {
+            const int K = S.ncen, tasks = nseg * K;
+            const float inv_K = 1.0f / (float)K;
+            auto fetch = [&](int t, int &k, int &j) {
+                const int b = t < tasks ? (int)(((float)t + 0.5f) * inv_K) : 0;   // t / K, tasks < 2^20
+                k = qseg[b];
+                j = t < tasks ? t - b * K : 0;
+                return G.mcen[(size_t)cslot[k] * K + j];
+            };
+            int k, j;
+            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (tasks > 0) c = fetch(lane, k, j);
+            for (int base = 0; base < tasks && !overlap; base += GW) {
+                int k1 = 0, j1 = 0;
+                float4 c1 = c;
+                if (base + GW < tasks) c1 = fetch(base + GW + lane, k1, j1);   // the next row's, in flight
+                const float4 q = cpos[k];
+                const float bx = q.x - pn.x + c.x, by = q.y - pn.y + c.y, bz = q.z - pn.z + c.z;
+                int cls = 0;
+                for (int a = 0; a < K; a++) {
+                    const float4 m = wx[a];
+                    const float dx = bx - m.x, dy = by - m.y, dz = bz - m.z;
+                    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    if (d2 <= wthr[MAX_CEN * MAX_CEN + a * MAX_CEN + j])
+                        cls = d2 < wthr[a * MAX_CEN + j] ? 1 : (cls == 1 ? 1 : 2);
+                }
+                if (base + lane >= tasks || __float_as_int(q.w) == pid) cls = 0;
+                if (grp.ballot(cls == 1)) overlap = true;
+                const unsigned b2 = grp.ballot(cls == 2);
+                if (b2) {
+                    if (nun + __popc(b2) > cap) unall = true;
+                    else {
+                        if (cls == 2) qun[nun + __popc(b2 & lt)] = (uint16_t)k;
+                        nun += __popc(b2);
+                    }
+                }
+                k = k1;
+                j = j1;
+                c = c1;
+            }
+            grp.sync();
+        }
+        // ---- ... with the pair log, every centre pair of a near body, one body per lane ----
+        if (!COUNT && KIND == 2 && LEARN && !overlap) {
             const int K = S.ncen;
             for (int base = 0; base < nseg; base += GW) {
                 const int i = base + lane;
@@ -926,7 +990,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 if (i < nseg) {
                     k = qseg[i];
                     const float4 q = cpos[k];
-                    if (LEARN || __float_as_int(q.w) != pid) cls = poly_body_class(K, wx, wthr, make_float3(q.x - pn.x, q.y - pn.y, q.z - pn.z),
+                    cls = poly_body_class(K, wx, wthr, make_float3(q.x - pn.x, q.y - pn.y, q.z - pn.z),
                                           G.mcen + (size_t)cslot[k] * K);
                 }
                 if (LEARN && A.pair_every > 0 && ((mi + cell) % A.pair_every) == 0) {
@@ -1101,7 +1165,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 // the same image: s + (c + f) / n, minus the stored position's wrap k.
                 bool maywrap = false;
                 {
-                    float3 f0 = mat32(G.cellinv, pcur.x, pcur.y, pcur.z);
+                    const float3 f0 = mat32(G.cellinv, pcur.x, pcur.y, pcur.z), fnew = mat32(G.cellinv, pn.x, pn.y, pn.z);
                     float fm[3] = {fnew.x, fnew.y, fnew.z}, fo[3] = {f0.x, f0.y, f0.z};
                     const float mg = S.fc.cell_margin;
                     for (int d = 0; d < 3; d++) {
@@ -1148,6 +1212,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 if (dom == 2) {
                     // ActiveDomain::isInside (core/ActiveDomain.cpp:8-21) on the exact position
                     bool out = false;
+                    const double lo_d = G.bounds[boff_ld + 2 * c_ld], hi_d = G.bounds[boff_ld + 2 * c_ld + 1];
                     if (lane < 3 && dims_ld > 1) {
                         if (hi_d > lo_d) out = rel_own <= lo_d || rel_own >= hi_d;
                         else out = rel_own <= lo_d && rel_own >= hi_d;
@@ -1243,7 +1308,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                         }
                     }
                 }
-                ws.fp64 += nu;
+                n_fp64 += nu;
                 if (ov) code = 1;
             }
             if (KIND != 2 && code == 0 && nun > 0) {
@@ -1268,7 +1333,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                         break;
                     }
                 }
-                ws.fp64 += nun;
+                n_fp64 += nun;
                 if (ov) code = 1;
             }
             if (SOFT && code == 0 && soft == 2) {
@@ -1293,7 +1358,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                     e1 = dadd(e1, grp.shfl_xor(e1, d));
                 }
                 soft = metropolis(uni, dsub(e1, e0), A.temperature) ? 1 : 0;
-                ws.fp64 += total - 1;
+                n_fp64 += total - 1;
             }
             // hard walls: the mover at its exact new state (Packing::countParticleOverlaps adds
             // the wall overlaps after the pairs, core/Packing.cpp:424-428)
@@ -1318,16 +1383,13 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 // the candidates within reach of either state, classified below on full warps (a
                 // classification on the spot ran the segment stage for a few lanes of every row)
                 const float far = A.fp64_only ? CUDART_INF_F : S.fc.far_hi;
-                for (int k = lane; k < padded; k += GW) {
-                    const float4 q = cpos[k];
+                auto in_reach = [&](const float4 &q) {
                     const float ax = q.x - pn.x, ay = q.y - pn.y, az = q.z - pn.z;
                     const float bx = q.x - pcur.x, by = q.y - pcur.y, bz = q.z - pcur.z;
-                    const float d2 = fminf(fmaf(ax, ax, fmaf(ay, ay, az * az)), fmaf(bx, bx, fmaf(by, by, bz * bz)));
-                    const bool near = d2 <= far && __float_as_int(q.w) >= 0;
-                    const unsigned b = grp.ballot(near);
-                    if (near) qseg[nseg + __popc(b & lt)] = (uint16_t)k;
-                    nseg += __popc(b);
-                }
+                    return fminf(fmaf(ax, ax, fmaf(ay, ay, az * az)), fmaf(bx, bx, fmaf(by, by, bz * bz))) <= far &&
+                           __float_as_int(q.w) >= 0;
+                };
+                queue_rows<GW>(grp, cpos, padded, lane, lt, qseg, nseg, in_reach);
                 grp.sync();
             }
             if (KIND == 2) {
@@ -1426,7 +1488,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 before += grp.shfl_xor(before, d);
                 after += grp.shfl_xor(after, d);
             }
-            if (lane == 0) ws.pairs += (unsigned)(2 * (total - 1));
+            n_pairs += (unsigned)(2 * (total - 1));
             cdelta = after - before;
             code = cdelta < 0 ? 3 : (cdelta > 0 ? 1 : 0);
         }
@@ -1453,7 +1515,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 if (!exact_rel) rel_own = mrow(S.inv, ld, pnew);
                 if (lane == 0) nacc[slot] = 0;
                 // new cell-local FP32 position from the FP64 relative coordinates
-                double u = rel_own - shift_ld;
+                double u = rel_own - (ld == 0 ? G.shift[0] : (ld == 1 ? G.shift[1] : G.shift[2]));
                 if (u < 0.0) u += 1.0;
                 double fd = u * dims_ld - c_ld;
                 if (fd < -0.5) fd += dims_ld;
@@ -1522,13 +1584,23 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 A.log_codes[(size_t)ntypes * (size_t)gbase + mi] = full_code;
             }
         }
-        ws.moves++;
-        if (acc) ws.accepted++;
-        if (code == 1) ws.rej_overlap++;
-        if (code == 2) ws.rej_domain++;
-        if (type == 0) ws.trans++;
-        else ws.rots++;
-        if (type == 0 && acc) ws.acc_trans++;
+        // (a cell holds far fewer than 2^15 particles: two 16-bit counts to a word)
+        if (LIST) n_listed++;
+        if (acc) n_acc += type == 0 ? 0x10001u : 1u;
+        if (code == 1 || code == 2) n_rej += code == 2 ? 0x10000u : 1u;
+        n_trans += type == 0 ? 1u : 0u;
+    }
+    if (lane == 0) {
+        const unsigned n = LIST ? n_listed : (unsigned)nmoves;
+        ws.moves += n;
+        ws.accepted += n_acc & 0xffffu;
+        ws.acc_trans += n_acc >> 16;
+        ws.rej_overlap += n_rej & 0xffffu;
+        ws.rej_domain += n_rej >> 16;
+        ws.trans += n_trans;
+        ws.rots += n - n_trans;
+        ws.pairs += n_pairs;
+        ws.fp64 += n_fp64;
     }
 }
 
