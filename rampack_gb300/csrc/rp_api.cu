@@ -79,7 +79,7 @@ cudaError_t launch_commit_single(const DevState &s, SingleTry *t, uint8_t *disp_
 namespace {
 
 constexpr int OVF_WARPS = 152;          // overflow rerun: one warp per block, grid-stride over cells
-constexpr size_t OVF_SMEM = 200 * 1024; // shared memory of one overflow warp
+constexpr size_t OVF_SMEM = 208 * 1024; // shared memory of one overflow warp
 constexpr int64_t CLUSTER_MAX_N = 32768;     // particles and cells of a cluster sweep's rebuild (16 blocks)
 constexpr int CLUSTER_MAX_CELLS = 16384;
 
@@ -553,6 +553,12 @@ DevState dev_state(Handle *h) {
 size_t staging_capacity(size_t bytes, int kind, int ncen) {
     const size_t fixed = sweep_smem_per_warp(kind, 0, false, ncen);
     return std::min<size_t>((bytes - fixed) * 32 / (sweep_smem_per_warp(kind, 32, false, ncen) - fixed), 65504);
+}
+
+// ... and a warp of a batch.
+size_t batch_capacity(size_t bytes, int kind) {
+    const size_t fixed = batch_smem_per_warp(kind, 0), per32 = batch_smem_per_warp(kind, 32) - fixed;
+    return std::min<size_t>((bytes - fixed) / per32 * 32, 65504);
 }
 
 // Chooses the checkerboard grid for a box: cells at least one interaction range high
@@ -3148,8 +3154,7 @@ int rp_batch_sweep(void *batch, const rp_sweep_params *p, rp_sweep_stats *stats)
     }
     // the staging capacity of every replica: two warps per block must fit
     {
-        const size_t per_cap = batch_smem_per_warp(b->kind, 32) / 32;
-        const int fit = static_cast<int>(static_cast<size_t>(b->smem_optin) / 2 / per_cap) / 32 * 32;
+        const int fit = static_cast<int>(batch_capacity(static_cast<size_t>(b->smem_optin) / 2, b->kind));
         cap = std::min(cap, fit);
     }
     int total_items = 0, total_p = 0, total_c = 0;
@@ -3208,7 +3213,7 @@ int rp_batch_sweep(void *batch, const rp_sweep_params *p, rp_sweep_stats *stats)
     int wpb = b->wpb;
     while (wpb > 2 && static_cast<size_t>(wpb) * batch_smem_per_warp(b->kind, cap) > static_cast<size_t>(b->smem_optin))
         wpb /= 2;
-    const int ovf_cap = static_cast<int>(OVF_SMEM / (batch_smem_per_warp(b->kind, 32) / 32)) / 32 * 32;
+    const int ovf_cap = static_cast<int>(batch_capacity(OVF_SMEM, b->kind));
     for (int k = 0; k < maxph; k++) {
         const int *ib = b->d_bases + (2 + k) * (b->R + 1);
         int blocks = std::max(1, std::min((phase_total[k] + wpb - 1) / wpb, b->num_sms * (16 / wpb)));

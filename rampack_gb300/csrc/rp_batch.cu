@@ -173,13 +173,14 @@ __global__ void __launch_bounds__(WPB * 32, 16 / WPB)
     extern __shared__ float4 smem[];
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int per_warp = ARGS_F4 + cap * (KIND == 1 ? 2 : 1) + cap / 4 + cap / 16;
+    const int per_warp = ARGS_F4 + cap * (KIND == 1 ? 2 : 1) + cap / 4 + cap / 16 + sweep_scratch(KIND);
     SweepArgs *Aw = reinterpret_cast<SweepArgs *>(smem + (size_t)wib * per_warp);
     float4 *cpos = smem + (size_t)wib * per_warp + ARGS_F4;
     float4 *cax = cpos + cap;
     uint16_t *qseg = reinterpret_cast<uint16_t *>(cpos + cap * (KIND == 1 ? 2 : 1));
     uint16_t *qun = qseg + cap;
     uint8_t *nacc = reinterpret_cast<uint8_t *>(qun + cap);
+    float4 *wx = reinterpret_cast<float4 *>(nacc + cap);
     const int total = item_base[R];
     __shared__ WarpStats stats[WPB];
     WarpStats &ws = stats[wib];
@@ -212,7 +213,7 @@ __global__ void __launch_bounds__(WPB * 32, 16 / WPB)
         for (int d = 0; d < 3; d++) c[d] = ring_cell(G.dims[d], phase_digit(ph, d), cc[d]);
         const int cell = c[0] + G.dims[0] * (c[1] + G.dims[1] * c[2]);
         sweep_cell<KIND, false, MODE>(A, local, cell, cap, A.overflow, A.overflow_count, cpos, cax, qseg, qun, nacc,
-                                          nullptr, nullptr, nullptr, ws);
+                                          nullptr, nullptr, wx, ws);
         __syncwarp();
         flush_stats(A, ws);
         __syncwarp();
@@ -232,12 +233,13 @@ __global__ void __launch_bounds__(32) k_b_overflow(const BatchRep *T, int k, int
     uint16_t *qseg = reinterpret_cast<uint16_t *>(cpos + cap * (KIND == 1 ? 2 : 1));
     uint16_t *qun = qseg + cap;
     uint8_t *nacc = reinterpret_cast<uint8_t *>(qun + cap);
+    float4 *wx = reinterpret_cast<float4 *>(nacc + cap);
     __shared__ WarpStats ws;
     if (threadIdx.x == 0) ws = WarpStats{};
     __syncwarp();
     for (int q = 0; q < count; q++) {
         sweep_cell<KIND, false, MODE>(A, q, A.overflow[q], cap, nullptr, nullptr, cpos, cax, qseg, qun, nacc,
-                                          nullptr, nullptr, nullptr, ws);
+                                          nullptr, nullptr, wx, ws);
         __syncwarp();
     }
     flush_stats(A, ws);
@@ -310,7 +312,7 @@ cudaError_t launch_b_count(const BatchRep *T, const int *pbase, const int *cbase
 }
 
 size_t batch_smem_per_warp(int kind, int cap) {
-    return (size_t)(ARGS_F4 + cap * (kind == 1 ? 2 : 1) + cap / 4 + cap / 16) * sizeof(float4);
+    return (size_t)(ARGS_F4 + cap * (kind == 1 ? 2 : 1) + cap / 4 + cap / 16 + sweep_scratch(kind)) * sizeof(float4);
 }
 
 cudaError_t launch_b_sweep(const BatchRep *T, const int *item_base, int R, int kind, int k, int *next_item, int cap,

@@ -16,7 +16,7 @@
 namespace rp {
 
 constexpr int CL_MAX_WARPS = 16;             // warps per block (the sweep's 128 registers a thread)
-constexpr size_t CL_SMEM = 200 * 1024;       // a block's shared memory: also one overfull cell's staging
+constexpr size_t CL_SMEM = 208 * 1024;       // a block's shared memory: also one overfull cell's staging
 
 // What the host adds to the sweep's arguments.
 struct ClusterSweep {
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(CL_MAX_WARPS * 32, 1)
         for (int pass = 0; pass < 2; pass++) {
             const int cap = pass == 0 ? A.cap : P.cap_big;
             const int extra = KIND == 1 ? cap : (KIND == 2 ? cap / 4 : 0);
-            const int per_warp = cap + extra + cap / 4 + cap / 16 + (KIND == 2 ? SWEEP_POLY_SCRATCH : 0);
+            const int per_warp = cap + extra + cap / 4 + cap / 16 + sweep_scratch(KIND);
             float4 *cpos = smem + (pass == 0 ? (size_t)w * per_warp : 0);
             float4 *cax = cpos + cap;
             uint32_t *cslot = reinterpret_cast<uint32_t *>(cpos + cap);

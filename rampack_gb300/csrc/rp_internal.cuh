@@ -200,6 +200,12 @@ RP_HD int cell_phase(const int *dims, int cell) {
 constexpr int SWEEP_POLY_SCRATCH = MAX_CEN + 3 * MAX_CEN * MAX_CEN / 4 + 9 * MAX_CEN / 2 + MAX_CEN + 16;
 
 constexpr int SWEEP_CONVEX_SCRATCH = 5;  // convex bodies: the mover's FP64 orientation
+// the next 32 moves' proposals (rods and multi-centre bodies, one cell a warp): a translation and
+// the type and slot each [32], their rotations' FP32 rows [3 x 32], table indices [32 words]
+constexpr int SWEEP_PROPOSALS = 32 + 96 + 8;
+__host__ __device__ constexpr int sweep_scratch(int kind) {
+    return kind == 0 ? 0 : SWEEP_PROPOSALS + (kind == 2 ? SWEEP_POLY_SCRATCH : (kind == 3 ? SWEEP_CONVEX_SCRATCH : 0));
+}
 
 constexpr int NUM_COUNTERS = 9;     // sweep statistics words per handle (rp_sweep_stats order)
 constexpr int SWEEP_WARPS = 4;       // warps per block of the sweep kernel

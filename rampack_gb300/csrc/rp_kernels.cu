@@ -288,12 +288,11 @@ __global__ void __launch_bounds__(SWEEP_WARPS * 32, KIND == 3 ? 3 : SWEEP_MIN_BL
     // per-group shared memory (float4 units): staged positions [cap], spherocylinder axes
     // [cap] (with two cells per warp their mirror slots [cap uint32] instead) or polysphere
     // mirror slots [cap uint32], two uint16 queues and a byte counter per slot [5 cap bytes],
-    // partner slots [LEARN], polysphere scratch [SWEEP_POLY_SCRATCH]
+    // partner slots [LEARN], scratch [sweep_scratch]
     constexpr bool AXM = GW == 16 && KIND == 1;
     const int extra = KIND == 1 ? (AXM ? A.cap / 4 : A.cap) : (KIND >= 2 ? A.cap / 4 : 0);
     constexpr bool LEARN = MODE == 1;
-    const int per_group = A.cap + extra + A.cap / 4 + A.cap / 16 + (LEARN ? A.cap / 4 : 0) +
-                          (KIND == 2 ? SWEEP_POLY_SCRATCH : (KIND == 3 ? SWEEP_CONVEX_SCRATCH : 0));
+    const int per_group = A.cap + extra + A.cap / 4 + A.cap / 16 + (LEARN ? A.cap / 4 : 0) + (GW == 32 ? sweep_scratch(KIND) : 0);
     __shared__ XcFlat flat;
     if (KIND == 3) {
         const int *from = reinterpret_cast<const int *>(&A.s.xc->flat32);
@@ -469,9 +468,7 @@ cudaError_t launch_abs_centres(const DevState &s, cudaStream_t st) {
 
 size_t sweep_smem_per_warp(int kind, int cap, bool learn, int ncen) {
     const int extra = kind == 1 ? cap : (kind >= 2 ? cap / 4 : 0);
-    return (size_t)(cap + extra + cap / 4 + cap / 16 + (learn ? cap / 4 : 0) +
-                    (kind == 2 ? SWEEP_POLY_SCRATCH : (kind == 3 ? SWEEP_CONVEX_SCRATCH : 0))) *
-           sizeof(float4);
+    return (size_t)(cap + extra + cap / 4 + cap / 16 + (learn ? cap / 4 : 0) + sweep_scratch(kind)) * sizeof(float4);
 }
 
 // Shared memory of one cell's lane group when each warp sweeps two cells (spheres and

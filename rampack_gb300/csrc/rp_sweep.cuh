@@ -57,6 +57,11 @@ struct Grp {
     __device__ __forceinline__ void sync() const { __syncwarp(mask); }
 };
 
+__device__ __forceinline__ void copy_async16(float4 *to, const float4 *from) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(to)), "l"(from) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Queues the staged candidates for which `in_reach` holds, in order, four rows of the group at a
 // time: tests, votes and counts of the four are independent of one another.
 template <int GW, class F>
@@ -379,6 +384,10 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                                            uint32_t *cslot, float4 *wx, WarpStats &ws,
                                            const XcFlat *flat = nullptr) {
     static_assert(KIND != 3 || (!LIST && MODE == 0), "convex bodies: the plain sweep");
+    constexpr bool PROPS = KIND >= 1 && GW == 32 && !LIST;   // 32 proposals decoded at a time, in shared memory
+    float4 *const props = wx, *const prot = wx + 32;
+    uint32_t *const pidx = reinterpret_cast<uint32_t *>(wx + 128);
+    if (KIND >= 1 && GW == 32) wx += SWEEP_PROPOSALS;
     constexpr bool LEARN = MODE == 1;
     constexpr bool COUNT = MODE == 2;
     constexpr bool SOFT = MODE == 4;
@@ -614,6 +623,25 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             rnd_lane = philox(u4{(uint32_t)(mi + lane), (uint32_t)cell, (uint32_t)A.counter,
                                  (uint32_t)(A.counter >> 32)},
                               (uint32_t)A.seed, (uint32_t)(A.seed >> 32));
+            if (PROPS) {
+                const u4 r = rnd_lane;
+                const bool rt = RT || (COUNT && A.types == SWEEP_ROTOTRANSLATION);
+                const int type = rt ? 2 : (ntypes == 2 ? (int)(r.a >> 31) : ((A.types & 1) ? 0 : 1));
+                const int slot = (int)(((uint64_t)(r.a & 0x7fffffffu) * (uint32_t)occ) >> 31);
+                // pm1f takes the top 24 bits of a word: a rototranslation's rotation takes the low bytes
+                const float s = type == 1 ? 0.f : A.tstep;
+                props[lane] = make_float4(pm1f(r.b) * s, pm1f(r.c) * s, pm1f(r.d) * s, __uint_as_float((uint32_t)slot << 2 | type));
+                if (type != 0 && mi + lane < nmoves) {
+                    // a rotation of this sweep's table, or its transpose (the inverse): all of the
+                    // batch on their way from L2 at once
+                    const uint32_t idx = (rt ? (r.b & 0xffu) | ((r.c & 0xffu) << 8) : r.b) & A.rtab_mask;
+                    pidx[lane] = idx | ((rt ? r.d : r.c) & 1u) << 31;
+                    const float4 *from = reinterpret_cast<const float4 *>(A.rtab32) + 3 * (size_t)idx;
+                    for (int q = 0; q < 3; q++) copy_async16(prot + 3 * lane + q, from + q);
+                }
+                copy_async_wait();
+                grp.sync();
+            }
             if (SOFT) uni_lane = soft_uniform_bits(A.seed, A.counter, cell, mi + lane);
         }
         // ---- the proposal (FP32 view; FP64 inputs kept for the exact path) ----
@@ -650,6 +678,20 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             t64_lane = mrec->translation[ld];
             uni = mrec->uniform;
             for (int q = 0; q < 9; q++) R32[q] = (float)mrec->rotation[q];
+        } else if (PROPS) {
+            const int src = mi & 31;
+            const float4 pr = props[src];
+            type = (int)(__float_as_uint(pr.w) & 3u);
+            slot = (int)(__float_as_uint(pr.w) >> 2);
+            t32 = make_float3(pr.x, pr.y, pr.z);
+            if (type != 0) {
+                const uint32_t e = pidx[src];
+                rot_idx = e & 0x7fffffffu;
+                rot_inv = (e >> 31) != 0;
+                const float4 x0 = prot[3 * src], x1 = prot[3 * src + 1], x2 = prot[3 * src + 2];
+                const float R[9] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w, x2.x};
+                for (int q = 0; q < 9; q++) R32[q] = rot_inv ? R[3 * (q % 3) + q / 3] : R[q];
+            }
         } else {
             const int src = mi & (GW - 1);
             u4 r = u4{grp.shfl(rnd_lane.a, src), grp.shfl(rnd_lane.b, src),
@@ -664,7 +706,6 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 // pm1f takes the top 24 bits of a word: a rototranslation's rotation takes
                 // the low bytes
                 t32 = make_float3(pm1f(r.b) * A.tstep, pm1f(r.c) * A.tstep, pm1f(r.d) * A.tstep);
-                t64_lane = ld == 0 ? (double)t32.x : (ld == 1 ? (double)t32.y : (double)t32.z);
             }
             if (type != 0) {
                 // a rotation of this sweep's table, or its transpose (the inverse)
@@ -1239,37 +1280,51 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             if (KIND == 2) {
                 // the mover's centres: rotated by R (Packing::rotateTempInteractionCentres,
                 // core/Packing.cpp:357-361), then position + centre wrapped into the box
-                // (core/Packing.cpp:1041-1047); one centre per lane
-                double R[9];
-                for (int d = 0; d < 3; d++) {
-                    R[3 * d] = grp.shfl(rrow[0], 3 * d);
-                    R[3 * d + 1] = grp.shfl(rrow[1], 3 * d);
-                    R[3 * d + 2] = grp.shfl(rrow[2], 3 * d);
+                // (core/Packing.cpp:1041-1047); a coordinate per lane, row `row` of centre `ctr` (the FP64
+                // pipe takes as long for one lane as for 32, and it bounded sweeps of bent rods)
+                const int ctr = lane / 3, row = lane - 3 * ctr, first = lane - row, own = row < 2 ? row : 2;
+                const bool mine = lane < 3 * S.ncen;
+                const double p_row = row == 0 ? pnew.x : (row == 1 ? pnew.y : pnew.z);
+                double c = mine ? S.cen64[3 * (size_t)pid * S.ncen + lane] : 0.0;
+                if (type != 0) {
+                    const double r0 = grp.shfl(rrow[0], 3 * own), r1 = grp.shfl(rrow[1], 3 * own), r2 = grp.shfl(rrow[2], 3 * own);
+                    const double x = grp.shfl(c, first), y = grp.shfl(c, first + 1), z = grp.shfl(c, min(first + 2, 31));
+                    c = dadd(dadd(dadd(0.0, dmul(r0, x)), dmul(r1, y)), dmul(r2, z));
                 }
-                if (lane < S.ncen) {
-                    d3 c = load_d3(S.cen64 + 3 * ((size_t)pid * S.ncen + lane));
-                    if (type != 0) c = mv3(R, c);
-                    d3 q = add3(pnew, c);
-                    d3 a = add3(q, pbc_correction(S.box, S.inv, q, nullptr));
-                    wcen[3 * lane] = c.x;
-                    wcen[3 * lane + 1] = c.y;
-                    wcen[3 * lane + 2] = c.z;
-                    wabs[3 * lane] = a.x;
-                    wabs[3 * lane + 1] = a.y;
-                    wabs[3 * lane + 2] = a.z;
+                const double q = dadd(p_row, c);
+                // FP32 shows most centres clear of the box's faces: a correction of box * 0 = +0
+                float f0, f1, f2;
+                {
+                    const float qf = (float)q;
+                    f0 = grp.shfl(qf, first), f1 = grp.shfl(qf, first + 1), f2 = grp.shfl(qf, min(first + 2, 31));
                 }
-                if (segs) {
+                const float i0 = S.inv32[3 * own], i1 = S.inv32[3 * own + 1], i2 = S.inv32[3 * own + 2];
+                const float rel = i0 * f0 + i1 * f1 + i2 * f2;
+                const float mg = 1e-5f * (1.f + fabsf(i0 * f0) + fabsf(i1 * f1) + fabsf(i2 * f2));
+                double ab = dadd(q, 0.0);
+                if (grp.ballot(mine && !(rel > mg && rel < 1.f - mg))) {
+                    const d3 Q{grp.shfl(q, first), grp.shfl(q, first + 1), grp.shfl(q, min(first + 2, 31))};
+                    const double r = mrow(S.inv, own, Q);
+                    double k = 0.0;
+                    if (mine) {
+                        while (dadd(r, k) < 0.0) k = dadd(k, 1.0);
+                        while (dadd(r, k) >= 1.0) k = dsub(k, 1.0);
+                    }
+                    const d3 C{grp.shfl(k, first), grp.shfl(k, first + 1), grp.shfl(k, min(first + 2, 31))};
+                    ab = dadd(q, mrow(S.box, own, C));
+                }
+                if (mine) {
+                    wcen[lane] = c;
+                    wabs[lane] = ab;
+                }
+                if (segs && (type != 0 || nun > 0 || unall || S.walls || COUNT)) {
                     // orientation * half axis with the mover's new orientation
                     // (PolyspherocylinderTraits.cpp:118-119)
                     const double oe = type != 0 ? onew_own : rot_own;
-                    double O[9];
-                    for (int e = 0; e < 9; e++) O[e] = grp.shfl(oe, e);
-                    if (lane < S.ncen) {
-                        d3 h = mv3(O, d3{S.chax[lane][0], S.chax[lane][1], S.chax[lane][2]});
-                        whax[3 * lane] = h.x;
-                        whax[3 * lane + 1] = h.y;
-                        whax[3 * lane + 2] = h.z;
-                    }
+                    const double o0 = grp.shfl(oe, 3 * own), o1 = grp.shfl(oe, 3 * own + 1), o2 = grp.shfl(oe, 3 * own + 2);
+                    const double *hb = S.chax[mine ? ctr : 0];
+                    const double h = dadd(dadd(dadd(0.0, dmul(o0, hb[0])), dmul(o1, hb[1])), dmul(o2, hb[2]));
+                    if (mine) whax[lane] = h;
                 }
                 grp.sync();
             }
@@ -1539,18 +1594,14 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                     G.maxis[gslot] = na;
                 }
             }
-            if (KIND == 2 && lane < S.ncen) {
+            if (KIND == 2 && lane < 3 * S.ncen) {
                 // Packing::acceptTempInteractionCentres (core/Packing.cpp:339-348)
-                const size_t ci = (size_t)pid * S.ncen + lane;
-                for (int d = 0; d < 3; d++) S.abs64[3 * ci + d] = wabs[3 * lane + d];
+                const size_t ci = 3 * (size_t)pid * S.ncen + lane, mi4 = 4 * (gslot * S.ncen + lane / 3) + lane % 3;
+                S.abs64[ci] = wabs[lane];
                 if (type != 0) {
-                    for (int d = 0; d < 3; d++) S.cen64[3 * ci + d] = wcen[3 * lane + d];
-                    const float4 c32 = make_float4((float)wcen[3 * lane], (float)wcen[3 * lane + 1],
-                                                   (float)wcen[3 * lane + 2], 0.f);
-                    G.mcen[gslot * S.ncen + lane] = c32;
-                    if (segs)
-                        G.mhax[gslot * S.ncen + lane] = make_float4((float)whax[3 * lane], (float)whax[3 * lane + 1],
-                                                                    (float)whax[3 * lane + 2], 0.f);
+                    S.cen64[ci] = wcen[lane];
+                    reinterpret_cast<float *>(G.mcen)[mi4] = (float)wcen[lane];
+                    if (segs) reinterpret_cast<float *>(G.mhax)[mi4] = (float)whax[lane];
                 }
             }
             if (self_images) {
@@ -1572,7 +1623,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             if (lane == 0 && A.codes) A.codes[out_index] = full_code;
         } else if (A.log) {
             rp_move *rec = A.log + (size_t)ntypes * (size_t)gbase + mi;
-            if (lane < 3) rec->translation[lane] = t64_lane;
+            if (lane < 3) rec->translation[lane] = (double)(lane == 0 ? t32.x : (lane == 1 ? t32.y : t32.z));
             const double rj = ej == 0 ? rrow[0] : (ej == 1 ? rrow[1] : rrow[2]);
             if (lane < 9) rec->rotation[lane] = type != 0 ? rj : (lane % 4 == 0 ? 1.0 : 0.0);
             if (lane == 0) {
