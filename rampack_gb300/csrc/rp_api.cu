@@ -458,6 +458,7 @@ DevState dev_state(Handle *h) {
     s.xc_parts = h->xc_parts ? 1 : 0;
     std::memcpy(s.box, h->box, sizeof(s.box));
     std::memcpy(s.inv, h->inv, sizeof(s.inv));
+    s.diag = diagonal(s.inv) ? 1 : 0;
     for (int i = 0; i < 3; i++) {
         double z = 0.0;
         for (int j = 0; j < 3; j++) z = z + h->box[3 * i + j] * 0.0;
@@ -906,7 +907,7 @@ int run_overflow(Handle *h, SweepArgs a, bool list) {
     cap = cap / 32 * 32;
     a.cap = cap;
     a.work = h->overflow;
-    a.work_count = h->overflow_count;
+    a.work_count = a.overflow_count;
     a.partners = nullptr;  // the plain kernel: no partner pre-test, no pair log
     a.pair_every = 0;
     a.num_work = -1;
@@ -915,7 +916,8 @@ int run_overflow(Handle *h, SweepArgs a, bool list) {
         Group grp(h, RP_KERNEL_OVERFLOW, 1);
         RP_CUDA(h, launch_sweep(a, list, OVF_WARPS, h->stream));
     }
-    RP_CUDA(h, cudaMemsetAsync(h->overflow_count, 0, sizeof(int32_t), h->stream));
+    // (a sweep's phases have a count each, zeroed with its item counters)
+    if (list) RP_CUDA(h, cudaMemsetAsync(h->overflow_count, 0, sizeof(int32_t), h->stream));
     return RP_OK;
 }
 
@@ -1929,6 +1931,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
             a.pair_cap = static_cast<unsigned long long>(h->pair_cap);
             a.pair_every = h->pair_every;
         }
+        a.overflow_count = h->item_counters + 32 + phase_no;
         a.next_item = h->item_counters + phase_no++;
         int act[3];
         a.num_active = phase_cells(g, ph, act);

@@ -94,10 +94,22 @@ __global__ void k_b_scatter(const BatchRep *T, const int *pbase, int R) {
 }
 
 __global__ void k_b_finish(const BatchRep *T, const int *cbase, int R) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cbase[R]) return;
-    int r = find_rep(cbase, R, c);
-    finish_one(T[r].a.s, T[r].a.g, c - cbase[r]);
+    // a thread per cell sorts; where a warp's cells belong to one replica, their slots are one run and
+    // its lanes share the mirror's writing
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, total = cbase[R];
+    const int r = c < total ? find_rep(cbase, R, c) : -1;
+    const int r0 = __shfl_sync(0xffffffffu, r, 0);
+    if (r0 < 0) return;
+    if (__all_sync(0xffffffffu, r == r0 || c >= total)) {
+        const DevState &s = T[r0].a.s;
+        const GridDev &g = T[r0].a.g;
+        const int l = c - cbase[r0], l0 = l - (threadIdx.x & 31), l1 = min(l0 + 32, total - cbase[r0]);
+        if (c < total) sort_cell(g, l);
+        __syncwarp();
+        for (int k = g.start[l0] + (threadIdx.x & 31); k < g.start[l1]; k += 32) mirror_slot(s, g, k);
+    } else if (c < total) {
+        finish_one(T[r].a.s, T[r].a.g, c - cbase[r]);
+    }
 }
 
 // Box move: newBox · (oldBox^-1 · r) for the particles of every rescaled replica, and the
@@ -110,7 +122,8 @@ __global__ void k_b_rescale(const BatchRep *T, const int *pbase, int R) {
     if (!B.scale) return;
     const int64_t l = i - pbase[r];
     d3 p = d3{B.scale_src[3 * l], B.scale_src[3 * l + 1], B.scale_src[3 * l + 2]};
-    d3 q = mv3(B.new_box, mv3(B.old_inv, p));
+    const d3 q = diagonal(B.new_box) && diagonal(B.old_inv) ? mv3_diag(B.new_box, mv3_diag(B.old_inv, p))
+                                                            : mv3(B.new_box, mv3(B.old_inv, p));
     B.scale_dst[3 * l] = q.x;
     B.scale_dst[3 * l + 1] = q.y;
     B.scale_dst[3 * l + 2] = q.z;

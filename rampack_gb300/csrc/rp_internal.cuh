@@ -99,6 +99,7 @@ struct DevState {
     const XcShape *xc;    // generic convex bodies (kind 3): the body's geometry, device memory
     int xc_parts;         // ... and whether its flat form has entries beside the rounded box
     double box[9], inv[9];
+    int diag;             // the box (and its inverse) is diagonal
     double box_zero[3];   // box * (0, 0, 0) row by row (Matrix * Vector from zero): a no-wrap correction
     double *pos64;        // [n][3]
     double *rot64;        // [n][9]

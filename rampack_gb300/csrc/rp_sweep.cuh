@@ -248,6 +248,7 @@ __device__ __forceinline__ bool exact_convex_pair(const DevState &s, d3 pi, cons
 
 // FP32 orientation of the particle in slot k (convex bodies).
 __device__ __forceinline__ void load_mrot(const GridDev &g, size_t k, float *m) {
+#pragma unroll
     for (int a = 0; a < 3; a++) {
         const float4 r = g.mrot[3 * k + a];
         m[3 * a] = r.x, m[3 * a + 1] = r.y, m[3 * a + 2] = r.z;
@@ -1145,10 +1146,13 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         if (KIND == 3 && !overlap && nseg > 0) {
             float O[9], P[9];
             load_mrot(G, (size_t)gbase + slot, O);
+#pragma unroll
             for (int e = 0; e < 9; e++) P[e] = O[e];
-            if (type != 0)
+            if (type != 0) {
+#pragma unroll
                 for (int e = 0; e < 9; e++)
                     P[e] = fmaf(R32[3 * (e / 3)], O[e % 3], fmaf(R32[3 * (e / 3) + 1], O[3 + e % 3], R32[3 * (e / 3) + 2] * O[6 + e % 3]));
+            }
             for (int base = 0; base < nseg; base += GW) {
                 const int i = base + lane;
                 int cls = 0, k = 0;
@@ -1161,6 +1165,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                     if (cls == 3) {
                         float Q[9], rel[9];
                         load_mrot(G, cslot[k], Q);
+#pragma unroll
                         for (int e = 0; e < 9; e++)
                             rel[e] = fmaf(P[e / 3], Q[e % 3], fmaf(P[3 + e / 3], Q[3 + e % 3], P[6 + e / 3] * Q[6 + e % 3]));
                         cls = xc_flat_pair<SEG>(*flat, rel, fmtv(P, d), 3e-5f * (sqrtf(d2) + S.fc.xc_scale) + S.fc.xc_err);
@@ -1185,6 +1190,8 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         const bool needR = type != 0 && (need64 || A.log != nullptr);
         double rel_own = 0.0, pnew_own = 0.0, onew_own = 0.0, rrow[3] = {0.0, 0.0, 0.0};
         bool exact_rel = false;     // rel_own holds the exact FP64 relative coordinate
+        // the whole vectors on every lane: only for what needs them (most accepted moves do not)
+        const bool vectors = KIND == 2 || COUNT || SOFT || S.walls || nun > 0;
         d3 pnew{0, 0, 0}, anew{0, 0, 0};
         if (needR) {
             // row ei of the move's rotation (lanes 0-8 hold rows 0..2 three times over)
@@ -1249,7 +1256,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                     }
                     exact_rel = true;
                 }
-                pnew = d3{grp.shfl(pnew_own, 0), grp.shfl(pnew_own, 1), grp.shfl(pnew_own, 2)};
+                if (vectors) pnew = d3{grp.shfl(pnew_own, 0), grp.shfl(pnew_own, 1), grp.shfl(pnew_own, 2)};
                 if (dom == 2) {
                     // ActiveDomain::isInside (core/ActiveDomain.cpp:8-21) on the exact position
                     bool out = false;
@@ -1260,7 +1267,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                     }
                     if (grp.ballot(out)) code = 2;
                 }
-            } else {
+            } else if (vectors) {
                 pnew = d3{grp.shfl(pos_own, 0), grp.shfl(pos_own, 1), grp.shfl(pos_own, 2)};
             }
             if (type != 0) {
@@ -1273,8 +1280,8 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 s = dadd(s, dmul(rrow[1], o1));
                 s = dadd(s, dmul(rrow[2], o2));
                 onew_own = s;
-                anew = d3{grp.shfl(s, 2), grp.shfl(s, 5), grp.shfl(s, 8)};
-            } else {
+                if (vectors) anew = d3{grp.shfl(s, 2), grp.shfl(s, 5), grp.shfl(s, 8)};
+            } else if (vectors) {
                 anew = d3{grp.shfl(rot_own, 2), grp.shfl(rot_own, 5), grp.shfl(rot_own, 8)};
             }
             if (KIND == 2) {
@@ -1567,7 +1574,8 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 np = make_float4(pn.x, pn.y, pn.z, pcur.w);
                 if (lane == 0) nacc[slot] = (uint8_t)(na_cnt + 1);
             } else if (type != 1) {
-                if (!exact_rel) rel_own = mrow(S.inv, ld, pnew);
+                if (!exact_rel)
+                    rel_own = mrow(S.inv, ld, d3{grp.shfl(pnew_own, 0), grp.shfl(pnew_own, 1), grp.shfl(pnew_own, 2)});
                 if (lane == 0) nacc[slot] = 0;
                 // new cell-local FP32 position from the FP64 relative coordinates
                 double u = rel_own - (ld == 0 ? G.shift[0] : (ld == 1 ? G.shift[1] : G.shift[2]));
@@ -1688,7 +1696,7 @@ __device__ __forceinline__ void validate_particle(const DevState &s, int64_t i) 
 // cell of each shifted coordinate and the in-cell fraction mapped through the FP32 cell matrix.
 __device__ __forceinline__ int locate_one(const DevState &s, const GridDev &g, int64_t i, float3 &loc) {
     d3 p = load_d3(s.pos64 + 3 * i);
-    d3 r = mv3(s.inv, p);
+    d3 r = s.diag ? mv3_diag(s.inv, p) : mv3(s.inv, p);
     double rr[3] = {r.x, r.y, r.z};
     if (s.strict_box) {
         validate_one(s, i, rr);
@@ -1723,9 +1731,8 @@ __device__ __forceinline__ void scatter_one(const GridDev &g, int64_t i) {
     g.slot_pid[g.start[g.pid_cell[i]] + g.rank[i]] = static_cast<int32_t>(i);
 }
 
-// Sorts a cell's particles by index (a deterministic order independent of the atomic
-// arrival order) and writes the FP32 mirror in cell order.
-__device__ __forceinline__ void finish_one(const DevState &s, const GridDev &g, int cell) {
+// Sorts a cell's particles by index: a deterministic order independent of the atomic arrival order.
+__device__ __forceinline__ void sort_cell(const GridDev &g, int cell) {
     int b = g.start[cell], e = g.start[cell + 1];
     for (int k = b + 1; k < e; k++) {
         int v = g.slot_pid[k];
@@ -1736,28 +1743,36 @@ __device__ __forceinline__ void finish_one(const DevState &s, const GridDev &g, 
         }
         g.slot_pid[j + 1] = v;
     }
-    for (int k = b; k < e; k++) {
-        int pid = g.slot_pid[k];
-        g.pid_slot[pid] = k;
-        float4 l = g.plocal[pid];
-        g.mpos[k] = make_float4(l.x, l.y, l.z, __int_as_float(pid));
-        const double *r = s.rot64 + 9 * (size_t)pid;
-        g.maxis[k] = make_float4(static_cast<float>(r[2]), static_cast<float>(r[5]), static_cast<float>(r[8]), 0.f);
-        if (g.mrot)
-            for (int a = 0; a < 3; a++)
-                g.mrot[3 * (size_t)k + a] = make_float4(static_cast<float>(r[3 * a]), static_cast<float>(r[3 * a + 1]),
-                                                        static_cast<float>(r[3 * a + 2]), 0.f);
-        for (int b = 0; b < s.ncen; b++) {
-            const double *c = s.cen64 + 3 * ((size_t)pid * s.ncen + b);
-            g.mcen[(size_t)k * s.ncen + b] =
-                make_float4(static_cast<float>(c[0]), static_cast<float>(c[1]), static_cast<float>(c[2]), 0.f);
-            if (s.segs) {
-                const d3 h = mv3(r, d3{s.chax[b][0], s.chax[b][1], s.chax[b][2]});
-                g.mhax[(size_t)k * s.ncen + b] =
-                    make_float4(static_cast<float>(h.x), static_cast<float>(h.y), static_cast<float>(h.z), 0.f);
-            }
+}
+
+// The FP32 mirror of one slot.
+__device__ __forceinline__ void mirror_slot(const DevState &s, const GridDev &g, int k) {
+    int pid = g.slot_pid[k];
+    g.pid_slot[pid] = k;
+    float4 l = g.plocal[pid];
+    g.mpos[k] = make_float4(l.x, l.y, l.z, __int_as_float(pid));
+    const double *r = s.rot64 + 9 * (size_t)pid;
+    g.maxis[k] = make_float4(static_cast<float>(r[2]), static_cast<float>(r[5]), static_cast<float>(r[8]), 0.f);
+    if (g.mrot)
+        for (int a = 0; a < 3; a++)
+            g.mrot[3 * (size_t)k + a] = make_float4(static_cast<float>(r[3 * a]), static_cast<float>(r[3 * a + 1]),
+                                                    static_cast<float>(r[3 * a + 2]), 0.f);
+    for (int b = 0; b < s.ncen; b++) {
+        const double *c = s.cen64 + 3 * ((size_t)pid * s.ncen + b);
+        g.mcen[(size_t)k * s.ncen + b] =
+            make_float4(static_cast<float>(c[0]), static_cast<float>(c[1]), static_cast<float>(c[2]), 0.f);
+        if (s.segs) {
+            const d3 h = mv3(r, d3{s.chax[b][0], s.chax[b][1], s.chax[b][2]});
+            g.mhax[(size_t)k * s.ncen + b] =
+                make_float4(static_cast<float>(h.x), static_cast<float>(h.y), static_cast<float>(h.z), 0.f);
         }
     }
+}
+
+// One thread for a whole cell (the fused small-system sweep).
+__device__ __forceinline__ void finish_one(const DevState &s, const GridDev &g, int cell) {
+    sort_cell(g, cell);
+    for (int k = g.start[cell]; k < g.start[cell + 1]; k++) mirror_slot(s, g, k);
 }
 
 // Recount of one particle by one thread: its pairs with higher particle indices in the 27 cells.
