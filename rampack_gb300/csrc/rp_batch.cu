@@ -199,25 +199,36 @@ __global__ void __launch_bounds__(WPB * 32, 16 / WPB)
     WarpStats &ws = stats[wib];
     if (lane == 0) ws = WarpStats{};
     __syncwarp();
+    // cells in runs of up to eight: finding and copying their replica's arguments (and adding its
+    // statistics) costs more than the move or two of a sphere's cell; at least four runs a warp
+    const int run = min(max(total / (int)(gridDim.x * WPB * 4), 1), 8);
+    const SweepArgs &A = *Aw;
+    const GridDev &G = A.g;
+    int item = 0, end = 0, r = -1, r_end = 0, ph = 0;
     for (;;) {
-        int it = 0;
-        if (lane == 0) it = atomicAdd(next_item, 1);
-        const int item = __shfl_sync(FULL, it, 0);
+        if (item >= end) {
+            int it = 0;
+            if (lane == 0) it = atomicAdd(next_item, run);
+            item = __shfl_sync(FULL, it, 0);
+            end = min(item + run, total);
+        }
         if (item >= total) break;
-        const int r = find_rep(item_base, R, item);
-        const BatchRep &B = T[r];
-        if (k >= B.nphases) continue;
-        // the replica's arguments, copied into this warp's shared memory (read all through the cell)
-        {
-            const float4 *src = reinterpret_cast<const float4 *>(&B.a);
+        if (r < 0 || item >= r_end || item < item_base[r]) {
+            // the replica's arguments, copied into this warp's shared memory (read all through its cells)
+            if (r >= 0) {
+                flush_stats(A, ws);
+                __syncwarp();
+            }
+            r = find_rep(item_base, R, item);
+            r_end = item_base[r + 1];
+            ph = T[r].phases[k];
+            const float4 *src = reinterpret_cast<const float4 *>(&T[r].a);
             float4 *dst = reinterpret_cast<float4 *>(Aw);
             for (int q = lane; q < ARGS_F4; q += 32) dst[q] = src[q];
             __syncwarp();
         }
-        const SweepArgs &A = *Aw;
-        const GridDev &G = A.g;
         const int local = item - item_base[r];
-        const int ph = B.phases[k];
+        item++;
         int act[3], cc[3], c[3];
         for (int d = 0; d < 3; d++) act[d] = ring_count(G.dims[d], phase_digit(ph, d));
         cc[0] = local % act[0];
@@ -228,9 +239,8 @@ __global__ void __launch_bounds__(WPB * 32, 16 / WPB)
         sweep_cell<KIND, false, MODE>(A, local, cell, cap, A.overflow, A.overflow_count, cpos, cax, qseg, qun, nacc,
                                           nullptr, nullptr, wx, ws);
         __syncwarp();
-        flush_stats(A, ws);
-        __syncwarp();
     }
+    if (r >= 0) flush_stats(A, ws);
 }
 
 // The cells of phase k whose neighbourhood did not fit: one block (one warp, large shared

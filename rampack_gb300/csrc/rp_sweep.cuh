@@ -475,6 +475,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
     }
     const int occ = grp.shfl(cnt[0], 0);
     const int gbase = grp.shfl(st[0], 0);
+    if (!LIST && occ == 0) return;   // nothing to move (a third of a sphere system's cells)
     if (total > cap) {
         if (lane == 0) {
             if (ovf) {
@@ -528,14 +529,29 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         if (!filt) {
             // every neighbour staged: positions known from the prefix sum (loads pipeline freely)
             const int base = pre[r];
-            for (int k = 0; k < cnt[r]; k++) {
-                float4 p = G.mpos[st[r] + k];
-                p.x += off[r].x;
-                p.y += off[r].y;
-                p.z += off[r].z;
-                cpos[base + k] = p;
-                if (KIND == 1 && !AXM) cax[base + k] = G.maxis[st[r] + k];
-                if (KIND >= 2 || AXM) cslot[base + k] = (uint32_t)(st[r] + k);  // its centres stay in the L2-resident mirror
+            if (KIND == 0) {
+                // spheres: the few particles of a cell with their loads in flight together (staging was
+                // half of a wca sweep's time, a cell's moves being one or two)
+                constexpr int U = 4;
+                for (int k0 = 0; k0 < cnt[r]; k0 += U) {
+                    float4 p[U];
+#pragma unroll
+                    for (int u = 0; u < U; u++) p[u] = G.mpos[st[r] + min(k0 + u, cnt[r] - 1)];
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (k0 + u < cnt[r])
+                            cpos[base + k0 + u] = make_float4(p[u].x + off[r].x, p[u].y + off[r].y, p[u].z + off[r].z, p[u].w);
+                }
+            } else {
+                for (int k = 0; k < cnt[r]; k++) {
+                    float4 p = G.mpos[st[r] + k];
+                    p.x += off[r].x;
+                    p.y += off[r].y;
+                    p.z += off[r].z;
+                    cpos[base + k] = p;
+                    if (KIND == 1 && !AXM) cax[base + k] = G.maxis[st[r] + k];
+                    if (KIND >= 2 || AXM) cslot[base + k] = (uint32_t)(st[r] + k);  // its centres stay in the L2-resident mirror
+                }
             }
         } else {
             int j = pre[r];
