@@ -109,7 +109,7 @@ typedef struct rp_sweep_stats {
     uint64_t accepted;
     uint64_t rejected_overlap;
     uint64_t rejected_domain;
-    uint64_t pair_tests;          /* candidate pairs the FP32 filter examined (scans stop at a certain overlap) */
+    uint64_t pair_tests;          /* candidate pairs the FP32 filter examined (spheres: scans stop at a certain overlap) */
     uint64_t fp64_pairs;          /* pairs re-decided in FP64 (the guard band) */
     uint64_t translations;
     uint64_t rotations;
@@ -501,7 +501,7 @@ int rp_get_cells_per_warp(void *handle, int32_t *last);
 /* Staging filter of the sweep: candidates of the 26 neighbour cells farther than the
  * interaction range from every face-slab of the mover's cell (its ActiveDomain) are not
  * staged; decisions are unchanged.  0 off, 1 (default) where cells are well above the range
- * (keeps < 90 % of the neighbourhood), 2 wherever no grid dimension has a single cell. */
+ * (keeps < 65 % of the neighbourhood, < 90 % with two cells per warp), 2 wherever no grid dimension has a single cell. */
 int rp_set_staging_filter(void *handle, int32_t mode);
 /* How a sweep stages each cell's 3x3x3 neighbourhood into shared memory: 1 with bulk
  * asynchronous copies (cp.async.bulk, one per neighbour cell and array, completing on an

@@ -1152,7 +1152,7 @@ static int create_common(Handle *h, int64_t n, int device, void **handle) {
         if ((e = cudaMalloc(&h->rtab64, sizeof(double) * 9 * ROT_TABLE)) != cudaSuccess) return bail(e);
         if ((e = cudaMalloc(&h->rtab32, sizeof(float) * 12 * ROT_TABLE)) != cudaSuccess) return bail(e);
     }
-    if ((e = cudaMalloc(&h->item_counters, sizeof(int32_t) * 64)) != cudaSuccess) return bail(e);
+    if ((e = cudaMalloc(&h->item_counters, sizeof(int32_t) * 96)) != cudaSuccess) return bail(e);
     if (!h->batch_member) {
         if ((e = cudaMalloc(&h->status, sizeof(uint32_t))) != cudaSuccess) return bail(e);
         if ((e = cudaMalloc(&h->counters, sizeof(unsigned long long) * NUM_COUNTERS)) != cudaSuccess) return bail(e);
@@ -1809,6 +1809,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     // the arguments every phase shares
     auto sweep_args = [&](double tstep) {
         SweepArgs a = base_args(h);
+        if (soft32 || convex32) a.bulk_stage = 0;   // per-lane loads, as their FP64 sweeps
         if (soft32) {
             a.soft32 = 1;
             a.temperature = h->temperature;
@@ -1827,11 +1828,13 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         return a;
     };
     // small systems: the rebuild and every phase in one launch of a thread-block cluster, where each
-    // active cell of a phase gets a warp there (1000 spheres: 180 -> 45 us a sweep; with more cells
-    // than that the whole chip's warps are worth the launches)
+    // active cell of a phase gets a warp there (1000 spheres: 180 -> 69 us a sweep; with more cells
+    // than that the whole chip's warps are worth the launches).  Soft spheres: where any neighbourhood
+    // fits, as their sweeps refuse none
     int cl_warps = 0;
     if (!fp64_sweep && !convex && !h->bulk_stage && h->cells_per_warp == 1 && h->order_mode == RP_ORDER_OFF && h->pair_cap == 0 &&
-        h->n <= CLUSTER_MAX_N && g.ncell <= CLUSTER_MAX_CELLS) {
+        h->n <= CLUSTER_MAX_N && g.ncell <= CLUSTER_MAX_CELLS &&
+        !(soft32 && h->n > static_cast<int64_t>(staging_capacity(OVF_SMEM, h->shape.kind, 0)))) {
         if (h->cl_blocks < 0) h->cl_blocks = cluster_blocks();
         int most = 0, act[3];
         for (int ph : phases) most = std::max(most, phase_cells(g, ph, act));
@@ -1857,7 +1860,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         }
     }
     if (stats) RP_CUDA(h, cudaMemsetAsync(h->counters, 0, sizeof(unsigned long long) * NUM_COUNTERS, h->stream));
-    if (!cl_warps) RP_CUDA(h, cudaMemsetAsync(h->item_counters, 0, sizeof(int32_t) * 64, h->stream));
+    if (!cl_warps) RP_CUDA(h, cudaMemsetAsync(h->item_counters, 0, sizeof(int32_t) * 96, h->stream));
     if (types & (2 | SWEEP_ROTOTRANSLATION)) {
         Group grp(h, RP_KERNEL_SWEEP, 1);
         RP_CUDA(h, launch_rot_table(h->rtab64, h->rtab32, ROT_TABLE, p->seed, p->counter,
@@ -1868,10 +1871,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         if (rc2) return rc2;
     }
     h->since_rank++;
-    if (fp64_sweep) {
-        // a soft part or a generic convex body: every move decided in FP64 (hard part, then the
-        // energy change with the Metropolis test at the handle's temperature), one warp per
-        // active cell
+    auto fp64_args = [&]() {
         SoftSweepArgs sa{};
         sa.c.s = dev_state(h);
         sa.c.g = g;
@@ -1887,6 +1887,13 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
             sa.log = h->d_log;
             sa.log_codes = h->d_log_codes;
         }
+        return sa;
+    };
+    if (fp64_sweep) {
+        // a soft part or a generic convex body: every move decided in FP64 (hard part, then the
+        // energy change with the Metropolis test at the handle's temperature), one warp per
+        // active cell
+        SoftSweepArgs sa = fp64_args();
         int soft_phase = 0;
         int soft_start[27] = {0};
         const bool soft_ordered = h->cell_order && g.order;
@@ -1970,8 +1977,18 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
             }
         }
         a.next_item = nullptr;
-        rc = run_overflow(h, a, false);
-        if (rc) return rc;
+        if (soft32 || convex32) {
+            // cells that did not fit their staging: the FP64 sweep, which has no such limit
+            SoftSweepArgs sa = fp64_args();
+            sa.work = h->overflow;
+            sa.work_count = a.overflow_count;
+            sa.next_item = h->item_counters + 63 + phase_no;
+            Group grp(h, RP_KERNEL_OVERFLOW, 1);
+            RP_CUDA(h, launch_soft_sweep(sa, OVF_WARPS, h->stream));
+        } else {
+            rc = run_overflow(h, a, false);
+            if (rc) return rc;
+        }
     }
     if (log) {
         h->log_valid = true;

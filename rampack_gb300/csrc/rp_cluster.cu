@@ -193,7 +193,7 @@ cudaError_t dispatch(const SweepArgs &a, const ClusterSweep &p, int blocks, int 
 
 size_t sweep_smem_per_warp(int kind, int cap, bool learn, int ncen);
 
-// Whether a cluster of 16 blocks (`big`) or 8 fits the device with a block's 200 KB.
+// Blocks of the largest cluster (16 or 8) that fits the device with a block's 208 KB; 0: none.
 int cluster_blocks() {
     SweepArgs a{};
     ClusterSweep p{};

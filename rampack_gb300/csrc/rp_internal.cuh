@@ -323,6 +323,9 @@ struct SoftSweepArgs {
     rp_move *log;
     uint8_t *log_codes;
     const int32_t *work;           // the phase's cells by occupancy, largest first (null: index order)
+    // the cells an FP32 sweep could not stage: their number (null: num_active), and the FP32 mirror is
+    // to follow their moves, as the rest of that sweep reads it
+    const int32_t *work_count;
 };
 
 // One replica of a batched launch (rp_batch_*): its sweep arguments, this sweep's phase

@@ -689,13 +689,13 @@ __global__ void __launch_bounds__(SOFT_WARPS * 32, 4) k_soft_sweep(SoftSweepArgs
     const SingleArgs &C = A.c;
     const DevState &S = C.s;
     const GridDev &G = C.g;
-    const int ntypes = sweep_move_types(A.types);
+    const int ntypes = sweep_move_types(A.types), items = A.work_count ? *A.work_count : A.num_active;
     unsigned n_moves = 0, n_acc = 0, n_ov = 0, n_dom = 0, n_tr = 0, n_rot = 0, n_acc_tr = 0;
     for (;;) {
         int item = 0;
         if (lane == 0) item = atomicAdd(A.next_item, 1);
         item = __shfl_sync(FULL, item, 0);
-        if (item >= A.num_active) break;
+        if (item >= items) break;
         int c[3];
         if (A.work) {  // the phase's cells by occupancy, largest first
             const int w = A.work[item];
@@ -774,6 +774,24 @@ __global__ void __launch_bounds__(SOFT_WARPS * 32, 4) k_soft_sweep(SoftSweepArgs
                     S.abs64[3 * (size_t)pid * S.ncen + q] = mv.abs[0][q];
                 }
                 if (S.counting) atomicAdd(S.overlaps, (unsigned long long)(long long)delta);
+                if (A.work_count) {
+                    // the mirror's cell-local FP32 position, as an accepted move of the FP32 sweep leaves it
+                    float f[3];
+                    for (int d = 0; d < 3; d++) {
+                        double u = mrow(S.inv, d, d3{mv.pos[0][0], mv.pos[0][1], mv.pos[0][2]}) - G.shift[d];
+                        if (u < 0.0) u += 1.0;
+                        double fd = u * G.dims[d] - c[d];
+                        if (fd < -0.5) fd += G.dims[d];
+                        if (fd > G.dims[d] - 0.5) fd -= G.dims[d];
+                        f[d] = (float)fd;
+                    }
+                    const float3 loc = mat32(G.cellmat, f[0], f[1], f[2]);
+                    G.mpos[gbase + slot] = make_float4(loc.x, loc.y, loc.z, __int_as_float(pid));
+                    if (G.mrot)
+                        for (int a = 0; a < 3; a++)
+                            G.mrot[3 * (size_t)(gbase + slot) + a] = make_float4(
+                                (float)mv.rot[0][3 * a], (float)mv.rot[0][3 * a + 1], (float)mv.rot[0][3 * a + 2], 0.f);
+                }
             }
             if (lane == 0 && A.log) {
                 A.log[(size_t)ntypes * (size_t)gbase + mi] = m;

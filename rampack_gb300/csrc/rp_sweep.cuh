@@ -876,9 +876,9 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             }
         }
         // bodies with a second pass: pass 1 only queues the candidates within reach (the mover among
-        // them), and the second pass classifies its few entries on full warps: a move of rods with
-        // 174 candidates takes 1130 instead of 1385 instructions (five sweeps
-        // of 10^6 rods: 9.0 against 11.7 ms; of 64,000 longer ones with 481 candidates: 6.0 against 9.7 ms)
+        // them), and the second pass classifies its few entries on full warps: a move of rods with 174
+        // candidates takes 565 instead of 690 instructions (five sweeps of 10^6 rods: 9.0 against
+        // 11.7 ms; of 64,000 longer ones with 481 candidates: 6.0 against 9.7 ms)
         if (NEAR && dom != 1) {
             const float far = A.fp64_only ? CUDART_INF_F : S.fc.far_hi;
             auto in_reach = [&](const float4 &q) {
@@ -939,8 +939,8 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
         grp.sync();
         // ---- FP32 pass 2 (polyspherocylinders): the centre pairs of a near body, one body per lane;
         //      pairs between the insphere and circumsphere thresholds are queued and their segments
-        //      decided 32 to a round (in FP64 those pairs bound the sweep: 25 against 8 ms for five
-        //      cycles of 10^5 bent rods) ----
+        //      decided 32 to a round (in FP64 those pairs bound the sweep: 25.3 against 5.7 ms for
+        //      the five sweeps of 10^5 bent rods) ----
         bool unall = false;   // more undecided pairs than the queue holds: every near body in FP64
         if (!COUNT && !LEARN && KIND == 2 && segs && !overlap) {
             const int K = S.ncen;
