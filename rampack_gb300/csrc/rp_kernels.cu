@@ -276,13 +276,14 @@ __global__ void k_count(DevState s, GridDev g, int early, unsigned long long *ou
     if (slot < s.n) count_one<KIND>(s, g, slot, early, out, flag);
 }
 
-// (Convex bodies: the portal loop beside the calls of the exact test needs the registers of three
-// resident blocks, 4.2 against 4.4 ms for two sweeps' moves of 262,144 bodies.)
+// (Convex bodies' portal loop and polyspherocylinders' segments want the registers of three resident
+// blocks: 4.2 against 4.4 ms a pass of 262,144 convex bodies, 4.04 against 4.23 of 10^5 bent rods; rods
+// and chains want the fourth block, 11.3 against 13.4 and 3.35 against 3.45 ms.)
 // MODE 1 instantiates the learned-ordering pre-test and the pair-outcome log, MODE 2 the
 // overlap counting, MODE 3 the plain scan of rototranslations (kept out of the plain
 // kernel, whose registers and branches they would crowd)
 template <int KIND, bool LIST, int MODE, int GW, bool SEG>
-__global__ void __launch_bounds__(SWEEP_WARPS * 32, KIND == 3 ? 3 : SWEEP_MIN_BLOCKS) k_sweep(const SweepArgs A) {
+__global__ void __launch_bounds__(SWEEP_WARPS * 32, KIND == 3 || (KIND == 2 && SEG) ? 3 : SWEEP_MIN_BLOCKS) k_sweep(const SweepArgs A) {
     extern __shared__ float4 smem[];
     const Grp<GW> grp;
     const int lane = grp.lane;
