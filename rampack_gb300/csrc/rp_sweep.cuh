@@ -630,7 +630,21 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
     }
     const int ntypes = sweep_move_types(A.types);
 
-    unsigned n_listed = 0, n_acc = 0, n_rej = 0, n_trans = 0, n_pairs = 0, n_fp64 = 0;
+    unsigned n_done = 0, n_acc = 0, n_rej = 0, n_trans = 0, n_pairs = 0, n_fp64 = 0;
+    auto flush = [&] {
+        if (lane == 0) {
+            const unsigned n = LIST ? n_done : (unsigned)nmoves;
+            ws.moves += n;
+            ws.accepted += n_acc & 0xffffu;
+            ws.acc_trans += n_acc >> 16;
+            ws.rej_overlap += n_rej & 0xffffu;
+            ws.rej_domain += n_rej >> 16;
+            ws.trans += n_trans;
+            ws.rots += n - n_trans;
+            ws.pairs += n_pairs;
+            ws.fp64 += n_fp64;
+        }
+    };
     u4 rnd_lane = u4{0u, 0u, 0u, 0u};  // Philox output of move (batch base + lane)
     uint64_t uni_lane = 0;             // soft sweeps: the bits of its Metropolis uniform
     for (int mi = 0; mi < nmoves; mi++) {
@@ -1659,24 +1673,18 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 A.log_codes[(size_t)ntypes * (size_t)gbase + mi] = full_code;
             }
         }
-        // (a cell holds far fewer than 2^15 particles: two 16-bit counts to a word)
-        if (LIST) n_listed++;
+        // (two 16-bit counts to a word: a staged cell holds far fewer than 2^15 particles, and a move
+        // list's counts are passed on before they could overflow)
+        if (LIST) n_done++;
         if (acc) n_acc += type == 0 ? 0x10001u : 1u;
         if (code == 1 || code == 2) n_rej += code == 2 ? 0x10000u : 1u;
         n_trans += type == 0 ? 1u : 0u;
+        if (LIST && n_done == 0x8000u) {
+            flush();
+            n_done = n_acc = n_rej = n_trans = n_pairs = n_fp64 = 0;
+        }
     }
-    if (lane == 0) {
-        const unsigned n = LIST ? n_listed : (unsigned)nmoves;
-        ws.moves += n;
-        ws.accepted += n_acc & 0xffffu;
-        ws.acc_trans += n_acc >> 16;
-        ws.rej_overlap += n_rej & 0xffffu;
-        ws.rej_domain += n_rej >> 16;
-        ws.trans += n_trans;
-        ws.rots += n - n_trans;
-        ws.pairs += n_pairs;
-        ws.fp64 += n_fp64;
-    }
+    flush();
 }
 
 // ---------------------------------------------------------------------------------
