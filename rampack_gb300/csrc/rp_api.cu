@@ -1920,6 +1920,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     if (ordered) order_starts(g, order_start);
     if (cl_warps) {
         SweepArgs a = sweep_args(tstep);
+        a.overflow_count = h->item_counters + 32;   // one a phase, zeroed by the kernel
         if (log) {
             a.log = h->d_log;
             a.log_codes = h->d_log_codes;

@@ -27,12 +27,15 @@ struct ClusterSweep {
 namespace {
 
 // The rebuild of launch_rebuild (assign, scan, scatter, finish), without the cells' occupancy
-// order, by all threads of the cluster; the scan by the first block.
-__device__ void cluster_rebuild(const DevState &s, const GridDev &g, const cooperative_groups::cluster_group &cl) {
+// order, by all threads of the cluster; the scan by the first block.  Also zeroes the phases' counts of
+// overfull neighbourhoods.
+__device__ void cluster_rebuild(const DevState &s, const GridDev &g, int32_t *overfull, int nphases,
+                                const cooperative_groups::cluster_group &cl) {
     __shared__ int32_t warp_tot[CL_MAX_WARPS], warp_max[CL_MAX_WARPS];
     const int rank = cl.block_rank(), T = blockDim.x;
     const int tid = rank * T + threadIdx.x, nth = cl.num_blocks() * T;
     for (int c = tid; c < g.ncell; c += nth) g.count[c] = 0;
+    if (tid < nphases) overfull[tid] = 0;
     cl.sync();
     for (int64_t i = tid; i < s.n; i += nth) assign_one(s, g, i);
     cl.sync();
@@ -86,7 +89,7 @@ __global__ void __launch_bounds__(CL_MAX_WARPS * 32, 1)
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, W = blockDim.x >> 5;
     const int rank = cl.block_rank(), nb = cl.num_blocks();
     const GridDev &G = A.g;
-    cluster_rebuild(A.s, G, cl);
+    cluster_rebuild(A.s, G, A.overflow_count, P.nphases, cl);
     __shared__ WarpStats stats[CL_MAX_WARPS];
     WarpStats &ws = stats[w];
     if (lane == 0) ws = WarpStats{};
@@ -96,7 +99,9 @@ __global__ void __launch_bounds__(CL_MAX_WARPS * 32, 1)
         int act[3];
         for (int d = 0; d < 3; d++) act[d] = ring_count(G.dims[d], phase_digit(ph, d));
         // pass 0: the phase's cells, one warp each; pass 1: those whose neighbourhood exceeds a
-        // warp's share of the shared memory, one block each
+        // warp's share of the shared memory, one block each.  Their count is the phase's own: a warp
+        // that reads it late, after others went on to the next phase, must not meet that phase's
+        int32_t *const overfull = A.overflow_count + p;
         int items = act[0] * act[1] * act[2];
         for (int pass = 0; pass < 2; pass++) {
             const int cap = pass == 0 ? A.cap : P.cap_big;
@@ -123,16 +128,13 @@ __global__ void __launch_bounds__(CL_MAX_WARPS * 32, 1)
                     cell = __ldcg(A.overflow + item);
                 }
                 sweep_cell<KIND, false, MODE, 32, SEG>(A, item, cell, cap, pass == 0 ? A.overflow : nullptr,
-                                                       A.overflow_count, cpos, cax, qseg, qun, nacc, nullptr, cslot, wx, ws);
+                                                       overfull, cpos, cax, qseg, qun, nacc, nullptr, cslot, wx, ws);
                 __syncwarp();
             }
             cl.sync();
             if (pass == 0) {
-                items = __ldcg(A.overflow_count);
+                items = __ldcg(overfull);
                 if (items == 0) break;
-            } else {
-                if (rank == 0 && threadIdx.x == 0) *A.overflow_count = 0;
-                cl.sync();
             }
         }
     }
