@@ -614,10 +614,9 @@ template <int F>
 cudaError_t launch_rows_t(const CorrGeom &G, const SortedPoints &S, const int32_t *start, int grid,
                           unsigned long long *hist, double *hsum, unsigned long long *tested, cudaStream_t st) {
     const size_t smem = size_t(G.nb) * (F != RP_CORR_DENSITY ? 12 : 4);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_corr_rows<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
+    // (always: 48 KB without asking hold the kernel's static shared memory too)
+    cudaError_t e = cudaFuncSetAttribute(k_corr_rows<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
     k_corr_rows<F><<<grid, CORR_THREADS, smem, st>>>(G, S, start, hist, hsum, tested);
     return cudaGetLastError();
 }
@@ -636,11 +635,9 @@ template <int E, int F>
 cudaError_t launch_pairs_t(const CorrGeom &G, const SortedPoints &S, const int32_t *start, int64_t n, int grid,
                            int use_smem, size_t smem, unsigned long long *hist, double *hsum,
                            unsigned long long *tested, cudaStream_t st) {
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(k_corr_pairs<E, F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(smem));
-        if (e != cudaSuccess) return e;
-    }
+    cudaError_t e = cudaFuncSetAttribute(k_corr_pairs<E, F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
     k_corr_pairs<E, F><<<grid, CORR_THREADS, smem, st>>>(G, S, start, n, use_smem, hist, hsum, tested);
     return cudaGetLastError();
 }
