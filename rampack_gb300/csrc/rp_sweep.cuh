@@ -1367,7 +1367,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
             }
             // the guard band: queued pairs re-decided in FP64
             if (KIND == 2 && code == 0 && (nun > 0 || unall)) {
-                const uint16_t *uq = unall ? qseg : qun;
+                const uint16_t *uq = unall ? qseg : qun;   // (qseg holds the mover too)
                 const int nu = unall ? nseg : nun;
                 // every centre pair of the queued bodies, one pair per lane: with K^2 <= 16,
                 // 32 / K^2 bodies per pass (the FP64 segment tests of polyspherocylinders
@@ -1385,7 +1385,7 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                     for (int tb = 0; tb < (per > 1 ? 1 : KK); tb += GW) {
                         const int t = per > 1 ? lane % KK : tb + lane;
                         bool hit = false;
-                        if (t < KK && qi < nu && (per == 1 || lane < per * KK)) {
+                        if (t < KK && qi < nu && (per == 1 || lane < per * KK) && __float_as_int(q.w) != pid) {
                             const int a = t / K, j = t % K;
                             const float4 m = wx[a];
                             const float4 c = cj[j];
