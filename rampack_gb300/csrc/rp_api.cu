@@ -1784,6 +1784,10 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     }
     RP_CUDA(h, cudaSetDevice(h->device));
     h->try_valid = false;
+    const bool convex = h->shape.kind == RP_SHAPE_CONVEX;
+    // (before the grid changes: a refused sweep leaves the lists that the grid's geometry names)
+    if ((h->soft || convex) && types == SWEEP_ROTOTRANSLATION)
+        return fail(h, RP_ERR_UNSUPPORTED, "rototranslations with a soft part or a convex body");
     // random grid origin and phase order from the Philox stream of this sweep
     u4 r = philox(u4{0x5eedu, 0x9e37u, static_cast<uint32_t>(p->counter), static_cast<uint32_t>(p->counter >> 32)},
                   static_cast<uint32_t>(p->seed), static_cast<uint32_t>(p->seed >> 32));
@@ -1798,12 +1802,9 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
                         !h->grid[h->gcur].no_ng && g.dims[0] >= 3 && g.dims[1] >= 3 && g.dims[2] >= 3 &&
                         (h->soft_only || !h->walls);
     // flat convex bodies take the FP32 sweep over such a grid too, with the pairs near contact in FP64
-    const bool convex = h->shape.kind == RP_SHAPE_CONVEX;
     const bool convex32 = convex && h->xc_flat && !h->counting && !h->walls && !(p->flags & RP_SWEEP_FP64_ONLY) &&
                           !h->grid[h->gcur].no_ng && g.dims[0] >= 3 && g.dims[1] >= 3 && g.dims[2] >= 3;
     const bool fp64_sweep = (h->soft && !soft32) || (convex && !convex32);
-    if ((soft32 || convex || fp64_sweep) && types == SWEEP_ROTOTRANSLATION)
-        return fail(h, RP_ERR_UNSUPPORTED, "rototranslations with a soft part or a convex body");
     std::vector<int> phases;
     grid_phases(g, r.d, phases);
     // the arguments every phase shares

@@ -1,0 +1,81 @@
+"""What the engine's host code does after an error: the engine's objects linked with a CUDA runtime that
+keeps device memory on the host, launches nothing and fails on request (tests/cpp/fake_cudart.cpp), each
+case in a process of its own."""
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+PROLOGUE = """
+import ctypes as C
+import sys
+import numpy as np
+from rampack_gb300 import _lib
+lib = _lib.load(sys.argv[1])
+lib.fake_launched.restype = C.c_char_p
+lib.fake_fail.argtypes = [C.c_char_p, C.c_int]
+from rampack_gb300 import workloads as W
+from rampack_gb300.packing import GpuPacking
+
+def fails(call, after, f):
+    lib.fake_fail(call.encode(), after)
+    try:
+        f()
+    except _lib.EngineError:
+        return True
+    finally:
+        lib.fake_fail(b"", -1)
+    return False
+
+def kernels(f):
+    lib.fake_launched()
+    f()
+    return lib.fake_launched().decode()
+
+def spheres(n=6):
+    return GpuPacking(W.SPHERE, np.array([0.5]), W.lattice((n,) * 3, (1.5,) * 3), W.aligned_rotations(n ** 3),
+                      W.diag_box(1.5 * n, 1.5 * n, 1.5 * n))
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(engine, tmp_path_factory):
+    from rampack_gb300 import build as B
+    objects = [os.path.join(B.HERE, "_build", s.replace(".cu", ".o")) for s in B.SOURCES]
+    if not all(os.path.exists(o) for o in objects):
+        B.build(force=True)
+    lib = str(tmp_path_factory.mktemp("fake") / "librampack_fake.so")
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(B.nvcc())))), "include")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-I", include,
+                    os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp"), *objects, "-o", lib], check=True)
+    return lib
+
+
+def run(fake, code):
+    p = subprocess.run([sys.executable, "-c", PROLOGUE + code, fake], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, p.stderr[-3000:]
+
+
+SHAPES = {
+    "convex": 'GpuPacking(W.CONVEX, "cuboid 1 1 2; sphere 0.1; sum", W.lattice((5, 5, 5), (4.0,) * 3),'
+              ' W.aligned_rotations(125), W.diag_box(20.0, 20.0, 20.0))',
+    "soft": "spheres()",
+}
+
+
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+def test_refused_rototranslations_leave_the_grid(fake, shape):
+    run(fake, f"""
+g = {SHAPES[shape]}
+if {shape!r} == "soft":
+    g.set_soft(_lib.SOFT_REPULSIVE_LJ, 1.0, 1.0, False)
+g.set_grid((0.25, 0.5, 0.75))
+before = g.grid()[2]
+assert fails("", -1, lambda: g.sweep(0.1, 0.1, seed=3, counter=0, rototranslation=True))
+# the lists are the grid's that was set: nothing rebuilt them, so its bounds must stand
+rebuilt = "k_scatter" in kernels(lambda: g.grid())
+assert rebuilt or np.array_equal(before, g.grid()[2])
+""")
