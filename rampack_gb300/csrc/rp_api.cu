@@ -1793,8 +1793,15 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
                   static_cast<uint32_t>(p->seed), static_cast<uint32_t>(p->seed >> 32));
     double shift[3] = {(r.a >> 8) * (1.0 / 16777216.0), (r.b >> 8) * (1.0 / 16777216.0),
                        (r.c >> 8) * (1.0 / 16777216.0)};
+    // the lists are out of date until the launch that builds them for the new origin has succeeded
+    h->grid_stale = true;
+    h->grid_patched = false;
     int rc = setup_grid(h, h->grid[h->gcur], h->box, shift);
     if (rc) return rc;
+    auto current = [h]() {
+        h->grid_stale = false;
+        h->stale_unshifted = false;
+    };
     const GridDev &g = h->grid[h->gcur].d;
     // spheres with a soft part take the FP32 sweep with an error bound on the energy change, over a
     // grid where a staged candidate is one image of another particle
@@ -1841,10 +1848,11 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         for (int ph : phases) most = std::max(most, phase_cells(g, ph, act));
         cl_warps = cluster_warps(sweep_args(0.0), h->cl_blocks, most);
     }
-    rc = cl_warps ? rebuilt(h) : rebuild(h, h->gcur, h->pcur);
-    if (rc) return rc;
-    h->grid_stale = false;
-    h->stale_unshifted = false;
+    if (!cl_warps) {
+        rc = rebuild(h, h->gcur, h->pcur);
+        if (rc) return rc;
+        current();
+    }
     // translation step limited to half the smallest box height (TranslationSampler.cpp:39-46)
     double hgt[3];
     heights_of(h->box, hgt);
@@ -1927,8 +1935,13 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
             a.log_codes = h->d_log_codes;
         }
         h->last_cells_per_warp = 1;
-        Group grp(h, RP_KERNEL_SWEEP, 1);
-        RP_CUDA(h, launch_cluster_sweep(a, phases.data(), static_cast<int>(phases.size()), h->cl_blocks, cl_warps, h->stream));
+        {
+            Group grp(h, RP_KERNEL_SWEEP, 1);
+            RP_CUDA(h, launch_cluster_sweep(a, phases.data(), static_cast<int>(phases.size()), h->cl_blocks, cl_warps, h->stream));
+        }
+        rc = rebuilt(h);
+        if (rc) return rc;
+        current();
     }
     for (int ph : (fp64_sweep || cl_warps ? std::vector<int>{} : phases)) {
         SweepArgs a = sweep_args(tstep);

@@ -171,7 +171,8 @@ cudaError_t launch_t(const SweepArgs &a, const ClusterSweep &p, int blocks, int 
     cfg.numAttrs = 1;
     if (probe) return cudaOccupancyMaxActiveClusters(fits, kernel, &cfg);
     e = cudaLaunchKernelEx(&cfg, kernel, a, p);
-    return e != cudaSuccess ? e : cudaGetLastError();
+    const cudaError_t last = cudaGetLastError();   // (taken: the next launch must not report this one's)
+    return e != cudaSuccess ? e : last;
 }
 
 cudaError_t dispatch(const SweepArgs &a, const ClusterSweep &p, int blocks, int warps, cudaStream_t st, bool probe, int *fits) {

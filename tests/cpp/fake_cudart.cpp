@@ -15,6 +15,7 @@ std::string launched;
 std::string fail_call;
 int fail_after = -1;
 int allocations = 0;
+cudaError_t last_error = cudaSuccess;
 struct {
     dim3 grid, block;
     size_t smem;
@@ -39,7 +40,7 @@ cudaError_t launch(const void *f) {
     const auto it = names.find(f);
     const std::string name = it == names.end() ? "?" : it->second;
     if (fails("launch") || (fail_after >= 0 && name.find(fail_call) != std::string::npos && fail_after-- == 0))
-        return cudaErrorLaunchOutOfResources;
+        return last_error = cudaErrorLaunchOutOfResources;
     launched += name + "\n";
     return cudaSuccess;
 }
@@ -150,7 +151,11 @@ cudaError_t cudaGetSymbolAddress(void **p, const void *s) {
     return cudaSuccess;
 }
 const char *cudaGetErrorString(cudaError_t) { return "a fake error"; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError() {
+    const cudaError_t e = last_error;
+    last_error = cudaSuccess;
+    return e;
+}
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaDeviceSetLimit(cudaLimit, size_t) { return cudaSuccess; }
 cudaError_t cudaDeviceSynchronize() { return cudaSuccess; }

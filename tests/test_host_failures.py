@@ -79,3 +79,16 @@ assert fails("", -1, lambda: g.sweep(0.1, 0.1, seed=3, counter=0, rototranslatio
 rebuilt = "k_scatter" in kernels(lambda: g.grid())
 assert rebuilt or np.array_equal(before, g.grid()[2])
 """)
+
+
+@pytest.mark.parametrize("call", ["cudaMalloc", "cudaMemsetAsync", "k_rot_table", "k_cluster_sweep"])
+def test_a_failed_small_sweep_leaves_no_grid_behind(fake, call):
+    run(fake, f"""
+g = spheres()
+g.set_grid()
+assert "k_cluster_sweep" in kernels(lambda: g.sweep(0.1, 0.0, seed=3, counter=0))
+reads = [g.count_total_overlaps, lambda: fails("", -1, lambda: g.try_move(0, 0, (0.1, 0.0, 0.0))), g.grid]
+for counter, read in enumerate(reads):
+    assert fails({call!r}, 0, lambda: g.sweep(0.1, 0.1, seed=3, counter=counter, log=True))
+    assert "k_scatter" in kernels(read), counter
+""")
