@@ -2239,15 +2239,20 @@ int rp_try_move(void *handle, const rp_move *move, const double *domain6, double
     if (move->particle < 0 || move->particle >= h->n) return fail(h, RP_ERR_ARG, "particle index out of range");
     RP_CUDA(h, cudaSetDevice(h->device));
     h->try_valid = false;
-    if (!h->d_try) {
-        RP_CUDA(h, cudaMalloc(&h->d_try, sizeof(SingleTry)));
-        RP_CUDA(h, cudaMallocHost(&h->try_result, sizeof(SingleResult)));
-        *h->try_result = SingleResult{};
-        RP_CUDA(h, cudaMalloc(&h->d_disp_list, sizeof(int32_t) * Handle::DISP_CAP));
-        RP_CUDA(h, cudaMalloc(&h->d_disp_flag, static_cast<size_t>(h->n)));
-        RP_CUDA(h, cudaMemsetAsync(h->d_disp_flag, 0, static_cast<size_t>(h->n), h->stream));
+    // (the flags last: buffers that an earlier call could not get are asked for again)
+    if (!h->d_disp_flag) {
+        if (!h->d_try) RP_CUDA(h, cudaMalloc(&h->d_try, sizeof(SingleTry)));
+        if (!h->try_result) {
+            RP_CUDA(h, cudaMallocHost(&h->try_result, sizeof(SingleResult)));
+            *h->try_result = SingleResult{};
+        }
+        if (!h->d_disp_list) RP_CUDA(h, cudaMalloc(&h->d_disp_list, sizeof(int32_t) * Handle::DISP_CAP));
         h->disp_flag_host.assign(static_cast<size_t>(h->n), 0);
         h->disp_host.clear();
+        uint8_t *flags = nullptr;
+        RP_CUDA(h, cudaMalloc(&flags, static_cast<size_t>(h->n)));
+        h->d_disp_flag = flags;
+        RP_CUDA(h, cudaMemsetAsync(h->d_disp_flag, 0, static_cast<size_t>(h->n), h->stream));
     }
     // the grid serves single moves while only particles moved by single moves are out of
     // place (and few enough of them); otherwise it is rebuilt first

@@ -92,3 +92,20 @@ for counter, read in enumerate(reads):
     assert fails({call!r}, 0, lambda: g.sweep(0.1, 0.1, seed=3, counter=counter, log=True))
     assert "k_scatter" in kernels(read), counter
 """)
+
+
+@pytest.mark.parametrize("call,after", [("cudaMalloc", 0), ("cudaMalloc", 1), ("cudaMalloc", 2), ("cudaHostAlloc", 0)])
+def test_a_single_move_after_a_failed_allocation_has_its_buffers(fake, call, after):
+    run(fake, f"""
+def buffers(after):
+    g = spheres()
+    g.set_grid()
+    lib.fake_allocations()
+    if after >= 0:
+        assert fails({call!r}, after, lambda: g.try_move(0, 0, (0.1, 0.0, 0.0)))
+    # (the kernel does nothing here: its answer is missed, not looked for at a null address)
+    assert "k_try_single" in kernels(lambda: fails("", -1, lambda: g.try_move(0, 0, (0.1, 0.0, 0.0))))
+    return lib.fake_allocations()
+
+assert buffers({after}) == buffers(-1) > 3
+""")
