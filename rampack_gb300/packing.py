@@ -54,6 +54,17 @@ assert C.sizeof(MoveRecord) == MOVE_DTYPE.itemsize
 IDENTITY = (1.0, 0.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0, 1.0)
 
 
+def int32_of(value) -> int:
+    """A value as the assignment to a numpy int32 array takes it: one number, in any shape."""
+    if type(value) is not int:
+        a = np.zeros(1, dtype=np.int32)
+        a[:] = value
+        return int(a[0])
+    if not -0x80000000 <= value <= 0x7fffffff:
+        raise OverflowError("an integer beyond 32 bits")
+    return value
+
+
 class GpuPacking:
     def __init__(self, kind: int, params, pos, rot, box, device: int = 0):
         self.lib = _lib.load()
@@ -202,9 +213,7 @@ class GpuPacking:
         """Packing::tryTranslation / tryRotation / tryMove (rp_try_move), with no ActiveDomain or
         with `domain` = its relative bounds (lo[3], hi[3]): the move's energy (0 or +inf; -inf,
         0 or +inf in overlap counting); the tried state waits for accept_move."""
-        particle, type_ = int(particle), int(type_)
-        if not -0x80000000 <= particle <= 0x7fffffff or not -0x80000000 <= type_ <= 0x7fffffff:
-            raise OverflowError("a particle index or move type beyond 32 bits")
+        particle, type_ = int32_of(particle), int32_of(type_)
         m = MoveRecord(particle=particle, type=type_, domain=-1)
         m.translation[:] = np.asarray(translation, dtype=np.float64).reshape(3).tolist()
         m.rotation[:] = IDENTITY if rotation is None else np.asarray(rotation, dtype=np.float64).reshape(9).tolist()
