@@ -1886,6 +1886,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         sa.c.g = g;
         sa.c.temperature = h->temperature;
         set_prefilter(sa.c, h);
+        sa.c.fp64_only = (p->flags & RP_SWEEP_FP64_ONLY) ? 1 : 0;
         sa.seed = p->seed;
         sa.counter = p->counter;
         sa.tstep = static_cast<float>(tstep);

@@ -188,7 +188,7 @@ __device__ int candidate_overlaps(const SingleArgs &A, const double *p, d3 a, co
                     ai = make_float3(static_cast<float>(a.x), static_cast<float>(a.y), static_cast<float>(a.z));
                     aj = make_float3(static_cast<float>(rj[2]), static_cast<float>(rj[5]), static_cast<float>(rj[8]));
                 }
-                const int cls = classify<KIND>(s.fc, d, ai, aj);
+                const int cls = A.fp64_only ? 2 : classify<KIND>(s.fc, d, ai, aj);
                 if (cls == 0) return false;
                 if (cls == 2 && !body_overlap<KIND>(s, pp, a, rot, j, &t)) return false;
             } else if (!body_overlap<KIND>(s, pp, a, rot, j, &t)) {

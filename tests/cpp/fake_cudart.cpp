@@ -8,6 +8,8 @@
 #include <map>
 #include <string>
 
+#include "rp_internal.cuh"
+
 namespace {
 
 std::map<const void *, std::string> names;
@@ -15,6 +17,7 @@ std::string launched;
 std::string fail_call;
 int fail_after = -1;
 int allocations = 0;
+rp::SoftSweepArgs soft{};   // of the last FP64 sweep
 cudaError_t last_error = cudaSuccess;
 struct {
     dim3 grid, block;
@@ -36,12 +39,13 @@ cudaError_t allocate(const char *call, void **p, size_t bytes) {
     return cudaSuccess;
 }
 
-cudaError_t launch(const void *f) {
+cudaError_t launch(const void *f, void **args) {
     const auto it = names.find(f);
     const std::string name = it == names.end() ? "?" : it->second;
     if (fails("launch") || (fail_after >= 0 && name.find(fail_call) != std::string::npos && fail_after-- == 0))
         return last_error = cudaErrorLaunchOutOfResources;
     launched += name + "\n";
+    if (name.find("k_soft_sweep") != std::string::npos) soft = *static_cast<const rp::SoftSweepArgs *>(args[0]);
     return cudaSuccess;
 }
 
@@ -67,6 +71,9 @@ int fake_allocations() {
     allocations = 0;
     return n;
 }
+
+// Whether the last FP64 sweep was to do without the FP32 filter.
+int fake_soft_fp64_only() { return soft.c.fp64_only; }
 
 void **__cudaRegisterFatBinary(void *) {
     static void *handle = nullptr;
@@ -94,8 +101,8 @@ cudaError_t __cudaPopCallConfiguration(dim3 *grid, dim3 *block, size_t *smem, vo
     *static_cast<cudaStream_t *>(stream) = config.stream;
     return cudaSuccess;
 }
-cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void **, size_t, cudaStream_t) { return launch(k); }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *f, void **) { return launch(f); }
+cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void **args, size_t, cudaStream_t) { return launch(k, args); }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *f, void **args) { return launch(f, args); }
 
 cudaError_t cudaMalloc(void **p, size_t bytes) { return allocate("cudaMalloc", p, bytes); }
 cudaError_t cudaHostAlloc(void **p, size_t bytes, unsigned) { return allocate("cudaHostAlloc", p, bytes); }

@@ -1,4 +1,4 @@
-"""What the engine's host code does after an error: the engine's objects linked with a CUDA runtime that
+"""What the engine's host code does after an error, and what it asks of its kernels: the engine's objects linked with a CUDA runtime that
 keeps device memory on the host, launches nothing and fails on request (tests/cpp/fake_cudart.cpp), each
 case in a process of its own."""
 import os
@@ -49,8 +49,8 @@ def fake(engine, tmp_path_factory):
         B.build(force=True)
     lib = str(tmp_path_factory.mktemp("fake") / "librampack_fake.so")
     include = os.path.join(os.path.dirname(os.path.dirname(os.path.realpath(shutil.which(B.nvcc())))), "include")
-    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-I", include,
-                    os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp"), *objects, "-o", lib], check=True)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-I", include, "-I", B.CSRC,
+                    "-I", os.path.join(ROOT, "include"), os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp"), *objects, "-o", lib], check=True)
     return lib
 
 
@@ -108,4 +108,16 @@ def buffers(after):
     return lib.fake_allocations()
 
 assert buffers({after}) == buffers(-1) > 3
+""")
+
+
+@pytest.mark.parametrize("kind", ["W.SPHERE, np.array([0.5])", "W.SPHEROCYLINDER, np.array([0.3, 0.5])"])
+def test_fp64_only_reaches_the_hard_pairs_of_soft_sweeps(fake, kind):
+    run(fake, f"""
+g = GpuPacking({kind}, W.lattice((6, 6, 6), (1.9,) * 3), W.aligned_rotations(216), W.diag_box(11.4, 11.4, 11.4))
+g.set_soft(_lib.SOFT_SQUARE_INVERSE_CORE, 1.0, 1.2, True)
+for only in (True, False, True):
+    k = kernels(lambda: g.sweep(0.1, 0.1, seed=3, counter=0, fp64_only=only))
+    assert "k_soft_sweep" in k or not only
+    assert "k_soft_sweep" not in k or lib.fake_soft_fp64_only() == only
 """)
