@@ -312,7 +312,9 @@ __device__ __forceinline__ bool examine_pair(const CorrGeom &G, const SortedPoin
 template <int E, int F>
 __global__ void __launch_bounds__(CORR_THREADS, 2) k_corr_pairs(CorrGeom G, SortedPoints S, const int32_t *start,
                                                              int64_t n, int use_smem, unsigned long long *hist,
-                                                             double *hsum, unsigned long long *tested) {
+                                                             double *hsum, unsigned long long *tested,
+                                                             const int32_t *max_occ, int row_occ) {
+    if (*max_occ <= row_occ) return;   // k_corr_rows took this snapshot
     extern __shared__ unsigned long long sh[];
     unsigned long long *hc = hist;
     double *hs = hsum;
@@ -433,12 +435,15 @@ __global__ void __launch_bounds__(CORR_THREADS, 2) k_corr_pairs(CorrGeom G, Sort
 // part of d / step unless d / step lies within `row_margin` of an integer or of the last bin's end;
 // those pairs are queued for decide_pair, and so are, for the averaged correlations, all in-range pairs
 // (with their bin), so that the FP64 axis functions run on full warps.  Counts are 32 bits wide per
-// block; the host gives every block at most 2^32 pairs.
+// block; a snapshot whose fullest cell holds more than `row_occ` points, which could overflow them or
+// leave most of the work to a few warps, is left to the general kernel (launched behind it).
 constexpr int ROW_POINTS = 4;   // 2.87, 2.54 and 2.55 ms a snapshot of 10^6 points for 2, 4 and 8
 template <int F>
 __global__ void __launch_bounds__(CORR_THREADS) k_corr_rows(CorrGeom G, SortedPoints S, const int32_t *start,
                                                             unsigned long long *hist, double *hsum,
-                                                            unsigned long long *tested) {
+                                                            unsigned long long *tested, const int32_t *max_occ,
+                                                            int row_occ) {
+    if (*max_occ > row_occ) return;
     extern __shared__ unsigned long long sh[];
     constexpr bool AVG = F != RP_CORR_DENSITY;
     double *hs = reinterpret_cast<double *>(sh);                        // averaged correlations: value sums
@@ -612,51 +617,53 @@ __global__ void __launch_bounds__(CORR_THREADS) k_corr_rows(CorrGeom G, SortedPo
 
 template <int F>
 cudaError_t launch_rows_t(const CorrGeom &G, const SortedPoints &S, const int32_t *start, int grid,
-                          unsigned long long *hist, double *hsum, unsigned long long *tested, cudaStream_t st) {
+                          unsigned long long *hist, double *hsum, unsigned long long *tested, const int32_t *max_occ,
+                          int row_occ, cudaStream_t st) {
     const size_t smem = size_t(G.nb) * (F != RP_CORR_DENSITY ? 12 : 4);
     // (always: 48 KB without asking hold the kernel's static shared memory too)
     cudaError_t e = cudaFuncSetAttribute(k_corr_rows<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    k_corr_rows<F><<<grid, CORR_THREADS, smem, st>>>(G, S, start, hist, hsum, tested);
+    k_corr_rows<F><<<grid, CORR_THREADS, smem, st>>>(G, S, start, hist, hsum, tested, max_occ, row_occ);
     return cudaGetLastError();
 }
 
 cudaError_t launch_rows(int f, const CorrGeom &G, const SortedPoints &S, const int32_t *start, int grid,
-                        unsigned long long *hist, double *hsum, unsigned long long *tested, cudaStream_t st) {
+                        unsigned long long *hist, double *hsum, unsigned long long *tested, const int32_t *max_occ,
+                        int row_occ, cudaStream_t st) {
     switch (f) {
-        case RP_CORR_DENSITY: return launch_rows_t<RP_CORR_DENSITY>(G, S, start, grid, hist, hsum, tested, st);
-        case RP_CORR_S110: return launch_rows_t<RP_CORR_S110>(G, S, start, grid, hist, hsum, tested, st);
-        case RP_CORR_S220: return launch_rows_t<RP_CORR_S220>(G, S, start, grid, hist, hsum, tested, st);
-        default: return launch_rows_t<RP_CORR_AXES_ANGLE>(G, S, start, grid, hist, hsum, tested, st);
+        case RP_CORR_DENSITY: return launch_rows_t<RP_CORR_DENSITY>(G, S, start, grid, hist, hsum, tested, max_occ, row_occ, st);
+        case RP_CORR_S110: return launch_rows_t<RP_CORR_S110>(G, S, start, grid, hist, hsum, tested, max_occ, row_occ, st);
+        case RP_CORR_S220: return launch_rows_t<RP_CORR_S220>(G, S, start, grid, hist, hsum, tested, max_occ, row_occ, st);
+        default: return launch_rows_t<RP_CORR_AXES_ANGLE>(G, S, start, grid, hist, hsum, tested, max_occ, row_occ, st);
     }
 }
 
 template <int E, int F>
 cudaError_t launch_pairs_t(const CorrGeom &G, const SortedPoints &S, const int32_t *start, int64_t n, int grid,
                            int use_smem, size_t smem, unsigned long long *hist, double *hsum,
-                           unsigned long long *tested, cudaStream_t st) {
+                           unsigned long long *tested, const int32_t *max_occ, int row_occ, cudaStream_t st) {
     cudaError_t e = cudaFuncSetAttribute(k_corr_pairs<E, F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     if (e != cudaSuccess) return e;
-    k_corr_pairs<E, F><<<grid, CORR_THREADS, smem, st>>>(G, S, start, n, use_smem, hist, hsum, tested);
+    k_corr_pairs<E, F><<<grid, CORR_THREADS, smem, st>>>(G, S, start, n, use_smem, hist, hsum, tested, max_occ, row_occ);
     return cudaGetLastError();
 }
 
 template <int E>
 cudaError_t launch_pairs_e(int f, const CorrGeom &G, const SortedPoints &S, const int32_t *start, int64_t n,
                            int grid, int use_smem, size_t smem, unsigned long long *hist, double *hsum,
-                           unsigned long long *tested, cudaStream_t st) {
+                           unsigned long long *tested, const int32_t *max_occ, int row_occ, cudaStream_t st) {
     switch (f) {
         case RP_CORR_DENSITY:
-            return launch_pairs_t<E, RP_CORR_DENSITY>(G, S, start, n, grid, use_smem, smem, hist, hsum, tested, st);
+            return launch_pairs_t<E, RP_CORR_DENSITY>(G, S, start, n, grid, use_smem, smem, hist, hsum, tested, max_occ, row_occ, st);
         case RP_CORR_S110:
-            return launch_pairs_t<E, RP_CORR_S110>(G, S, start, n, grid, use_smem, smem, hist, hsum, tested, st);
+            return launch_pairs_t<E, RP_CORR_S110>(G, S, start, n, grid, use_smem, smem, hist, hsum, tested, max_occ, row_occ, st);
         case RP_CORR_S220:
-            return launch_pairs_t<E, RP_CORR_S220>(G, S, start, n, grid, use_smem, smem, hist, hsum, tested, st);
+            return launch_pairs_t<E, RP_CORR_S220>(G, S, start, n, grid, use_smem, smem, hist, hsum, tested, max_occ, row_occ, st);
         case RP_CORR_S221:
-            return launch_pairs_t<E, RP_CORR_S221>(G, S, start, n, grid, use_smem, smem, hist, hsum, tested, st);
+            return launch_pairs_t<E, RP_CORR_S221>(G, S, start, n, grid, use_smem, smem, hist, hsum, tested, max_occ, row_occ, st);
         default:
-            return launch_pairs_t<E, RP_CORR_AXES_ANGLE>(G, S, start, n, grid, use_smem, smem, hist, hsum, tested,
+            return launch_pairs_t<E, RP_CORR_AXES_ANGLE>(G, S, start, n, grid, use_smem, smem, hist, hsum, tested, max_occ, row_occ,
                                                          st);
     }
 }
@@ -961,6 +968,20 @@ int add_snapshot(Corr *c, void *handle) {
         G.row_thr2 = static_cast<float>(reach_row * reach_row * (1 + 1e-6));
         G.row_margin = static_cast<float>(m_row / G.step * (1 + 1e-6) + 1e-6 * d.num_bins);
         by_rows = by_rows && G.row_margin < 0.25f;
+        // A warp per cell saves the general kernel's set-up of a warp per point and most of its work per
+        // pair, and pays with one warp's chain of candidate rounds (four points, 32 candidates each) over
+        // its cell's rows, where the general kernel spreads a cell over its points' warps, and for the
+        // averaged functions with its queues in every cell.  Both sides in microseconds, fitted to
+        // snapshots of 400 to 330,000 points at 0.5 to 60 a cell (the rule takes the faster kernel, or
+        // one at most 6 % slower for the density and 10 % for the averaged functions): 2,250 points in
+        // 128 cells took 138 us by rows and 88 us without; 31,104 points in 6,975 cells 152 and 216 us.
+        const double occ = static_cast<double>(v.n) / static_cast<double>(ncell);
+        const double rows = (2 * G.span[1] + 1) * (2 * G.span[2] + 1), wide = 2 * G.span[0] + 1;
+        const double pairs = 0.5 * static_cast<double>(v.n) * rows * wide * occ;
+        const double chain = (occ / 4 + 0.7) * rows * (wide * occ / 32 + 0.7);
+        by_rows = by_rows && (is_density(d) ? 13.5e-6 * pairs + 1e-3 * static_cast<double>(v.n) > 0.8 * chain + 5
+                                            : 4e-6 * pairs + 3e-3 * static_cast<double>(v.n) >
+                                                  0.6 * chain + 2.5e-3 * static_cast<double>(ncell));
     }
 
     rc = ensure_buffers(c, v, ncell, axes);
@@ -1007,31 +1028,31 @@ int add_snapshot(Corr *c, void *handle) {
         const int use_smem = nb <= SMEM_BINS ? 1 : 0;
         const size_t smem = use_smem ? size_t(nb) * (axes ? 16 : 8) : 0;
         cudaError_t le = cudaSuccess;
-        int32_t occ = 0;
+        // the fullest cell for which the row kernel takes the snapshot (0: never): a few times the mean,
+        // so that no warp's cell holds the work of many (half of 64,000 points in a droplet: 0.31 ms by
+        // rows, 0.24 without), and at most what lets a block count its pairs in 32 bits, each of its
+        // cells' points with every point of 125 cells.  The kernels compare it on the device: reading
+        // the fullest cell back cost 10 us a snapshot
+        int row_occ = 0;
         if (by_rows) {
-            // a block's pairs fit its 32-bit counts: at most max_occ points of each of its cells, each
-            // with every point of 125 cells
-            CORR_CUDA(c, cudaMemcpyAsync(&occ, c->max_occ, sizeof(occ), cudaMemcpyDeviceToHost, st));
-            CORR_CUDA(c, cudaStreamSynchronize(st));
             const int64_t wpb = CORR_THREADS / 32, cblk = (ncell + wpb - 1) / wpb;
-            int64_t blocks = std::min<int64_t>(cblk, int64_t(dev_sms) * 8);
-            const double most = 125.0 * occ * occ;   // pairs of one cell
-            while (blocks < cblk && static_cast<double>((cblk + blocks - 1) / blocks * wpb) * most > 4.2e9) blocks *= 2;
-            by_rows = wpb * most <= 4.2e9;
-            if (by_rows)
-                le = launch_rows(d.function, G, c->S, c->start, static_cast<int>(std::min(blocks, cblk)), c->hist, c->hsum,
-                                 c->tested, st);
+            const int64_t blocks = std::min<int64_t>(cblk, int64_t(dev_sms) * 8);
+            const double cells = static_cast<double>((cblk + blocks - 1) / blocks * wpb);
+            row_occ = static_cast<int>(std::min(4.0 * static_cast<double>(v.n) / static_cast<double>(ncell) + 16.0,
+                                                std::sqrt(4.2e9 / (125.0 * cells))));
+            le = launch_rows(d.function, G, c->S, c->start, static_cast<int>(blocks), c->hist, c->hsum, c->tested,
+                             c->max_occ, row_occ, st);
+            CORR_CUDA(c, le);
         }
-        if (by_rows) {
-        } else if (d.enumerator == RP_PAIRS_RADIAL)
+        if (d.enumerator == RP_PAIRS_RADIAL)
             le = launch_pairs_e<RP_PAIRS_RADIAL>(d.function, G, c->S, c->start, v.n, grid, use_smem, smem, c->hist,
-                                                 c->hsum, c->tested, st);
+                                                 c->hsum, c->tested, c->max_occ, row_occ, st);
         else if (d.enumerator == RP_PAIRS_LINEAR)
             le = launch_pairs_e<RP_PAIRS_LINEAR>(d.function, G, c->S, c->start, v.n, grid, use_smem, smem, c->hist,
-                                                 c->hsum, c->tested, st);
+                                                 c->hsum, c->tested, c->max_occ, row_occ, st);
         else
             le = launch_pairs_e<RP_PAIRS_LAYERWISE>(d.function, G, c->S, c->start, v.n, grid, use_smem, smem,
-                                                    c->hist, c->hsum, c->tested, st);
+                                                    c->hist, c->hsum, c->tested, c->max_occ, row_occ, st);
         CORR_CUDA(c, le);
     }
     std::vector<unsigned long long> cnt(nb);
