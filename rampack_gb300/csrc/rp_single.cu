@@ -19,6 +19,8 @@
 // order than the reference's neighbour-grid walk).  Candidates come from the handle's cell
 // grid (cells at least one interaction range high); particles moved by single moves since the
 // grid was built are skipped in their old cells and tested from a short list instead.
+#include <algorithm>
+
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
@@ -159,16 +161,48 @@ __device__ __forceinline__ void for_each_image(const SingleArgs &A, float3 sep, 
                 if (within_reach(A, sep, mx, my, mz) && f(mx, my, mz)) return;
 }
 
+// Overlapping centre pairs of a multi-centre mover state (absolute centres abs, half axes hax) with body
+// j over every periodic image within reach (each absolute centre is wrapped into the box on its own, so
+// images are enumerated per centre pair); at most 1 with `early`.  Out of line: inlined into the loop
+// over a warp's candidates, its early returns kept the lanes apart for the rest of the loop (a five-sphere
+// chain's move on eight warps took 178 us, now 59; the segments of bent rods 70 and 52 us).
+__device__ __noinline__ int centre_overlaps(const SingleArgs &A, const double *abs, const double *hax, int j, bool early) {
+    const DevState &s = A.s;
+    int cnt = 0;
+    for (int ca = 0; ca < s.ncen; ca++) {
+        const d3 pa{abs[3 * ca], abs[3 * ca + 1], abs[3 * ca + 2]};
+        const d3 ha = hax ? d3{hax[3 * ca], hax[3 * ca + 1], hax[3 * ca + 2]} : d3{0.0, 0.0, 0.0};
+        for (int b = 0; b < s.ncen; b++) {
+            if (s.pbc_fold) {
+                if (centre_overlap(s, pa, ha, ca, j, b, nullptr)) {
+                    if (early) return 1;
+                    cnt++;
+                }
+                continue;
+            }
+            const float3 sep = separation32(s.abs64 + 3 * ((size_t)j * s.ncen + b), abs + 3 * ca);
+            for_each_image(A, sep, [&](int mx, int my, int mz) {
+                const d3 t = image_translation(s, mx, my, mz);
+                if (!centre_overlap(s, pa, ha, ca, j, b, &t)) return false;
+                cnt++;
+                return early;
+            });
+            if (early && cnt) return 1;
+        }
+    }
+    return cnt;
+}
+
 // Overlapping pairs of a mover state (position p, axis a; multi-centre: absolute centres abs,
-// half axes hax) with body j over every periodic image within reach (each absolute centre is
-// wrapped into the box on its own, so images are enumerated per centre pair); at most 1 with
-// `early`.
+// half axes hax) with body j over every periodic image within reach; at most 1 with `early`.
 template <int KIND>
 __device__ int candidate_overlaps(const SingleArgs &A, const double *p, d3 a, const double *rot, const double *abs,
                                   const double *hax, int j, bool early) {
-    const DevState &s = A.s;
-    int cnt = 0;
-    if constexpr (KIND != 2) {
+    if constexpr (KIND == 2) {
+        return centre_overlaps(A, abs, hax, j, early);
+    } else {
+        const DevState &s = A.s;
+        int cnt = 0;
         const d3 pp{p[0], p[1], p[2]};
         if (s.pbc_fold) return body_overlap<KIND>(s, pp, a, rot, j, nullptr) ? 1 : 0;
         const float3 sep = separation32(s.pos64 + 3 * (size_t)j, p);
@@ -197,29 +231,6 @@ __device__ int candidate_overlaps(const SingleArgs &A, const double *p, d3 a, co
             cnt++;
             return early;
         });
-        return cnt;
-    } else {
-        for (int ca = 0; ca < s.ncen; ca++) {
-            const d3 pa{abs[3 * ca], abs[3 * ca + 1], abs[3 * ca + 2]};
-            const d3 ha = hax ? d3{hax[3 * ca], hax[3 * ca + 1], hax[3 * ca + 2]} : d3{0.0, 0.0, 0.0};
-            for (int b = 0; b < s.ncen; b++) {
-                if (s.pbc_fold) {
-                    if (centre_overlap(s, pa, ha, ca, j, b, nullptr)) {
-                        if (early) return 1;
-                        cnt++;
-                    }
-                    continue;
-                }
-                const float3 sep = separation32(s.abs64 + 3 * ((size_t)j * s.ncen + b), abs + 3 * ca);
-                for_each_image(A, sep, [&](int mx, int my, int mz) {
-                    const d3 t = image_translation(s, mx, my, mz);
-                    if (!centre_overlap(s, pa, ha, ca, j, b, &t)) return false;
-                    cnt++;
-                    return early;
-                });
-                if (early && cnt) return 1;
-            }
-        }
         return cnt;
     }
 }
@@ -584,16 +595,18 @@ __device__ double move_energy(const SingleArgs &A, const Mover &mv, int pid, int
     return dsub(final_, initial);
 }
 
-// One single move: the first warp builds the mover, TRY_WARPS warps share its candidates (a warp
-// alone walked a rod's 200 candidates in seven dependent rounds), and the
-// host reads the answer from page-locked memory.
-constexpr int TRY_WARPS = 8;
-template <int KIND>
-__global__ void __launch_bounds__(TRY_WARPS * 32) k_try_single(const __grid_constant__ SingleArgs A) {
+// One single move: the first warp builds the mover, WARPS warps share its candidates, and the host
+// reads the answer from page-locked memory.  Eight warps (a warp alone walked a rod's 200 candidates in
+// seven dependent rounds), but one for convex bodies with at most four rounds of candidates on average,
+// unless overlaps are counted: it ends at the first certain overlap, and eight share the SM for portal
+// refinements that are then not needed (110 candidates: a rejected move 43 against 77 us, an accepted
+// one 34 either way; 196 candidates: 84 against 68 us).
+template <int KIND, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) k_try_single(const __grid_constant__ SingleArgs A) {
     __shared__ Mover mv;
-    __shared__ int xq[KIND == 3 ? TRY_WARPS : 1][XC_QUEUE];
+    __shared__ int xq[KIND == 3 ? WARPS : 1][XC_QUEUE];
     __shared__ int count[2];
-    __shared__ double part[2][TRY_WARPS];
+    __shared__ double part[2][WARPS];
     const DevState &s = A.s;
     const int pid = A.m.particle, w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x < 2) count[threadIdx.x] = 0;
@@ -602,7 +615,7 @@ __global__ void __launch_bounds__(TRY_WARPS * 32) k_try_single(const __grid_cons
                           A.has_domain ? A.dom_hi : nullptr, nullptr);
     __syncthreads();
     // move_energy with the candidates shared (every branch is the whole block's)
-    const int first = 32 * w, step = 32 * TRY_WARPS;
+    const int first = 32 * w, step = 32 * WARPS;
     int *q = xq[KIND == 3 ? w : 0];
     int delta = 0;
     double dE = mv.outside ? CUDART_INF : 0.0;
@@ -627,7 +640,7 @@ __global__ void __launch_bounds__(TRY_WARPS * 32) k_try_single(const __grid_cons
         __syncthreads();
         double e[2] = {0.0, 0.0};
         for (int which = 0; which < 2; which++)
-            for (int k = 0; k < TRY_WARPS; k++) e[which] = dadd(e[which], part[which][k]);
+            for (int k = 0; k < WARPS; k++) e[which] = dadd(e[which], part[which][k]);
         dE = dsub(e[0], e[1]);
     }
     __syncthreads();   // every thread's status bits are raised
@@ -989,10 +1002,11 @@ __global__ void k_sum_fixed(const double *v, int64_t n, double *out) {
 }  // namespace
 
 cudaError_t launch_try_single(const SingleArgs &a, cudaStream_t st) {
-    if (a.s.kind == 0) k_try_single<0><<<1, TRY_WARPS * 32, 0, st>>>(a);
-    else if (a.s.kind == 1) k_try_single<1><<<1, TRY_WARPS * 32, 0, st>>>(a);
-    else if (a.s.kind == 2) k_try_single<2><<<1, TRY_WARPS * 32, 0, st>>>(a);
-    else k_try_single<3><<<1, TRY_WARPS * 32, 0, st>>>(a);
+    if (a.s.kind == 0) k_try_single<0, 8><<<1, 256, 0, st>>>(a);
+    else if (a.s.kind == 1) k_try_single<1, 8><<<1, 256, 0, st>>>(a);
+    else if (a.s.kind == 2) k_try_single<2, 8><<<1, 256, 0, st>>>(a);
+    else if (a.s.counting || a.s.n * std::min(a.g.ncell, 27) > 128ll * a.g.ncell) k_try_single<3, 8><<<1, 256, 0, st>>>(a);
+    else k_try_single<3, 1><<<1, 32, 0, st>>>(a);
     return cudaGetLastError();
 }
 

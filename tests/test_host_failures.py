@@ -121,3 +121,16 @@ for only in (True, False, True):
     assert "k_soft_sweep" in k or not only
     assert "k_soft_sweep" not in k or lib.fake_soft_fp64_only() == only
 """)
+
+
+CONVEX = 'GpuPacking(W.CONVEX, "cuboid 1 1 2; sphere 0.1; sum", W.lattice(({0}, {0}, {0}), ({1},) * 3), W.aligned_rotations({0} ** 3),' \
+         ' W.diag_box({0} * {1}, {0} * {1}, {0} * {1}))'
+
+
+@pytest.mark.parametrize("side,cell,counting,warps", [(6, 2.8, False, 1), (6, 2.8, True, 8), (6, 1.1, False, 8)])
+def test_warps_of_a_convex_single_move(fake, side, cell, counting, warps):
+    run(fake, f"""
+g = {CONVEX.format(side, cell)}
+g.set_counting({counting})
+assert "k_try_singleILi3ELi{warps}E" in kernels(lambda: fails("", -1, lambda: g.try_move(0, 0, (0.1, 0.0, 0.0))))
+""")
