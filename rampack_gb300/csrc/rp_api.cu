@@ -565,7 +565,7 @@ size_t batch_capacity(size_t bytes, int kind) {
 // Chooses the checkerboard grid for a box: cells at least one interaction range high
 // in every direction, an even count per direction (or a single cell), so that cells of
 // one colour never interact.
-int setup_grid(Handle *h, GridHost &G, const double *box, const double *shift) {
+int setup_grid(Handle *h, GridHost &G, const double *box, const double *shift, bool fp64_only = false) {
     double hgt[3];
     heights_of(box, hgt);
     // at least one interaction range (bodies in two cells of one colour never interact),
@@ -718,8 +718,9 @@ int setup_grid(Handle *h, GridHost &G, const double *box, const double *shift) {
         const bool allowed = h->stage_mode != 0 && h->order_mode == RP_ORDER_OFF && h->pair_cap == 0;
         // (staging through the filter walks the neighbours twice: at 0.83 to 0.88 kept it costs more than
         // the shorter scans save, 6.96 against 6.55 ms for five sweeps of 64,000 rods; two cells per warp
-        // need the room)
-        const double worth = h->cells_per_warp == 2 ? 0.9 : 0.65;
+        // need the room, and a sweep that decides every staged pair in FP64 wants few of them: 20.3
+        // against 17.1 ms for 14,391 bent rods in one launch)
+        const double worth = h->cells_per_warp == 2 || fp64_only ? 0.9 : 0.65;
         if (dims[0] > 1 && dims[1] > 1 && dims[2] > 1 && allowed && (kept < worth || h->stage_mode == 2))
             g.stage_filter = 1;
         if (!g.stage_filter) kept = 1.0;
@@ -1796,7 +1797,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     // the lists are out of date until the launch that builds them for the new origin has succeeded
     h->grid_stale = true;
     h->grid_patched = false;
-    int rc = setup_grid(h, h->grid[h->gcur], h->box, shift);
+    int rc = setup_grid(h, h->grid[h->gcur], h->box, shift, (p->flags & RP_SWEEP_FP64_ONLY) != 0);
     if (rc) return rc;
     auto current = [h]() {
         h->grid_stale = false;
@@ -1838,10 +1839,11 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     // small systems: the rebuild and every phase in one launch of a thread-block cluster, where each
     // active cell of a phase gets a warp there (1000 spheres: 180 -> 69 us a sweep; with more cells
     // than that the whole chip's warps are worth the launches).  Soft spheres: where any neighbourhood
-    // fits, as their sweeps refuse none
+    // fits, as their sweeps refuse none.  Not multi-centre bodies in FP64 alone, which are bound by the
+    // FP64 pipes, 16 SMs' there (14,391 bent rods: 17.1 against 9.7 ms)
     int cl_warps = 0;
     if (!fp64_sweep && !convex && !h->bulk_stage && h->cells_per_warp == 1 && h->order_mode == RP_ORDER_OFF && h->pair_cap == 0 &&
-        h->n <= CLUSTER_MAX_N && g.ncell <= CLUSTER_MAX_CELLS &&
+        h->n <= CLUSTER_MAX_N && g.ncell <= CLUSTER_MAX_CELLS && !(h->ncen > 0 && (p->flags & RP_SWEEP_FP64_ONLY)) &&
         !(soft32 && h->n > static_cast<int64_t>(staging_capacity(OVF_SMEM, h->shape.kind, 0)))) {
         if (h->cl_blocks < 0) h->cl_blocks = cluster_blocks();
         int most = 0, act[3];
@@ -3174,7 +3176,7 @@ int rp_batch_sweep(void *batch, const rp_sweep_params *p, rp_sweep_stats *stats)
         double shift[3];
         uint32_t shuffle = 0;
         sweep_origin(replica_seed(p->seed, r), p->counter, shift, shuffle);
-        int rc = setup_grid(h, h->grid[h->gcur], h->box, shift);
+        int rc = setup_grid(h, h->grid[h->gcur], h->box, shift, (p->flags & RP_SWEEP_FP64_ONLY) != 0);
         if (rc) return bfail(b, rc, h->err);
         const GridHost &G = h->grid[h->gcur];
         phase_order(G.d, shuffle, phases[r]);

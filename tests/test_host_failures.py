@@ -134,3 +134,16 @@ g = {CONVEX.format(side, cell)}
 g.set_counting({counting})
 assert "k_try_singleILi3ELi{warps}E" in kernels(lambda: fails("", -1, lambda: g.try_move(0, 0, (0.1, 0.0, 0.0))))
 """)
+
+
+@pytest.mark.parametrize("shape,fp64_only,cluster", [
+    ("spheres()", False, True), ("spheres()", True, True),
+    ('GpuPacking(W.POLYSPHEROCYLINDER, W.polyspherocylinder_params(W.BENT_ROD), W.lattice((5, 5, 5), (2.0,) * 3),'
+     ' W.aligned_rotations(125), W.diag_box(10.0, 10.0, 10.0))', False, True),
+    ('GpuPacking(W.POLYSPHEROCYLINDER, W.polyspherocylinder_params(W.BENT_ROD), W.lattice((5, 5, 5), (2.0,) * 3),'
+     ' W.aligned_rotations(125), W.diag_box(10.0, 10.0, 10.0))', True, False)])
+def test_small_sweeps_in_fp64_alone_spread_multi_centre_bodies_over_the_chip(fake, shape, fp64_only, cluster):
+    run(fake, f"""
+g = {shape}
+assert ("k_cluster_sweep" in kernels(lambda: g.sweep(0.1, 0.1, seed=1, counter=0, fp64_only={fp64_only}))) == {cluster}
+""")
