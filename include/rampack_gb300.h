@@ -515,6 +515,13 @@ int rp_set_bulk_staging(void *handle, int32_t on);
  * ends on short cells), 0 in cell-index order.  Cells of one phase are never neighbours, so
  * decisions, logs and states are the same either way. */
 int rp_set_cell_order(void *handle, int32_t on);
+/* How a small system's plain sweep runs (one whose phases have at most as many active cells as one
+ * thread-block cluster holds warps): 1 (default) in one launch, the rebuild and every phase inside the
+ * cluster, where the cell order has no meaning; 0 phase by phase, as larger systems' sweeps.
+ * Decisions, logs and states are the same either way. */
+int rp_set_cluster_sweep(void *handle, int32_t on);
+/* Whether the last sweep ran in one launch (1 or 0). */
+int rp_get_cluster_sweep(void *handle, int32_t *last);
 
 /* ---- the Monte Carlo cycle loop (Simulation for hard bodies) -----------------------
  *

@@ -123,6 +123,8 @@ SIGNATURES = {
     "rp_set_cells_per_warp": (C.c_int, [_P, C.c_int32]),
     "rp_set_bulk_staging": (C.c_int, [_P, C.c_int32]),
     "rp_set_cell_order": (C.c_int, [_P, C.c_int32]),
+    "rp_set_cluster_sweep": (C.c_int, [_P, C.c_int32]),
+    "rp_get_cluster_sweep": (C.c_int, [_P, C.POINTER(C.c_int32)]),
     "rp_set_soft": (C.c_int, [_P, C.c_int32, C.c_double, C.c_double, C.c_int32]),
     "rp_set_temperature": (C.c_int, [_P, C.c_double]),
     "rp_total_energy": (C.c_int, [_P, C.POINTER(C.c_double)]),

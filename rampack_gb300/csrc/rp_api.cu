@@ -183,6 +183,7 @@ struct Handle {
     float *rtab32 = nullptr;
     int32_t *item_counters = nullptr;  // work counters of persistent sweep launches
     int num_sms = 0;
+    int cluster_sweep = 1, last_cluster = 0;   // rp_set_cluster_sweep, and whether the last sweep was one
     int cl_blocks = -1;                // blocks of a cluster sweep on this device (-1: not asked yet)
     // the answers of recounts and box moves in one device block, so that one copy brings them to the
     // page-locked `answers` (their order here): overlaps, early-exit flag, particles that changed cell
@@ -1842,7 +1843,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     // fits, as their sweeps refuse none.  Not multi-centre bodies in FP64 alone, which are bound by the
     // FP64 pipes, 16 SMs' there (14,391 bent rods: 17.1 against 9.7 ms)
     int cl_warps = 0;
-    if (!fp64_sweep && !convex && !h->bulk_stage && h->cells_per_warp == 1 && h->order_mode == RP_ORDER_OFF && h->pair_cap == 0 &&
+    if (h->cluster_sweep && !fp64_sweep && !convex && !h->bulk_stage && h->cells_per_warp == 1 && h->order_mode == RP_ORDER_OFF && h->pair_cap == 0 &&
         h->n <= CLUSTER_MAX_N && g.ncell <= CLUSTER_MAX_CELLS && !(h->ncen > 0 && (p->flags & RP_SWEEP_FP64_ONLY)) &&
         !(soft32 && h->n > static_cast<int64_t>(staging_capacity(OVF_SMEM, h->shape.kind, 0)))) {
         if (h->cl_blocks < 0) h->cl_blocks = cluster_blocks();
@@ -1850,6 +1851,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
         for (int ph : phases) most = std::max(most, phase_cells(g, ph, act));
         cl_warps = cluster_warps(sweep_args(0.0), h->cl_blocks, most);
     }
+    h->last_cluster = cl_warps ? 1 : 0;
     if (!cl_warps) {
         rc = rebuild(h, h->gcur, h->pcur);
         if (rc) return rc;
@@ -2768,6 +2770,20 @@ int rp_set_cell_order(void *handle, int32_t on) {
     Handle *h = static_cast<Handle *>(handle);
     if (!h || (on != 0 && on != 1)) return fail(h, RP_ERR_ARG, "cell order must be 0 or 1");
     h->cell_order = on;
+    return RP_OK;
+}
+
+int rp_set_cluster_sweep(void *handle, int32_t on) {
+    Handle *h = static_cast<Handle *>(handle);
+    if (!h || (on != 0 && on != 1)) return fail(h, RP_ERR_ARG, "cluster sweep must be 0 or 1");
+    h->cluster_sweep = on;
+    return RP_OK;
+}
+
+int rp_get_cluster_sweep(void *handle, int32_t *last) {
+    Handle *h = static_cast<Handle *>(handle);
+    if (!h || !last) return RP_ERR_ARG;
+    *last = h->last_cluster;
     return RP_OK;
 }
 

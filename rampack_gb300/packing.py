@@ -269,6 +269,16 @@ class GpuPacking:
         (rp_set_cell_order)."""
         self._check(self.lib.rp_set_cell_order(self.h, 1 if on else 0))
 
+    def set_cluster_sweep(self, on: bool):
+        """Small systems' sweeps in one launch (1) or phase by phase (0) (rp_set_cluster_sweep)."""
+        self._check(self.lib.rp_set_cluster_sweep(self.h, 1 if on else 0))
+
+    def cluster_sweep(self) -> bool:
+        """Whether the last sweep ran in one launch (rp_get_cluster_sweep)."""
+        v = C.c_int32()
+        self._check(self.lib.rp_get_cluster_sweep(self.h, C.byref(v)))
+        return v.value == 1
+
     def set_cells_per_warp(self, cells: int):
         """1: a warp sweeps one cell; 2: each half-warp sweeps its own (rp_set_cells_per_warp)."""
         self._check(self.lib.rp_set_cells_per_warp(self.h, int(cells)))
