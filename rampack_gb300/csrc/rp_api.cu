@@ -80,8 +80,7 @@ namespace {
 
 constexpr int OVF_WARPS = 152;          // overflow rerun: one warp per block, grid-stride over cells
 constexpr size_t OVF_SMEM = 208 * 1024; // shared memory of one overflow warp
-constexpr int64_t CLUSTER_MAX_N = 32768;     // particles and cells of a cluster sweep's rebuild (16 blocks)
-constexpr int CLUSTER_MAX_CELLS = 16384;
+constexpr int64_t CLUSTER_MAX_N = 32768;     // particles of a cluster sweep's rebuild (16 blocks)
 
 struct GridHost {
     GridDev d{};
@@ -1844,7 +1843,7 @@ int rp_sweep(void *handle, const rp_sweep_params *p, rp_sweep_stats *stats) {
     // FP64 pipes, 16 SMs' there (14,391 bent rods: 17.1 against 9.7 ms)
     int cl_warps = 0;
     if (h->cluster_sweep && !fp64_sweep && !convex && !h->bulk_stage && h->cells_per_warp == 1 && h->order_mode == RP_ORDER_OFF && h->pair_cap == 0 &&
-        h->n <= CLUSTER_MAX_N && g.ncell <= CLUSTER_MAX_CELLS && !(h->ncen > 0 && (p->flags & RP_SWEEP_FP64_ONLY)) &&
+        h->n <= CLUSTER_MAX_N && !(h->ncen > 0 && (p->flags & RP_SWEEP_FP64_ONLY)) &&
         !(soft32 && h->n > static_cast<int64_t>(staging_capacity(OVF_SMEM, h->shape.kind, 0)))) {
         if (h->cl_blocks < 0) h->cl_blocks = cluster_blocks();
         int most = 0, act[3];

@@ -32,7 +32,7 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 constexpr int SOFT_WARPS = 4;   // warps per block of the soft sweep
-constexpr int XC_QUEUE = 256;   // convex bodies: near (candidate, image) pairs queued per warp
+constexpr int XC_QUEUE = 256;   // convex bodies: near pairs queued per warp, each candidate * 28 + image
 
 // One mover in shared memory: [0] the tried state, [1] the current one.
 struct Mover {
@@ -44,7 +44,6 @@ struct Mover {
     int ncells[2];
     int cstart[2][28];                  // prefix of those cells' occupancies
     int outside;                        // the tried position lies outside the ActiveDomain
-    mutable int xq[XC_QUEUE];           // convex bodies: candidate * 28 + image of the near pairs
 };
 
 // Grid cell coordinate d of fractional coordinate r: the rebuild's own arithmetic (assign_one).
@@ -572,20 +571,21 @@ __device__ void build_mover(const SingleArgs &A, Mover &mv, const rp_move &m, in
 
 // The move's energy (the whole warp, after build_mover): the ActiveDomain, then the hard part
 // (any overlap, or in overlap counting the sign of the change of the mover's count:
-// core/Packing.cpp:304-323), then the soft part's energy change (core/Packing.cpp:103-108).
+// core/Packing.cpp:304-323), then the soft part's energy change (core/Packing.cpp:103-108).  xq: the
+// warp's queue of near pairs (convex bodies).
 template <int KIND>
-__device__ double move_energy(const SingleArgs &A, const Mover &mv, int pid, int &delta) {
+__device__ double move_energy(const SingleArgs &A, const Mover &mv, int pid, int *xq, int &delta) {
     const DevState &s = A.s;
     delta = 0;
     if (mv.outside) return CUDART_INF;
     if (!s.soft_only) {
         if (s.counting) {
-            const int after = warp_overlaps<KIND>(A, mv, 0, false, pid, 0, 32, mv.xq);
-            const int before = warp_overlaps<KIND>(A, mv, 1, false, pid, 0, 32, mv.xq);
+            const int after = warp_overlaps<KIND>(A, mv, 0, false, pid, 0, 32, xq);
+            const int before = warp_overlaps<KIND>(A, mv, 1, false, pid, 0, 32, xq);
             delta = after - before;
             if (delta < 0) return -CUDART_INF;
             if (delta > 0) return CUDART_INF;
-        } else if (warp_overlaps<KIND>(A, mv, 0, true, pid, 0, 32, mv.xq)) {
+        } else if (warp_overlaps<KIND>(A, mv, 0, true, pid, 0, 32, xq)) {
             return CUDART_INF;
         }
     }
@@ -695,6 +695,7 @@ __global__ void k_commit_single(DevState s, SingleTry *t, uint8_t *disp_flag, in
 template <int KIND>
 __global__ void __launch_bounds__(SOFT_WARPS * 32, 4) k_soft_sweep(SoftSweepArgs A) {
     __shared__ Mover movers[SOFT_WARPS];
+    __shared__ int xq[KIND == 3 ? SOFT_WARPS : 1][XC_QUEUE];
     __shared__ rp_move moves[SOFT_WARPS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     Mover &mv = movers[wib];
@@ -772,7 +773,7 @@ __global__ void __launch_bounds__(SOFT_WARPS * 32, 4) k_soft_sweep(SoftSweepArgs
             __syncwarp();
             build_mover<KIND>(C, mv, m, pid, true, lo, hi, bounded);
             int delta = 0;
-            const double dE = move_energy<KIND>(C, mv, pid, delta);
+            const double dE = move_energy<KIND>(C, mv, pid, xq[KIND == 3 ? threadIdx.x >> 5 : 0], delta);
             // Metropolis (core/Simulation.cpp:483): u <= exp(-dE / T)
             const bool acc = metropolis(uni, dE, C.temperature);
             const uint8_t code = mv.outside ? 2 : (dE == CUDART_INF ? 1 : (dE == -CUDART_INF ? 3 : 0));
