@@ -480,8 +480,9 @@ int rp_batch_set_walls(void *batch, int32_t mask);
  * keeps the soft part alone (SphereTraits(r, centralInteraction), PolysphereTraits(geometry,
  * centralInteraction); spheres and polyspheres).  kind RP_SOFT_NONE removes it.  Moves then
  * return the energy change (core/Packing.cpp:103-108), box moves the change of the total
- * energy (:172-207); sweeps decide every move in FP64 at the handle's temperature; move lists
- * (rp_run_moves) are refused.  Lennard-Jones is refused: it has no cut-off, so the
+ * energy (:172-207); sweeps decide every move as FP64 does at the handle's temperature (spheres in
+ * FP32 where an error bound leaves one answer, see RP_SWEEP_FP64_ONLY); move lists (rp_run_moves)
+ * are refused.  Lennard-Jones is refused: it has no cut-off, so the
  * reference's particle energy sums over whatever its neighbour-grid cells hold. */
 int rp_set_soft(void *handle, int32_t kind, double epsilon, double sigma, int32_t hard);
 /* The Metropolis temperature of sweeps with a soft part (default 1; rp_sim sets it). */

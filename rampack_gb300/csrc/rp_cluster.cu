@@ -3,8 +3,7 @@
 //
 // A small system's sweep is bound by launches, not by work: with at most 256 active cells a phase,
 // a rebuild of six launches and 8 to 27 phases of two launches each (the sweep and the rerun of
-// overfull neighbourhoods) took 180 us a cycle for 1000 hard spheres, of which a warp's cell takes
-// about 5 us.  Up to 16 blocks (one per SM of a GPC) give every active cell a warp of its own; the
+// overfull neighbourhoods) took 180 us a sweep for 1000 hard spheres; one launch takes 69.  Up to 16 blocks (one per SM of a GPC) give every active cell a warp of its own; the
 // blocks of a cluster are scheduled together, so the barrier needs no cooperative launch and
 // several handles' sweeps may run side by side.  Cells, moves and their order within a cell are
 // the phase-by-phase sweep's, so the results are the same.

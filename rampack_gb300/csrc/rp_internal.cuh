@@ -121,7 +121,7 @@ struct DevState {
     int segs;
     double chax[RP_MAX_CENTRES][3];
     const double *circ64;
-    // the recount's deferred FP64 centre pairs (multi-centre bodies): queued by k_count_poly,
+    // the recount's deferred FP64 centre pairs (multi-centre bodies): queued by k_count_cells,
     // decided by k_count_deferred with every lane busy; null: decided inline
     struct DeferredPair *cq_buf;
     int *cq_count;
