@@ -661,7 +661,9 @@ __device__ __forceinline__ void sweep_cell(const SweepArgs &A, const int item, c
                 const int slot = (int)(((uint64_t)(r.a & 0x7fffffffu) * (uint32_t)occ) >> 31);
                 // pm1f takes the top 24 bits of a word: a rototranslation's rotation takes the low bytes
                 const float s = type == 1 ? 0.f : A.tstep;
-                props[lane] = make_float4(pm1f(r.b) * s, pm1f(r.c) * s, pm1f(r.d) * s, __uint_as_float((uint32_t)slot << 2 | type));
+                // (+ 0: a rotation's translation is logged as +0, not -0)
+                props[lane] = make_float4(fmaf(pm1f(r.b), s, 0.f), fmaf(pm1f(r.c), s, 0.f), fmaf(pm1f(r.d), s, 0.f),
+                                          __uint_as_float((uint32_t)slot << 2 | type));
                 if (type != 0 && mi + lane < nmoves) {
                     // a rotation of this sweep's table, or its transpose (the inverse): all of the
                     // batch on their way from L2 at once
