@@ -444,7 +444,7 @@ void poly_segment_consts(const Handle *h, const GridHost &g, FilterConsts &fc) {
     const double ddp = 4.0 * u32 * std::sqrt(3.0) * (2 * r + 4 * l);
     const double eval = 2.0 * 1.1 * (2 * r) * ddp + ddp * ddp + 16.0 * u32 * (2 * r) * l + 4.0 * u32 * 4 * r * r;
     const double noise = 8.0 * u64 * 2.0 * l * l * l * (2 * r + 2 * l), g64 = 2e-6;
-    const double d_min = std::max(4.0 * (2 * r) * l * std::sqrt(2.0) * noise / g64 * 10.0, 1e-9 * l * l * l * l);
+    const double d_min = std::max({4.0 * (2 * r) * l * std::sqrt(2.0) * noise / g64 * 10.0, 1e-9 * l * l * l * l, snap_d_min(l)});
     fc.seg_err = static_cast<float>(2.0 * (2.0 * (2 * r) * 2.0 * dend + 4.0 * dend * dend + eval) + g64);
     // (FP64's parallel branch, D below 1e-10, is never certified)
     fc.s2_min = static_cast<float>(std::max(d_min, 4e-10) / 16.0);

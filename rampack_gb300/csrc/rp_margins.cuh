@@ -18,6 +18,15 @@ namespace rp {
 // cylinder length l) or convex body (circumsphere radius r, insphere radius l) whose FP32 coordinates are cell-local: lrow is the largest row norm of
 // the cell matrix (box / dims), box the row-major box.  Polysphere thresholds depend on the
 // centres and are formed by the caller.
+
+// The least D = |u|^2 |v|^2 - (u.v)^2 of two segments of at most length l at which FP64's distance^2 is
+// within 1e-6 of the minimum for all that it takes numerators sN, tN below 1e-10 for zero
+// (SegmentDistanceCalculator.h:79-80).  At a free minimum (sD = tD = D) that moves the points by at most
+// 2 l 1e-10 / D, and the gradient is zero there, so the distance^2 grows by at most that squared; at a
+// clamped one (sD = |u|^2 or tD = |v|^2) by at most 1e-10, but where |v|^2 itself is below 1e-10, which
+// the second term excludes.
+inline double snap_d_min(double l) { return std::max(2e-7 * l, 1e-10 * l * l); }
+
 inline FilterConsts hard_filter_consts(int kind, double r, double l, double lrow, const double *box) {
     const double u32 = std::ldexp(1.0, -24);
     // Per-component bound of the FP32 separation error, in units of u32 times the largest
@@ -70,6 +79,7 @@ inline FilterConsts hard_filter_consts(int kind, double r, double l, double lrow
         // inputs; rounding in sN = b e - c d and D = a c - b^2 = l^4 sin^2 (|b|, |c| <= l^2,
         // |d|, |e| <= l (2r + 2l)) moves the parameters by at most noise / D, which raises
         // its distance^2 above the minimum by at most g64 = 2 (2r) l sqrt(2) noise / D.
+        // Its closest points move further where it takes small numerators for zero (snap_d_min).
         // Pairs whose (cancellation-free) D is below d_min are re-decided in FP64; g64 at
         // d_min joins the certificate's margin.
         double pmax = 0;
@@ -79,7 +89,7 @@ inline FilterConsts hard_filter_consts(int kind, double r, double l, double lrow
         const double noise = 8.0 * u64 * 2.0 * l * l * l * (2 * r + 2 * l);
         const double g64 = 2e-6;
         const double l4 = l * l * l * l;
-        const double d_min = std::max(4.0 * (2 * r) * l * std::sqrt(2.0) * noise / g64 * 10.0, 1e-9 * l4);
+        const double d_min = std::max({4.0 * (2 * r) * l * std::sqrt(2.0) * noise / g64 * 10.0, 1e-9 * l4, snap_d_min(l)});
         fc.s2_min = l > 0 ? static_cast<float>(d_min / l4) : 2.0f;   // l = 0: every pair in FP64
         fc.seg_err = static_cast<float>(safety * (2.0 * (2 * r) * 2.0 * dend + 4.0 * dend * dend + eval) + g64);
         // Parallel branch (SegmentDistanceCalculator.h:35-39, taken when FP64's D < 1e-10):
